@@ -116,6 +116,69 @@ struct DTree {
   double* node_gain;   // unrounded gain of each split (diagnostics)
 };
 
+// Growth in rounds (round_kernels.cuh): a node of the explored tree. Node 0
+// is the root; expansion e of the tree creates nodes 2e + 1 (left) and
+// 2e + 2 (right).
+struct RNode {
+  int32_t parent;        // -1: the root
+  int32_t begin, count;  // its rows, in index buffer `side`
+  int32_t side, depth;
+  int32_t buf;           // histogram buffer
+  int32_t need;          // before_find_best_split of this node and its sibling
+  int32_t pad;
+  DLeafSplits ls;
+  double cmin, cmax;     // basic monotone constraint
+};
+// One expansion of the running round: the node's rows, its place among the
+// round's row tiles, and the histogram buffer of its smaller child.
+struct RItem {
+  int32_t node, begin, count, side;
+  int32_t inner, tile0, buf, pad;
+};
+struct RoundState {
+  int32_t e0, nb;        // this round's expansions: [e0, e0 + nb)
+  int32_t ntiles;        // row tiles of the round
+  int32_t ticket;        // next row tile
+  uint32_t epoch;        // of the tiles' look-back words
+  int32_t popped;        // splits of the final tree replayed so far
+  int32_t done;
+  int32_t root;          // 1: the first round, which only searches the root
+  int32_t rounds;        // rounds run
+  int32_t ncopy;         // row pieces k_round_restore moves
+  int32_t ncand, nfree;  // lengths of cand and free
+  double root_value;     // the root's output
+};
+// A run of rows to copy into the other index buffer (k_round_restore).
+struct RCopy {
+  int32_t begin, count, side, pad;
+};
+struct DRounds {
+  RoundState* st;
+  RNode* node;           // [2 * ecap + 1]
+  DSplit* best;          // each node's best split
+  double* gain;          // its (penalized) gain, -inf none
+  int32_t* feat;         // its real feature, -1 none
+  int32_t* exp;          // the node's expansion (kReplayed set once the replay has split it), -1 not expanded
+  uint8_t* splittable;   // [node][num_features]
+  int32_t* exp_node;     // [ecap]: the node of each expansion
+  RItem* item;           // [bmax]
+  DSplit* fres;          // scan results [bmax][2][num_features]
+  int32_t* scan_cnt;     // [bmax][2] scans stored
+  int32_t* cand;         // [pool]: unexpanded nodes that may still be split
+  int32_t* free;         // [pool]: unused histogram buffers
+  int32_t* free_next;    // [pool]: scratch, the buffers a round gives back
+  int32_t* leaf_node;    // [num_leaves]: the node of each leaf of the replayed tree
+  int32_t* pop_node;     // [num_leaves]: the node and leaf of each split of the replayed tree
+  int32_t* pop_leaf;
+  int32_t* pop_time;     // [node] scratch of k_round_emit: split index, -1
+  int32_t* node_leaf;    // [node] scratch of k_round_emit: leaf index, -1
+  RCopy* copy;           // [ecap + 1]
+  unsigned long long* status;  // look-back words of a round's row tiles
+  int32_t ecap, bmax, pool;
+};
+constexpr int kRoundBins = 1024;
+constexpr int32_t kReplayed = 1 << 30;
+
 // Device pointers of one tree slot.
 struct DSlot {
   DSlotState* st;
@@ -144,6 +207,7 @@ struct DSlot {
   long long* root_ipartials;
   int32_t* root_counter;
   DTree tree;
+  DRounds r;
   // data-parallel growth: the split decision the partition leaves for the
   // finishing launch, and this rank's rows sent left
   unsigned char* dp_dec;
@@ -175,14 +239,6 @@ struct DCtx {
   int32_t q_in_row;        // 1: each row's packed gradient also fills its bin row's padding bytes 28..31
                            // (one tree slot, one feature tile of at most 28 features)
 };
-
-// Programmatic dependent launch: a kernel launched with programmatic stream
-// serialisation may start while its predecessor in the stream still runs.
-// pdl_wait blocks until the predecessor has finished and its writes are
-// visible (a no-op for an ordinary launch); pdl_trigger lets the next kernel
-// of the stream start launching.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- split arithmetic (learner/split.rs:124-231) -------------------------------------
 __device__ __forceinline__ double dsign(double x) { return (double)((x > 0.0) - (x < 0.0)); }

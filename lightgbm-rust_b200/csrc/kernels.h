@@ -63,26 +63,8 @@ const void* hist_kernel(int mode, int ng);
 // finish: one more cluster whose first CTA runs the previous split step's end,
 // which the partition posted (DCtx::defer)
 cudaError_t launch_hist(int mode, int ng, dim3 grid, size_t smem, cudaStream_t st, const DCtx& c, const DTileTable& tt,
-                        int32_t sub_rows, bool pdl, bool finish);
+                        int32_t sub_rows, bool finish);
 
-// A kernel launch, optionally with programmatic stream serialisation (the
-// kernel may start launching while its predecessor in the stream runs; it
-// calls pdl_wait before reading anything the predecessor writes).
-template <typename... Params, typename... Args>
-inline cudaError_t launch_ex(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl,
-                             Args&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
-}
 constexpr int kScanWideBlocks = 4;  // scan CTAs per SM when a step's scans span several waves
 template <bool kInt, int kMinBlocks>
 __global__ void k_scan(const __grid_constant__ DCtx c);
@@ -122,13 +104,32 @@ size_t grow_smem_bytes(int mode, int ng);
 cudaError_t launch_grow(int mode, int ng, int grid, size_t smem, cudaStream_t st, const DCtx& c, const DTileTable& tt,
                         int32_t sub_rows, int32_t ntiles, GrowSync* gs, int32_t num_steps, long long* phase_ns);
 __global__ void k_partition(const __grid_constant__ DCtx c);
-// the quantized threshold scan by one warp per (feature, side) item;
-// grid (CTAs, 1, slots), kScanThreads threads
-template <int kMinBlocks>
-__global__ void k_scan_warp(const __grid_constant__ DCtx c, const int32_t* items);
 // the last split step's end, when the partitions post theirs (DCtx::defer);
 // grid (1, 1, slots), kPartThreads threads
 __global__ void k_finish(const __grid_constant__ DCtx c);
+// Growth in rounds (round_kernels.cuh).
+constexpr int kMaxRoundItems = 256;     // expansions per round at most
+constexpr int kRoundMin = 24;           // and the least a round may take when that many are worth it
+constexpr int kF64ScanThreads = 128;
+constexpr int kScanF64Blocks = 4;       // CTAs of the FP64 scan per SM
+constexpr int kScanIntBlocks = 3;       // CTAs of the quantized scan per SM
+constexpr unsigned long long kRoundRows = 8000000;  // rows a round expands on speculation at most
+constexpr int kDecideThreads = 512;
+constexpr int kDecideSmemNodes = 3072;  // explored nodes the replay keeps in shared memory
+__global__ void k_round_part(const __grid_constant__ DCtx c);
+const void* round_hist_kernel(int mode, int ng);
+cudaError_t launch_round_hist(int mode, int ng, dim3 grid, size_t smem, cudaStream_t st, const DCtx& c,
+                              const DTileTable& tt, int32_t sub_rows);
+// the threshold scans of a round, on packed integer and on FP64 sums
+__global__ void k_round_scan_int(const __grid_constant__ DCtx c);
+__global__ void k_round_scan_f64(const __grid_constant__ DCtx c);
+size_t round_scan_int_smem(bool cat);
+size_t round_scan_f64_smem();
+size_t round_decide_smem(int num_leaves);
+__global__ void k_round_decide(const __grid_constant__ DCtx c, int32_t* ctrl, cudaGraphConditionalHandle cond,
+                               int32_t use_cond);
+__global__ void k_round_emit(const __grid_constant__ DCtx c);
+__global__ void k_round_restore(const __grid_constant__ DCtx c);
 __global__ void k_transpose_bins(const uint8_t* bins, int64_t n, int32_t stride, int32_t nf, uint8_t* colbins);
 __global__ void k_leaf_sums(const __grid_constant__ DCtx c, double* partial, int32_t* rank);
 __global__ void k_leaf_renew(const __grid_constant__ DCtx c, const double* partial, const int32_t* rank,

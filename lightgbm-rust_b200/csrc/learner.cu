@@ -160,10 +160,6 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
     h->scan_part_grid = std::min(h->part_grid, h->scan_part_max);
     if (h->scan_part_grid < 1) return Status(LGBM_B200_ERR_UNSUPPORTED, "scan + partition launch does not fit");
   }
-  // programmatic dependent launch per kernel edge, a bit mask: 1 the
-  // histogram (after the partition), 2 the scan (after the histogram), 4 the
-  // partition (after the scan)
-  if (const char* e = std::getenv("LGBM_B200_PDL")) h->use_pdl = std::atoi(e) & 7;
   if (cfg->persistent_grow) {
     // one resident CTA group per slot: the cooperative launch holds every CTA
     const void* gk = grow_kernel(mode, h->hist_ng);
@@ -197,41 +193,28 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
   if (!(s = A.alloc_n(&feats_d, (size_t)nf)).ok()) return s;
   CU(cudaMemcpy(feats_d, h->feats.data(), sizeof(DFeature) * nf, cudaMemcpyHostToDevice));
   const int K = h->K, L = h->L;
-  // The quantized scan by one warp per (feature, side) item, for steps whose
-  // block scans would run in waves (many features or tree slots): there the
-  // scan is bound by throughput, and eight items share a CTA without block
-  // barriers (multiclass K=10 x 200 features: 29.6 -> 25.1 ms per iteration).
-  // With few items each item's latency counts, and the block scan's 256
-  // threads per item are faster (binary x 28 features: 7.39 against 8.54 ms;
-  // lambdarank x 136: 29.9 against 31.1). Each CTA takes up to `per` items,
-  // at most one of them categorical (the CTA's scratch holds its sort).
-  // LGBM_B200_SCAN_WARP=0/1 forces either; LGBM_B200_SCAN_PER=<1..8> sets the
-  // items per CTA.
-  h->scan_warp = mode == LGBM_B200_HIST_QUANT && h->scan_wide;
-  if (const char* e = std::getenv("LGBM_B200_SCAN_WARP"))
-    h->scan_warp = mode == LGBM_B200_HIST_QUANT && std::atoi(e) != 0;
-  if (h->scan_warp) {
-    constexpr int kWarps = kScanThreads / 32;
-    std::vector<int32_t> numer, cats;
-    for (int f = 0; f < nf; ++f)
-      for (int side = 0; side < 2; ++side) (h->feats[f].bin_type == 1 ? cats : numer).push_back(f * 2 + side);
-    const int64_t items = (int64_t)numer.size() + (int64_t)cats.size();
-    int per = (int)std::min<int64_t>(kWarps, std::max<int64_t>(1, (items * K + h->num_sms - 1) / h->num_sms));
-    if (const char* e = std::getenv("LGBM_B200_SCAN_PER")) per = std::max(1, std::min(kWarps, std::atoi(e)));
-    const int64_t ctas = std::max<int64_t>((items + per - 1) / per, (int64_t)cats.size());
-    std::vector<int32_t> table((size_t)ctas * kWarps, -1);
-    size_t next = 0;
-    for (int64_t b = 0; b < ctas; ++b) {
-      int used = 0;
-      if ((size_t)b < cats.size()) table[(size_t)b * kWarps + used++] = cats[(size_t)b];
-      while (used < per && next < numer.size()) table[(size_t)b * kWarps + used++] = numer[next++];
-    }
-    if (!(s = A.alloc_n(&h->scan_items, table.size())).ok()) return s;
-    CU(cudaMemcpy(h->scan_items, table.data(), sizeof(int32_t) * table.size(), cudaMemcpyHostToDevice));
-    h->scan_warp_grid = (int)ctas;
-  }
   const size_t cells = (size_t)h->total_bins * (mode == LGBM_B200_HIST_QUANT ? 1 : 2);
   const size_t max_tiles = ((size_t)n + kPartTileRows - 1) / kPartTileRows + 1;
+  // Growth in rounds, unless a launch strategy that goes step by step is
+  // asked for (data-parallel growth also does, set after this). The explored
+  // tree may hold up to 16 times the splits of the finished one: 1.6 times is
+  // usual, 3 to 5 times on late trees of a run, whose gains hardly fall with
+  // depth. Only the nodes that may still be split hold a histogram, so three
+  // times the splits suffice there, less when that would take more than an
+  // eighth of the free memory (with none to spare, the rounds shrink to the
+  // one node the replay waits for).
+  h->rounds = !cfg->persistent_grow && !h->scan_part;
+  int32_t ecap = 0, bmax = 0, pool = 0;
+  if (h->rounds) {
+    const int32_t need = L - 1;
+    size_t free_b = 0, total_b = 0;
+    CU(cudaMemGetInfo(&free_b, &total_b));
+    const size_t hist_b = cells * 8 * (size_t)K + 1;
+    const size_t node_b = 2 * (sizeof(RNode) + sizeof(DSplit) + (size_t)nf + 64) * (size_t)K;
+    bmax = std::max(1, std::min(kMaxRoundItems, std::max(kRoundMin, (need + 3) / 4)));
+    ecap = need + (int32_t)std::min<size_t>(15 * (size_t)need, free_b / 16 / node_b);
+    pool = need + 1 + (int32_t)std::min<size_t>(2 * (size_t)need + 2 * (size_t)bmax, free_b / 8 / hist_b);
+  }
   {
     // the readback block: each slot's state, then its tree arrays, each
     // piece on a 256-byte boundary
@@ -244,6 +227,7 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
     auto& rb = h->rb;
     const size_t Ls = (size_t)L;
     rb.st = take(sizeof(DSlotState));
+    rb.rs = take(sizeof(RoundState));
     rb.sfi = take(4 * Ls);
     rb.sf = take(4 * Ls);
     rb.sg = take(4 * Ls);
@@ -288,7 +272,7 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
     ALLOC(d.cmax, L);
     {
       double* hp;
-      ALLOC(hp, cells * L);
+      ALLOC(hp, cells * (size_t)std::max(L, pool));
       d.hist = hp;
     }
     ALLOC(d.feat_res, 2 * (size_t)nf);
@@ -321,10 +305,63 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
     t.internal_count = reinterpret_cast<int32_t*>(rbk + rb.ic);
     t.cat_bits = reinterpret_cast<uint32_t*>(rbk + rb.cb);
     t.node_gain = reinterpret_cast<double*>(rbk + rb.ng);
+    if (h->rounds) {
+      DRounds& r = d.r;
+      const size_t nodes = 2 * (size_t)ecap + 1;
+      r.ecap = ecap;
+      r.bmax = bmax;
+      r.pool = pool;
+      r.st = reinterpret_cast<RoundState*>(rbk + rb.rs);
+      ALLOC(r.node, nodes);
+      ALLOC(r.best, nodes);
+      ALLOC(r.gain, nodes);
+      ALLOC(r.feat, nodes);
+      ALLOC(r.exp, nodes);
+      ALLOC(r.splittable, nodes * nf);
+      ALLOC(r.exp_node, ecap);
+      ALLOC(r.item, bmax);
+      ALLOC(r.fres, 2 * (size_t)bmax * nf);
+      ALLOC(r.scan_cnt, 2 * (size_t)bmax);
+      ALLOC(r.cand, pool);
+      ALLOC(r.free, pool);
+      ALLOC(r.free_next, pool);
+      ALLOC(r.leaf_node, L);
+      ALLOC(r.pop_node, L);
+      ALLOC(r.pop_leaf, L);
+      ALLOC(r.pop_time, nodes);
+      ALLOC(r.node_leaf, nodes);
+      ALLOC(r.copy, (size_t)ecap + 1);
+      ALLOC(r.status, max_tiles + bmax);
+      CU(cudaMemset(r.st, 0, sizeof(RoundState)));
+      CU(cudaMemset(r.status, 0, (max_tiles + bmax) * sizeof(unsigned long long)));
+    }
     CU(cudaMemset(d.st, 0, sizeof(DSlotState)));
     CU(cudaMemset(d.tile_status, 0, max_tiles * sizeof(unsigned long long)));
     CU(cudaMemset(d.root_counter, 0, sizeof(int32_t)));
     CU(cudaMemset(d.bytree, 1, nf));
+  }
+  if (h->rounds) {
+    if (!(s = A.alloc_n(&h->round_ctrl, 3)).ok()) return s;
+    CU(cudaMemset(h->round_ctrl, 0, 3 * sizeof(int32_t)));
+    // what is resident at once, shared by the slots (and feature tiles)
+    const void* hist = round_hist_kernel(mode, h->hist_ng);
+    CU(cudaFuncSetAttribute(hist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->hist_smem));
+    const bool quant = mode == LGBM_B200_HIST_QUANT;
+    bool cats = false;
+    for (auto& f : h->feats) cats |= f.bin_type == 1;
+    const void* scan = quant ? (const void*)k_round_scan_int : (const void*)k_round_scan_f64;
+    const int scan_threads = quant ? kScanThreads : kF64ScanThreads;
+    h->round_scan_smem = quant ? round_scan_int_smem(cats) : round_scan_f64_smem();
+    CU(cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->round_scan_smem));
+    CU(cudaFuncSetAttribute(k_round_decide, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)round_decide_smem(L)));
+    int per_sm = 0;
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, scan, scan_threads, h->round_scan_smem));
+    h->round_scan_grid = std::max(1, per_sm * h->num_sms / K);
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hist, kHistThreads, h->hist_smem));
+    h->hist_grid = std::max(1, per_sm * h->num_sms / (h->ntiles * K));
+    h->part_grid = std::max(1, h->part_grid / K);
+    CU(cudaStreamCreateWithFlags(&h->body_stream, cudaStreamNonBlocking));
   }
   if (!(s = A.alloc_n(&h->gh_all, (size_t)K * n)).ok()) return s;
   for (int k = 0; k < K; ++k) h->slots_h[k].gh = h->gh_all + (size_t)k * n;
@@ -442,8 +479,99 @@ Status quant_tables(LgbmB200Learner* h, int64_t rows) {
   return Status();
 }
 
-// Enqueue one whole tree (every slot) on the stream: init, the split steps
-// and leaf renewal. Nothing here reads device memory back.
+// CTAs of a step's histogram launch: whole clusters.
+static int step_hist_grid(const LgbmB200Learner* h) {
+  const int cl = hist_cluster(h->cfg.hist_precision);
+  return (h->hist_grid + cl - 1) / cl * cl;
+}
+
+// One round's launches on stream s (root: the first, which only searches the
+// root). ev: events around the histogram, scan and partition launches.
+static Status enqueue_round(LgbmB200Learner* h, cudaStream_t s, bool root, cudaGraphConditionalHandle cond,
+                            bool use_cond, cudaEvent_t* ev) {
+  const DCtx& c = h->ctx;
+  const int K = h->K;
+  if (ev) CU(cudaEventRecord(ev[0], s));
+  if (!root) {
+    k_round_part<<<dim3(h->part_grid, 1, K), kPartThreads, 0, s>>>(c);
+    CU_LAUNCH();
+  }
+  if (ev) CU(cudaEventRecord(ev[1], s));
+  CU(launch_round_hist(h->cfg.hist_precision, h->hist_ng, dim3(h->hist_grid, h->ntiles, K), h->hist_smem, s, c,
+                       h->tiles, h->sub_rows));
+  if (ev) CU(cudaEventRecord(ev[2], s));
+  const dim3 scan_grid(h->round_scan_grid, 1, K);
+  if (h->cfg.hist_precision == LGBM_B200_HIST_QUANT)
+    k_round_scan_int<<<scan_grid, kScanThreads, h->round_scan_smem, s>>>(c);
+  else k_round_scan_f64<<<scan_grid, kF64ScanThreads, h->round_scan_smem, s>>>(c);
+  CU_LAUNCH();
+  if (ev) CU(cudaEventRecord(ev[3], s));
+  k_round_decide<<<dim3(1, 1, K), kDecideThreads, round_decide_smem(h->L), s>>>(
+      c, h->round_ctrl, cond, use_cond ? 1 : 0);
+  CU_LAUNCH();
+  return Status();
+}
+
+// The rounds of one tree set. Under capture they are a conditional loop of
+// the graph, which the decision kernel ends; otherwise the host reads back
+// after every round whether another one runs.
+static Status enqueue_rounds(LgbmB200Learner* h) {
+  cudaStream_t s = h->stream;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaGraph_t graph = nullptr;
+  const cudaGraphNode_t* deps = nullptr;
+  size_t ndeps = 0;
+  CU(cudaStreamGetCaptureInfo(s, &cs, nullptr, &graph, &deps, &ndeps));
+  if (cs == cudaStreamCaptureStatusActive) {
+    cudaGraphConditionalHandle cond;
+    CU(cudaGraphConditionalHandleCreate(&cond, graph, 0, cudaGraphCondAssignDefault));
+    Status st = enqueue_round(h, s, true, cond, true, nullptr);
+    if (!st.ok()) return st;
+    CU(cudaStreamGetCaptureInfo(s, &cs, nullptr, &graph, &deps, &ndeps));
+    cudaGraphNodeParams np = {};
+    np.type = cudaGraphNodeTypeConditional;
+    np.conditional.handle = cond;
+    np.conditional.type = cudaGraphCondTypeWhile;
+    np.conditional.size = 1;
+    cudaGraphNode_t node;
+    CU(cudaGraphAddNode(&node, graph, deps, ndeps, &np));
+    cudaGraph_t body = np.conditional.phGraph_out[0];
+    CU(cudaStreamBeginCaptureToGraph(h->body_stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    st = enqueue_round(h, h->body_stream, false, cond, true, nullptr);
+    const cudaError_t e = cudaStreamEndCapture(h->body_stream, &body);
+    if (!st.ok()) return st;
+    CU(e);
+    CU(cudaStreamUpdateCaptureDependencies(s, &node, 1, cudaStreamSetCaptureDependencies));
+  } else {
+    // every round splits at least one leaf of the final tree
+    for (int round = 0; round < h->L; ++round) {
+      cudaEvent_t* ev = nullptr;
+      if (h->timing) {
+        while (h->ev.size() < (size_t)4 * (round + 1)) {
+          cudaEvent_t e;
+          CU(cudaEventCreate(&e));
+          h->ev.push_back(e);
+        }
+        ev = &h->ev[(size_t)4 * round];
+      }
+      Status st = enqueue_round(h, s, round == 0, 0, false, ev);
+      if (!st.ok()) return st;
+      int32_t more = 0;
+      CU(cudaMemcpyAsync(&more, h->round_ctrl + 2, sizeof(more), cudaMemcpyDeviceToHost, s));
+      CU(cudaStreamSynchronize(s));
+      h->last_rounds = round + 1;
+      if (!more) break;
+    }
+  }
+  k_round_emit<<<dim3(1, 1, h->K), kDecideThreads, 0, s>>>(h->ctx);
+  CU_LAUNCH();
+  k_round_restore<<<dim3(std::max(1, 2 * h->num_sms / h->K), 1, h->K), 256, 0, s>>>(h->ctx);
+  CU_LAUNCH();
+  return Status();
+}
+
+// Enqueue one whole tree (every slot) on the stream: init, its growth and
+// leaf renewal.
 Status enqueue_tree(LgbmB200Learner* h) {
   const DCtx& c = h->ctx;
   const int K = h->K, L = h->L;
@@ -452,57 +580,33 @@ Status enqueue_tree(LgbmB200Learner* h) {
   dim3 init_grid(h->root_grid, 1, K);
   k_tree_init<<<init_grid, 256, 0, s>>>(c, h->bagging ? h->bag : nullptr, h->n_used_dev);
   CU_LAUNCH();
-  dim3 hist_grid(h->hist_grid, h->ntiles, K);
-  dim3 scan_grid(h->nf, 2, K);
-  dim3 part_grid(h->part_grid, 1, K);
-  if (h->cfg.persistent_grow) {
+  if (h->rounds) {
+    Status st = enqueue_rounds(h);
+    if (!st.ok()) return st;
+  } else if (h->cfg.persistent_grow) {
     CU(cudaMemsetAsync(h->grow_sync, 0, sizeof(GrowSync), s));
     if (h->timing) CU(cudaMemsetAsync(h->phase_ns, 0, 4 * sizeof(long long), s));
     CU(launch_grow(mode, h->hist_ng, h->grow_grid, h->grow_smem, s, c, h->tiles, h->sub_rows, h->ntiles,
                    h->grow_sync, L - 1, h->timing ? h->phase_ns : nullptr));
-  }
-  for (int step = 0; step < (h->cfg.persistent_grow ? 0 : L - 1); ++step) {
-    cudaEvent_t* ev = h->timing ? &h->ev[(size_t)4 * step] : nullptr;
-    if (ev) CU(cudaEventRecordWithFlags(ev[0], s, cudaEventRecordExternal));
-    // the three launches of a step chain by programmatic dependent launch
-    // (not when events are recorded between them)
-    const int pdl_edges = h->timing ? 0 : h->use_pdl;
-    const bool pdl = (pdl_edges & 1) != 0, pdl_scan = (pdl_edges & 2) != 0, pdl_part = (pdl_edges & 4) != 0;
-    CU(launch_hist(mode, h->hist_ng, hist_grid, h->hist_smem, s, c, h->tiles, h->sub_rows, pdl && step > 0,
-                   c.defer && step > 0));
-    if (ev) CU(cudaEventRecordWithFlags(ev[1], s, cudaEventRecordExternal));
-    if (h->scan_part) {  // scans and partition in one launch: the scan interval records as empty
+  } else {  // step by step, the scans and the partition of a step in one launch
+    const dim3 hist_grid(step_hist_grid(h), h->ntiles, K);
+    const dim3 g(h->scan_part_grid, 1, K);
+    for (int step = 0; step < L - 1; ++step) {
+      cudaEvent_t* ev = h->timing ? &h->ev[(size_t)4 * step] : nullptr;
+      if (ev) CU(cudaEventRecordWithFlags(ev[0], s, cudaEventRecordExternal));
+      CU(launch_hist(mode, h->hist_ng, hist_grid, h->hist_smem, s, c, h->tiles, h->sub_rows, c.defer && step > 0));
+      if (ev) CU(cudaEventRecordWithFlags(ev[1], s, cudaEventRecordExternal));
+      // the scan interval records as empty
       if (ev) CU(cudaEventRecordWithFlags(ev[2], s, cudaEventRecordExternal));
-      const dim3 g(h->scan_part_grid, 1, K);
-      if (mode == LGBM_B200_HIST_QUANT) CU(launch_coop(k_scan_partition<true>, g, dim3(kPartThreads), h->scan_smem, s, c));
+      if (mode == LGBM_B200_HIST_QUANT)
+        CU(launch_coop(k_scan_partition<true>, g, dim3(kPartThreads), h->scan_smem, s, c));
       else CU(launch_coop(k_scan_partition<false>, g, dim3(kPartThreads), h->scan_smem, s, c));
       if (ev) CU(cudaEventRecordWithFlags(ev[3], s, cudaEventRecordExternal));
-      continue;
     }
-    if (mode == LGBM_B200_HIST_QUANT && h->scan_warp) {
-      const dim3 g(h->scan_warp_grid, 1, K);
-      if (h->scan_wide)
-        CU(launch_ex(k_scan_warp<kScanWideBlocks>, g, dim3(kScanThreads), 0, s, pdl_scan, c,
-                     (const int32_t*)h->scan_items));
-      else CU(launch_ex(k_scan_warp<2>, g, dim3(kScanThreads), 0, s, pdl_scan, c, (const int32_t*)h->scan_items));
-    } else if (mode == LGBM_B200_HIST_QUANT) {
-      if (h->scan_wide)
-        CU(launch_ex(k_scan<true, kScanWideBlocks>, scan_grid, dim3(kScanThreads), h->scan_smem, s, pdl_scan, c));
-      else CU(launch_ex(k_scan<true, 1>, scan_grid, dim3(kScanThreads), h->scan_smem, s, pdl_scan, c));
-    } else if (h->scan_wide) {
-      CU(launch_ex(k_scan<false, kScanWideBlocks>, scan_grid, dim3(kScanThreads), h->scan_smem, s, pdl_scan, c));
-    } else {
-      CU(launch_ex(k_scan<false, 1>, scan_grid, dim3(kScanThreads), h->scan_smem, s, pdl_scan, c));
+    if (c.defer) {  // the last split step's end (the earlier ones ran beside the histograms)
+      k_finish<<<dim3(1, 1, K), kPartThreads, 0, s>>>(c);
+      CU_LAUNCH();
     }
-    if (ev) CU(cudaEventRecordWithFlags(ev[2], s, cudaEventRecordExternal));
-    CU(launch_ex(k_partition, part_grid, dim3(256), 0, s, pdl_part, c));
-    if (ev) CU(cudaEventRecordWithFlags(ev[3], s, cudaEventRecordExternal));
-  }
-  // the last split step's end (the earlier ones ran beside the histograms)
-  const bool tail = c.defer && !h->cfg.persistent_grow && L > 1;
-  if (tail) {
-    k_finish<<<dim3(1, 1, K), kPartThreads, 0, s>>>(c);
-    CU_LAUNCH();
   }
   if (mode == LGBM_B200_HIST_QUANT && h->cfg.quant_train_renew_leaf) {
     k_leaf_sums<<<dim3(leaf_sum_warps(h) / 8, 1, K), 256, 16 * (size_t)L, s>>>(c, h->leaf_sums, h->leaf_rank);
@@ -510,9 +614,9 @@ Status enqueue_tree(LgbmB200Learner* h) {
     k_leaf_renew<<<dim3(1, 1, K), 256, 0, s>>>(c, h->leaf_sums, h->leaf_rank, leaf_sum_warps(h), nullptr);
     CU_LAUNCH();
   }
-  h->last_launches = 1 + (h->cfg.persistent_grow ? 1 : (h->scan_part ? 2 * (L - 1)
-                                                                                   : 3 * (L - 1))) +
-                     (tail ? 1 : 0) + ((mode == LGBM_B200_HIST_QUANT && h->cfg.quant_train_renew_leaf) ? 2 : 0);
+  // a tree in rounds adds its rounds' launches when it is read back
+  h->last_launches = 1 + (h->rounds ? 2 : h->cfg.persistent_grow ? 1 : 2 * (L - 1) + (c.defer ? 1 : 0)) +
+                     ((mode == LGBM_B200_HIST_QUANT && h->cfg.quant_train_renew_leaf) ? 2 : 0);
   return Status();
 }
 
@@ -525,23 +629,19 @@ Status dp_allreduce(LgbmB200Learner* h, void* buf, int64_t count, int32_t dtype,
   return Status();
 }
 
-static Status launch_scan(LgbmB200Learner* h, bool pdl) {
+static Status launch_scan(LgbmB200Learner* h) {
   const DCtx& c = h->ctx;
   const dim3 g(h->nf, 2, h->K);
   cudaStream_t s = h->stream;
-  if (h->cfg.hist_precision == LGBM_B200_HIST_QUANT && h->scan_warp) {
-    const dim3 gw(h->scan_warp_grid, 1, h->K);
-    if (h->scan_wide)
-      CU(launch_ex(k_scan_warp<kScanWideBlocks>, gw, dim3(kScanThreads), 0, s, pdl, c, (const int32_t*)h->scan_items));
-    else CU(launch_ex(k_scan_warp<2>, gw, dim3(kScanThreads), 0, s, pdl, c, (const int32_t*)h->scan_items));
-  } else if (h->cfg.hist_precision == LGBM_B200_HIST_QUANT) {
-    if (h->scan_wide) CU(launch_ex(k_scan<true, kScanWideBlocks>, g, dim3(kScanThreads), h->scan_smem, s, pdl, c));
-    else CU(launch_ex(k_scan<true, 1>, g, dim3(kScanThreads), h->scan_smem, s, pdl, c));
+  if (h->cfg.hist_precision == LGBM_B200_HIST_QUANT) {
+    if (h->scan_wide) k_scan<true, kScanWideBlocks><<<g, kScanThreads, h->scan_smem, s>>>(c);
+    else k_scan<true, 1><<<g, kScanThreads, h->scan_smem, s>>>(c);
   } else if (h->scan_wide) {
-    CU(launch_ex(k_scan<false, kScanWideBlocks>, g, dim3(kScanThreads), h->scan_smem, s, pdl, c));
+    k_scan<false, kScanWideBlocks><<<g, kScanThreads, h->scan_smem, s>>>(c);
   } else {
-    CU(launch_ex(k_scan<false, 1>, g, dim3(kScanThreads), h->scan_smem, s, pdl, c));
+    k_scan<false, 1><<<g, kScanThreads, h->scan_smem, s>>>(c);
   }
+  CU_LAUNCH();
   return Status();
 }
 
@@ -566,20 +666,21 @@ static Status run_tree_dp(LgbmB200Learner* h) {
   k_dp_root_apply<<<1, 1, 0, s>>>(c, h->dp_f64, h->dp_i64);
   CU_LAUNCH();
   const size_t cells = (size_t)h->total_bins * (mode == LGBM_B200_HIST_QUANT ? 1 : 2);
-  const dim3 hist_grid(h->hist_grid, h->ntiles, 1);
+  const dim3 hist_grid(step_hist_grid(h), h->ntiles, 1);
   for (int step = 0; step < L - 1; ++step) {
     DSlotState ss;
     CU(cudaMemcpyAsync(&ss, d.st, sizeof(ss), cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
     if (ss.done) break;
-    CU(launch_hist(mode, h->hist_ng, hist_grid, h->hist_smem, s, c, h->tiles, h->sub_rows, false, false));
+    CU(launch_hist(mode, h->hist_ng, hist_grid, h->hist_smem, s, c, h->tiles, h->sub_rows, false));
     if (ss.need_find) {  // the smaller leaf's histogram, summed over the ranks
       void* buf = static_cast<char*>(d.hist) + (size_t)ss.s_buf * cells * 8;
       const int32_t dt = mode == LGBM_B200_HIST_QUANT ? LGBM_B200_DT_INT64 : LGBM_B200_DT_FLOAT64;
       if (!(st = dp_allreduce(h, buf, (int64_t)cells, dt, LGBM_B200_OP_SUM)).ok()) return st;
     }
-    if (!(st = launch_scan(h, false)).ok()) return st;
-    CU(launch_ex(k_partition, dim3(h->part_grid, 1, 1), dim3(kPartThreads), 0, s, false, c));
+    if (!(st = launch_scan(h)).ok()) return st;
+    k_partition<<<dim3(h->part_grid, 1, 1), kPartThreads, 0, s>>>(c);
+    CU_LAUNCH();
     CU(cudaMemcpyAsync(&ss, d.st, sizeof(ss), cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
     if (ss.done) break;  // no leaf had a positive gain: the tree is finished
@@ -604,7 +705,7 @@ static Status run_tree(LgbmB200Learner* h) {
   if (h->dp) return run_tree_dp(h);
   cudaStream_t s = h->stream;
   // a cooperative launch is enqueued directly rather than captured
-  const bool graph = h->cfg.use_cuda_graph != 0 && !h->cfg.persistent_grow;
+  const bool graph = h->cfg.use_cuda_graph != 0 && !h->cfg.persistent_grow && !(h->rounds && h->timing);
   const int key = (h->bagging ? 1 : 0) + 2 * h->ctx.bagging + 4 * (h->timing ? 1 : 0);
   if (!graph) return enqueue_tree(h);
   if (h->graph_exec == nullptr || h->graph_key != key) {
@@ -825,13 +926,15 @@ Status train_collect(LgbmB200Learner* h) {
     // phase times seen by the first CTA: histogram, scan, partition, bookkeeping
     for (int i = 0; i < 4; ++i) h->last_ms[i] = (double)ph[i] / 1e6;
   } else if (h->timing) {  // per-kernel-family device time of this tree
-    h->last_step_ms.assign((size_t)3 * (h->L - 1), 0.0f);
-    for (int step = 0; step < h->L - 1; ++step) {
+    const bool rounds = h->rounds;
+    const int steps = rounds ? h->last_rounds : h->L - 1;
+    h->last_step_ms.assign((size_t)3 * steps, 0.0f);
+    for (int step = 0; step < steps; ++step) {
       cudaEvent_t* ev = &h->ev[(size_t)4 * step];
-      float a, b, d;
-      CU(cudaEventElapsedTime(&a, ev[0], ev[1]));
-      CU(cudaEventElapsedTime(&b, ev[1], ev[2]));
-      CU(cudaEventElapsedTime(&d, ev[2], ev[3]));
+      float a, b, d;  // histogram, scan, partition (which comes first in a round)
+      CU(cudaEventElapsedTime(rounds ? &d : &a, ev[0], ev[1]));
+      CU(cudaEventElapsedTime(rounds ? &a : &b, ev[1], ev[2]));
+      CU(cudaEventElapsedTime(rounds ? &b : &d, ev[2], ev[3]));
       h->last_ms[0] += a;
       h->last_ms[1] += b;
       h->last_ms[2] += d;
@@ -839,6 +942,15 @@ Status train_collect(LgbmB200Learner* h) {
       h->last_step_ms[(size_t)3 * step + 1] = b;
       h->last_step_ms[(size_t)3 * step + 2] = d;
     }
+  }
+  if (h->rounds) {
+    int rounds = 0;
+    for (int k = 0; k < K; ++k) {
+      RoundState rs;
+      std::memcpy(&rs, h->rb_host + (size_t)k * h->rb_slot + h->rb.rs, sizeof(rs));
+      rounds = std::max(rounds, rs.rounds);
+    }
+    h->last_launches += 3 + 4 * rounds;
   }
   h->last_hist_rows = 0;
   h->last_part_rows = 0;
@@ -977,8 +1089,8 @@ Status histogram_of_rows(LgbmB200Learner* h, int slot, const uint32_t* rows, int
   // one slot only: a context whose slot array starts at `slot`
   DCtx c = h->ctx;
   c.slots[0] = h->ctx.slots[slot];
-  dim3 grid(h->hist_grid, h->ntiles, 1);
-  CU(launch_hist(mode, h->hist_ng, grid, h->hist_smem, s, c, h->tiles, h->sub_rows, false, false));
+  dim3 grid(step_hist_grid(h), h->ntiles, 1);
+  CU(launch_hist(mode, h->hist_ng, grid, h->hist_smem, s, c, h->tiles, h->sub_rows, false));
   CU_LAUNCH();
   CU(cudaMemcpyAsync(out, d.hist, cells * 8, cudaMemcpyDeviceToHost, s));
   CU(cudaStreamSynchronize(s));
@@ -1262,6 +1374,7 @@ int lgbm_b200_learner_set_data_parallel(LgbmB200Learner* h, int64_t row_offset, 
   h->ctx.slots[0] = d;
   h->ctx.dp = 1;
   h->ctx.defer = 0;  // the step's end waits for the left count summed over the ranks
+  h->rounds = false;  // step by step: the ranks reduce between a step's launches
   h->scan_part = false;
   h->cfg.persistent_grow = 0;
   h->cfg.use_cuda_graph = 0;

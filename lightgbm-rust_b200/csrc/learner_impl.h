@@ -251,7 +251,6 @@ struct LgbmB200Learner {
   DTileTable tiles{};
   int ntiles = 1;
   int hist_ng = 1;  // 32-feature groups per histogram tile
-  int use_pdl = 0;  // kernel edges chained by programmatic dependent launch (bits: histogram, scan, partition)
   int grow_grid = 0;       // CTAs of the persistent grow launch
   size_t grow_smem = 0;
   GrowSync* grow_sync = nullptr;
@@ -288,7 +287,7 @@ struct LgbmB200Learner {
   // per slot, at the offsets in rb), so that one copy into the pinned mirror
   // reads a whole tree set back.
   struct ReadbackLayout {
-    size_t st, sfi, sf, sg, tib, dt, lc, rc, lp, lv, lw, lcnt, ld, iv, iw, ic, cb, ng;
+    size_t st, rs, sfi, sf, sg, tib, dt, lc, rc, lp, lv, lw, lcnt, ld, iv, iw, ic, cb, ng;
   } rb{};
   unsigned char* rb_dev = nullptr;
   unsigned char* rb_host = nullptr;
@@ -311,12 +310,6 @@ struct LgbmB200Learner {
   int64_t last_hist_rows = 0;
   int64_t last_part_rows = 0;
   bool scan_wide = false;  // the register-capped scan variant (many CTAs per step)
-  // the quantized scan by one warp per (feature, side): the item of each
-  // warp of each CTA (feature * 2 + side, -1 none; at most one categorical
-  // item per CTA) and the CTAs per slot
-  bool scan_warp = false;
-  int32_t* scan_items = nullptr;
-  int scan_warp_grid = 0;
   bool scan_part = false;  // scans and partition of a step in one cooperative launch
   int scan_part_grid = 0;
   int scan_part_max = 0;  // CTAs of that launch resident at once, shared by the slots
@@ -327,6 +320,13 @@ struct LgbmB200Learner {
   // changes (launch shape, bagging): graphs captured before it are stale
   int config_epoch = 0;
   int32_t last_launches = 0;
+  // growth in rounds (round_kernels.cuh)
+  bool rounds = false;
+  cudaStream_t body_stream = nullptr;  // captures the body of the rounds' loop
+  int32_t* round_ctrl = nullptr;       // [3]: slots arrived, slots going on, whether another round runs
+  int round_scan_grid = 0;
+  size_t round_scan_smem = 0;
+  int last_rounds = 0;
   // captured tree growth
   cudaGraphExec_t graph_exec = nullptr;
   int graph_key = -1;
@@ -339,6 +339,7 @@ struct LgbmB200Learner {
     chunks.release();
     if (start_h) cudaFreeHost(start_h);
     if (rb_host) cudaFreeHost(rb_host);
+    if (body_stream) cudaStreamDestroy(body_stream);
     if (stream) cudaStreamDestroy(stream);
   }
 };

@@ -62,6 +62,44 @@ __device__ bool before_find_best_split(const DCtx& c, const DSlot& s, int32_t le
   return true;
 }
 
+// The root as node 0 of a tree grown in rounds; one thread.
+__device__ void round_init(const DCtx& c, const DSlot& s, int32_t need) {
+  const DRounds& r = s.r;
+  const DSlotState* st = s.st;
+  RNode nd;
+  nd.parent = -1;
+  nd.begin = 0;
+  nd.count = st->num_used;
+  nd.side = 0;
+  nd.depth = 0;
+  nd.buf = 0;
+  nd.need = need;
+  nd.pad = 0;
+  nd.ls = st->smaller;
+  nd.ls.weight = 0.0;
+  nd.cmin = s.cmin[0];
+  nd.cmax = s.cmax[0];
+  r.node[0] = nd;
+  r.gain[0] = -INFINITY;
+  r.feat[0] = -1;
+  r.exp[0] = -1;
+  r.leaf_node[0] = 0;
+  r.scan_cnt[0] = 0;
+  RoundState* rs = r.st;
+  rs->e0 = 0;
+  rs->nb = 0;
+  rs->ntiles = 0;
+  rs->ticket = 0;
+  rs->popped = 0;
+  rs->done = 0;
+  rs->root = 1;
+  rs->rounds = 0;
+  rs->ncopy = 0;
+  rs->ncand = 0;
+  rs->nfree = r.pool - 1;
+  rs->root_value = s.tree.leaf_value[0];
+}
+
 // Grid (kRootBlocks, 1, slots), 256 threads.
 __global__ void __launch_bounds__(256) k_tree_init(const __grid_constant__ DCtx c, const uint32_t* bag, const int32_t* n_used) {
   const DSlot& s = c.slots[blockIdx.z];
@@ -193,6 +231,9 @@ __global__ void __launch_bounds__(256) k_tree_init(const __grid_constant__ DCtx 
     s.leaf_side[l] = 0;
   }
   for (int f = tid; f < c.num_features; f += blockDim.x) s.splittable[f] = 1;
+  if (s.r.st) {  // buffer 0 is the root's; the lowest free one is taken first
+    for (int i = tid; i < s.r.pool - 1; i += blockDim.x) s.r.free[i] = s.r.pool - 1 - i;
+  }
   __syncthreads();
   if (tid != 0) return;
   *s.root_counter = 0;
@@ -237,6 +278,7 @@ __global__ void __launch_bounds__(256) k_tree_init(const __grid_constant__ DCtx 
   t.leaf_count[0] = 0;
   t.leaf_depth[0] = 0;
   st->need_find = before_find_best_split(c, s, 0, -1) ? 1 : 0;
+  if (s.r.st) round_init(c, s, st->need_find);
 }
 
 // =====================================================================================
@@ -771,8 +813,6 @@ template <int kMode, int kNG>
 __global__ void __cluster_dims__(hist_cluster(kMode), 1, 1) __launch_bounds__(kHistThreads, 2)
     k_hist(const __grid_constant__ DCtx c, DTileTable tt, int32_t sub_rows, int32_t lead) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  pdl_wait();
-  pdl_trigger();
   const DSlot& s = c.slots[blockIdx.z];
   if ((int)blockIdx.x < lead) {
     if (blockIdx.x == 0 && blockIdx.y == 0) deferred_finish(c, s, smem_raw);
@@ -818,16 +858,12 @@ const void* hist_kernel(int mode, int ng) {
 }
 
 cudaError_t launch_hist(int mode, int ng, dim3 grid, size_t smem, cudaStream_t st, const DCtx& c, const DTileTable& tt,
-                        int32_t sub_rows, bool pdl, bool finish) {
+                        int32_t sub_rows, bool finish) {
   // the step-end CTA leads as one whole cluster, so the row CTAs' clusters keep their alignment
-  const int32_t lead = finish ? hist_cluster(mode) : 0;
+  int32_t lead = finish ? hist_cluster(mode) : 0;
   grid.x += (unsigned)lead;
-  if (mode == 0) return launch_ex(k_hist<0, 1>, grid, dim3(kHistThreads), smem, st, pdl, c, tt, sub_rows, lead);
-  if (mode == 1) return launch_ex(k_hist<1, 1>, grid, dim3(kHistThreads), smem, st, pdl, c, tt, sub_rows, lead);
-  if (ng == 1) return launch_ex(k_hist<2, 1>, grid, dim3(kHistThreads), smem, st, pdl, c, tt, sub_rows, lead);
-  if (ng == 2) return launch_ex(k_hist<2, 2>, grid, dim3(kHistThreads), smem, st, pdl, c, tt, sub_rows, lead);
-  if (ng == 3) return launch_ex(k_hist<2, 3>, grid, dim3(kHistThreads), smem, st, pdl, c, tt, sub_rows, lead);
-  return launch_ex(k_hist<2, 4>, grid, dim3(kHistThreads), smem, st, pdl, c, tt, sub_rows, lead);
+  void* args[] = {const_cast<DCtx*>(&c), const_cast<DTileTable*>(&tt), &sub_rows, &lead};
+  return cudaLaunchKernel(hist_kernel(mode, ng), grid, dim3(kHistThreads), args, smem, st);
 }
 
 // =====================================================================================
@@ -865,8 +901,9 @@ __device__ __forceinline__ int32_t warp_min_i(int32_t v) {
 // split.rs:448-670 / :1194-1400 categorical threshold search, in lane 0
 // (the candidate lists are at most a few dozen bins; the stable sort is a
 // rank sort done by the whole warp).
-template <bool kInt>
-__device__ __noinline__ bool scan_categorical(ScanSmem& sm, const DFeature& m, const DParams& p, const LeafCtx& lc, DSplit& out) {
+template <bool kInt, class Scratch>
+__device__ __noinline__ bool scan_categorical(Scratch& sm, const DFeature& m, const DParams& p, const LeafCtx& lc,
+                                              DSplit& out) {
   const int lane = threadIdx.x & 31;
   const int offset = m.offset;
   const int bin_start = 1 - offset, bin_end = m.num_bin - offset;
@@ -875,10 +912,21 @@ __device__ __noinline__ bool scan_categorical(ScanSmem& sm, const DFeature& m, c
   double sum_gradient = kInt ? (double)int_grad(lc.int_sum) * gs : lc.sum_g;
   double sum_hessian = kInt ? (double)int_hess(lc.int_sum) * hs : lc.sum_h;
   const double cnt_factor = kInt ? (double)lc.num_data / (double)int_hess(lc.int_sum) : (double)lc.num_data / lc.sum_h;
-  auto G = [&](int t) { return kInt ? (double)int_grad(sm.ig[t]) * gs : sm.g[t]; };
-  auto H = [&](int t) { return kInt ? (double)int_hess(sm.ig[t]) * hs : sm.h[t]; };
+  auto G = [&](int t) {
+    if constexpr (kInt) return (double)int_grad(sm.ig[t]) * gs;
+    else return sm.g[t];
+  };
+  auto H = [&](int t) {
+    if constexpr (kInt) return (double)int_hess(sm.ig[t]) * hs;
+    else return sm.h[t];
+  };
   auto CNT = [&](int t) {
-    return kInt ? round_int((double)int_hess(sm.ig[t]) * cnt_factor) : round_int(sm.h[t] * cnt_factor);
+    if constexpr (kInt) return round_int((double)int_hess(sm.ig[t]) * cnt_factor);
+    else return round_int(sm.h[t] * cnt_factor);
+  };
+  auto Q = [&](int t) {
+    if constexpr (kInt) return (int64_t)sm.ig[t];
+    else return (int64_t)0;
   };
   int32_t used_bin = 0;
   if (!use_onehot) {
@@ -925,7 +973,7 @@ __device__ __noinline__ bool scan_categorical(ScanSmem& sm, const DFeature& m, c
         if (other_count < p.min_data_in_leaf) continue;
         double soh, sog;
         if (kInt) {
-          int64_t other = (int64_t)((uint64_t)lc.int_sum - (uint64_t)sm.ig[t]);
+          int64_t other = (int64_t)((uint64_t)lc.int_sum - (uint64_t)Q(t));
           soh = (double)int_hess(other) * hs;
           if (soh < p.min_sum_hessian_in_leaf) continue;
           sog = (double)int_grad(other) * gs;
@@ -943,7 +991,7 @@ __device__ __noinline__ bool scan_categorical(ScanSmem& sm, const DFeature& m, c
           best_slg = grad;
           best_slh = kInt ? hess : hess + kEpsilon;
           best_left_count = cnt;
-          best_left_int = kInt ? sm.ig[t] : 0;
+          best_left_int = Q(t);
           best_gain = gain;
         }
       }
@@ -962,7 +1010,7 @@ __device__ __noinline__ bool scan_categorical(ScanSmem& sm, const DFeature& m, c
           int32_t cnt = CNT(t);
           double srh, srg, slh_eff;
           if (kInt) {
-            sl_int = (int64_t)((uint64_t)sl_int + (uint64_t)sm.ig[t]);
+            sl_int = (int64_t)((uint64_t)sl_int + (uint64_t)Q(t));
             left_count += cnt;
             cnt_cur_group += cnt;
             slh_eff = (double)int_hess(sl_int) * hs;
@@ -1517,33 +1565,52 @@ __device__ void apply_split(const DCtx& c, const DSlot& s, int32_t bl, int32_t R
   st->num_leaves_cur = R + 1;
 }
 
-// Threshold scan of feature f for one leaf side (0: smaller, 1: larger) of
-// slot s, by the whole CTA (at least kScanThreads threads): the leaf's view
-// is fixed (histogram.rs:42-56), the larger leaf's is formed as parent -
-// smaller (histogram.rs:59-63) and stored, and the best threshold is written
-// to feat_res / feat_ok.
-template <bool kInt>
-__device__ void scan_item(const DCtx& c, const DSlot& s, int f, int side, ScanSmem& sm) {
-  DSlotState* st = s.st;
+// One threshold scan: a leaf side (0: smaller, 1: larger) of a split's two
+// new leaves (or the root, side 0), and where its result goes.
+struct ScanJob {
+  DLeafSplits sl;     // the smaller leaf
+  DLeafSplits ls;     // the leaf scanned
+  int32_t s_buf, l_buf;  // histogram buffers of the smaller and (the parent's) of the larger leaf
+  bool live;          // this side has a leaf to search
+  bool root;          // the root's scan
+  double cmin, cmax;
+  double gsc, hsc;    // quantized gradients' scales
+  DSplit* out;
+};
+
+__device__ __forceinline__ LeafCtx leaf_ctx(const DCtx& c, const ScanJob& j) {
+  LeafCtx lc;
+  lc.sum_g = j.ls.sum_gradients;
+  lc.sum_h = j.ls.sum_hessians;
+  lc.int_sum = j.ls.int_sum;
+  lc.gs = j.gsc;
+  lc.hs = j.hsc;
+  lc.num_data = j.ls.num_data;
+  // learner/mod.rs:1303-1309 parent output
+  lc.parent_output =
+      j.root ? root_output(j.ls.sum_gradients, j.ls.sum_hessians, c.p, j.ls.num_data) : j.ls.weight;
+  lc.mc = c.p.use_monotone != 0;
+  lc.cmin = j.cmin;
+  lc.cmax = j.cmax;
+  return lc;
+}
+
+// The scan of feature f by the whole CTA (at least kScanThreads threads):
+// the leaf's view is fixed (histogram.rs:42-56), the larger leaf's is formed
+// as parent - smaller (histogram.rs:59-63) and stored, and the best threshold
+// is stored to j.out (also left in sm.out). `flags` is loaded with the
+// histogram and says whether the feature is searched at all; returns whether
+// a candidate was splittable (thread-uniform), `ran` whether it was searched.
+template <bool kInt, class Flags>
+__device__ __forceinline__ bool scan_block(const DCtx& c, const DSlot& s, int f, int side, const DFeature& m,
+                                           const ScanJob& j, ScanSmem& sm, Flags flags, bool& ran) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const DFeature m = c.feats[f];
   const DParams& p = c.p;
-  const int32_t nf = c.num_features;
-  // The loads run in two waves so that their latencies overlap: the slot
-  // state, then everything that depends on it (the feature's flags, both
-  // histogram views, the leaf's output bounds).
-  const int32_t larger_leaf = st->larger.leaf, L = st->left_leaf, s_buf = st->s_buf, l_buf = st->l_buf;
-  const bool need = st->need_find != 0 && st->done == 0;
-  const int32_t nl_cur = st->num_leaves_cur;
-  const DLeafSplits sl = st->smaller;
-  const DLeafSplits ls = side == 0 ? sl : st->larger;
-  const double gsc = st->grad_scale, hsc = st->hess_scale;
-  const bool have_larger = larger_leaf >= 0;
-  // the buffers and the leaf are valid whenever this side has a leaf to search
-  const bool live = need && (side == 0 || have_larger);
+  const bool live = j.live;
+  const DLeafSplits& sl = j.sl;
   const int len = m.view_len;
-  const size_t sbase = (size_t)s_buf * c.total_bins + m.view_start;
-  const size_t lbase = (size_t)l_buf * c.total_bins + m.view_start;
+  const size_t sbase = (size_t)j.s_buf * c.total_bins + m.view_start;
+  const size_t lbase = (size_t)j.l_buf * c.total_bins + m.view_start;
   const bool in_view = live && tid < len;
   const bool sub = side == 1 && in_view;
   // histogram cells are written by other CTAs' atomics: loaded through L2
@@ -1564,10 +1631,8 @@ __device__ void scan_item(const DCtx& c, const DSlot& s, int f, int side, ScanSm
       phv = __ldcg(hs + 2 * (lbase + tid) + 1);
     }
   }
-  const uint8_t in_tree = s.bytree[f];
-  const uint8_t split_ok = have_larger ? s.splittable[L * nf + f] : (uint8_t)1;
-  const double cmin = live ? s.cmin[ls.leaf] : 0.0, cmax = live ? s.cmax[ls.leaf] : 0.0;
-  if (!(live && in_tree && split_ok)) return;
+  ran = flags() && live;
+  if (!ran) return false;
   {
     // the smaller leaf's view with its most frequent bin fixed (histogram.rs:42-56)
     if (kInt) {
@@ -1640,337 +1705,69 @@ __device__ void scan_item(const DCtx& c, const DSlot& s, int f, int side, ScanSm
       }
       __syncthreads();
     }
-    LeafCtx lc;
-    lc.sum_g = ls.sum_gradients;
-    lc.sum_h = ls.sum_hessians;
-    lc.int_sum = ls.int_sum;
-    lc.gs = gsc;
-    lc.hs = hsc;
-    lc.num_data = ls.num_data;
-    // learner/mod.rs:1303-1309 parent output
-    lc.parent_output = nl_cur == 1 ? root_output(ls.sum_gradients, ls.sum_hessians, p, ls.num_data) : ls.weight;
-    lc.mc = p.use_monotone != 0;
-    lc.cmin = cmin;
-    lc.cmax = cmax;
+    const LeafCtx lc = leaf_ctx(c, j);
     // the result is built in shared memory and stored once
     DSplit& out = sm.out;
-    bool ok = find_best_threshold_block<kInt>(sm, m, p, lc, out);
+    const bool ok = find_best_threshold_block<kInt>(sm, m, p, lc, out);
     if (tid == 0) {
       out.feature = m.real_index;
       out.inner = f;
-      s.feat_ok[side * nf + f] = ok ? 1 : 0;
     }
     __syncthreads();
     const uint32_t* src = reinterpret_cast<const uint32_t*>(&out);
-    uint32_t* dst = reinterpret_cast<uint32_t*>(&s.feat_res[side * nf + f]);
+    uint32_t* dst = reinterpret_cast<uint32_t*>(j.out);
     for (int i = tid; i < (int)(sizeof(DSplit) / 4); i += blockDim.x) dst[i] = src[i];
-    // the partition's goes-left table for this candidate, ready if it wins
-    if (ok) build_partition_lut(m, out, s.lut_cand + ((size_t)side * nf + f) * kMaxBins, tid, (int32_t)blockDim.x);
+    return ok;
   }
 }
 
-// =====================================================================================
-// Quantized threshold scan, one warp per (feature, side): the same search as
-// scan_item / find_best_threshold_block / scan_direction_block for packed
-// integer sums, with lane l holding stored bins 8l .. 8l + 7 in registers.
-// Integer cumulative sums are exact in any order, and every per-candidate
-// value comes from the same expressions, so the results are the block
-// version's bit for bit; candidates reduce with the same tie rules. No block
-// barrier is involved, so a CTA runs eight items side by side.
-// =====================================================================================
-
-// One direction of the quantized scan by one warp. vw[32 j + lane] is stored
-// bin 8 * lane + j of the leaf's view (the most frequent bin fixed, the
-// larger leaf's view already formed), in this warp's shared memory.
-__device__ __noinline__ bool scan_direction_warp(const int64_t* vw, const DFeature& m, const DParams& p, const LeafCtx& lc,
-                                    double min_gain_shift, double cnt_factor, bool reverse, bool skip_default,
-                                    bool na_as_missing, DSplit& out) {
-  const int lane = threadIdx.x & 31;
-  const int offset = m.offset;
-  const int len = m.view_len;
-  int32_t t_lo, t_hi;
-  if (reverse) {
-    t_hi = m.num_bin - 1 - offset - (int32_t)na_as_missing;
-    t_lo = 1 - offset;
-  } else {
-    t_lo = 0;
-    t_hi = m.num_bin - 2 - offset;
-  }
-  const int32_t skip_t = skip_default ? m.default_bin - offset : INT32_MIN;
-  auto visited = [&](int t) { return t >= t_lo && t <= t_hi && t != skip_t && t < len; };
-  const bool first_extra = !reverse && na_as_missing && offset == 1;
-  const int32_t nstored = m.num_bin - offset;
-  // cumulative sums in scan order: ascending, the visited bins up to t;
-  // reverse, the visited bins from t up (the total minus those below t)
-  uint64_t pre = 0, all = 0;
-#pragma unroll
-  for (int j = 0; j < kPer; ++j) {
-    const int t = lane * kPer + j;
-    const uint64_t x = (uint64_t)vw[32 * j + lane];
-    if (visited(t)) pre += x;
-    if (first_extra && t < len && t < nstored) all += x;
-  }
-  uint64_t incl = pre;  // inclusive over lanes of this lane's visited sum
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint64_t other = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += other;
-    all += __shfl_xor_sync(0xffffffffu, all, o);
-  }
-  const uint64_t total = __shfl_sync(0xffffffffu, incl, 31);
-  const uint64_t base = first_extra ? (uint64_t)lc.int_sum - all : 0ull;
-  const uint64_t run0 = incl - pre;  // visited bins below this lane's first
-  // visits this lane's visited candidates with their cumulative packed sum
-  // and count estimate, recomputed on each walk (no per-bin arrays live)
-  auto walk = [&](auto fn) {
-    uint64_t run = run0;
-#pragma unroll 1
-    for (int j = 0; j < kPer; ++j) {
-      const int t = lane * kPer + j;
-      const bool vis = visited(t);
-      const uint64_t below = run;  // visited bins below t
-      if (vis) {
-        run += (uint64_t)vw[32 * j + lane];
-        const int64_t q = (int64_t)(reverse ? total - below : base + run);
-        fn(t, round_int((double)int_hess(q) * cnt_factor), q);
-      }
-    }
-  };
-  // the extra candidate t = -1 (lane 0)
-  const int64_t eq = (int64_t)base;
-  const int32_t ec = round_int((double)int_hess(eq) * cnt_factor);
-  const int32_t min_data = p.min_data_in_leaf;
-  const double min_hess = p.min_sum_hessian_in_leaf;
-  const bool plain = plain_split(p, lc.mc);
-  const bool extra = lane == 0 && first_extra;
-  auto hsides = [&](int64_t aq, double& ha, double& hr) {
-    ha = (double)int_hess(aq) * lc.hs;
-    hr = (double)int_hess((int64_t)((uint64_t)lc.int_sum - (uint64_t)aq)) * lc.hs;
-  };
-  // pass 1: the first break in scan order
-  int32_t brk = reverse ? INT32_MIN : INT32_MAX;
-  auto break_at = [&](int t, int32_t ac, int64_t aq) {
-    double ha, hr;
-    hsides(aq, ha, hr);
-    const bool skip1 = ac < min_data || ha < min_hess;
-    if (!skip1 && (lc.num_data - ac < min_data || hr < min_hess)) brk = reverse ? max(brk, t) : min(brk, t);
-  };
-  walk(break_at);
-  if (extra) break_at(-1, ec, eq);
-  for (int o = 16; o > 0; o >>= 1) {
-    const int32_t ob = __shfl_xor_sync(0xffffffffu, brk, o);
-    brk = reverse ? max(brk, ob) : min(brk, ob);
-  }
-  // pass 2: gains of the candidates before the break
-  double best_gain = -INFINITY;
-  int32_t best_t = INT32_MIN;
-  bool splittable = false;
-  int64_t wq = 0;  // this lane's best candidate's cumulative values
-  int32_t wc = 0;
-  auto consider = [&](int t, int32_t ac, int64_t aq) {
-    if (t >= 0 ? (reverse ? t <= brk : t >= brk) : !(brk > -1)) return;
-    double ha, hr;
-    hsides(aq, ha, hr);
-    if (ac < min_data || ha < min_hess) return;
-    const int64_t rest = (int64_t)((uint64_t)lc.int_sum - (uint64_t)aq);
-    const double ga = (double)int_grad(aq) * lc.gs, gr = (double)int_grad(rest) * lc.gs;
-    ha += kEpsilon;
-    hr += kEpsilon;
-    const int32_t rc = lc.num_data - ac;
-    // the left child is the rest when scanning in reverse
-    const double g1 = reverse ? gr : ga, h1 = reverse ? hr : ha, g2 = reverse ? ga : gr, h2 = reverse ? ha : hr;
-    const int32_t c1 = reverse ? rc : ac, c2 = reverse ? ac : rc;
-    const double gain = split_gain_hot(plain, g1, h1, g2, h2, p, c1, c2, lc.parent_output, lc.mc, lc.cmin, lc.cmax,
-                                       m.monotone_type);
-    if (gain <= min_gain_shift) return;
-    splittable = true;
-    if (gain > best_gain || (gain == best_gain && best_t != INT32_MIN && (reverse ? t > best_t : t < best_t))) {
-      best_gain = gain;
-      best_t = t;
-      wq = aq;
-      wc = ac;
-    }
-  };
-  walk(consider);
-  if (extra) consider(-1, ec, eq);
-  warp_pick(reverse, best_gain, best_t);
-  const bool any = __any_sync(0xffffffffu, splittable);
-  ScanBest r;
-  r.splittable = any;
-  r.gain = best_gain;
-  r.t = best_t;
-  r.acc_g = r.acc_h = 0.0;
-  // the winner's cumulative values, from the lane whose best it was (the
-  // extra candidate t = -1 is lane 0's)
-  const int src = best_t >= 0 ? best_t / kPer : 0;
-  wq = (int64_t)__shfl_sync(0xffffffffu, (unsigned long long)wq, src);
-  wc = __shfl_sync(0xffffffffu, wc, src);
-  r.acc_q = best_t == INT32_MIN ? 0 : wq;
-  r.acc_c = best_t == INT32_MIN ? 0 : wc;
-  apply_direction<true>(r, m, p, lc.sum_g, lc.sum_h, lc.int_sum, lc.gs, lc.hs, lc.num_data, lc.parent_output, lc.mc,
-                        lc.cmin, lc.cmax, min_gain_shift, cnt_factor, reverse, out);
-  __syncwarp();
-  return any;
-}
-
-// find_best_threshold (split.rs:246-271, :930-950) of the quantized form for
-// one leaf and feature, by one warp; cat: the CTA's scratch, for a
-// categorical feature (its view is copied there first).
-__device__ bool find_best_threshold_warp(const int64_t* vw, ScanSmem* cat, const DFeature& m,
-                                         const DParams& p, const LeafCtx& lc, DSplit& out) {
-  const int lane = threadIdx.x & 31;
-  if (lane == 0) {
-    out.default_left = 1;
-    out.gain = -INFINITY;
-    out.num_cat = 0;
-    out.monotone_type = 0;
-  }
-  __syncwarp();
-  bool ok = false;
-  if (m.bin_type == 1) {
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) cat->ig[lane * kPer + j] = vw[32 * j + lane];
-    __syncwarp();
-    ok = scan_categorical<true>(*cat, m, p, lc, out);
-  } else {
-    if (lane == 0) out.monotone_type = m.monotone_type;
-    const double sg = (double)int_grad(lc.int_sum) * lc.gs;
-    const double sh = (double)int_hess(lc.int_sum) * lc.hs;
-    const double min_gain_shift =
-        leaf_gain_hot(plain_split(p, lc.mc), sg, sh, p, lc.num_data, lc.parent_output) + p.min_gain_to_split;
-    const double cnt_factor = (double)lc.num_data / (double)int_hess(lc.int_sum);
-    // split.rs:426-439: the directions scanned and their missing-value rules
-    const bool two = m.num_bin > 2 && m.missing_type != 0;
-    const bool skip_default = two && m.missing_type == 1;
-    const bool na_missing = two && m.missing_type == 2;
-#pragma unroll 1
-    for (int d = 0; d < (two ? 2 : 1); ++d)
-      ok |= scan_direction_warp(vw, m, p, lc, min_gain_shift, cnt_factor, d == 0, skip_default, na_missing, out);
-    if (!two && lane == 0 && m.missing_type == 2) out.default_left = 0;
-  }
-  __syncwarp();
-  if (lane == 0) out.gain *= m.penalty;
-  __syncwarp();
-  return ok;
-}
-
-// scan_item for the quantized form by one warp: feature f, side (0 smaller,
-// 1 larger) of slot s. vw: this warp's view in shared memory ([kPer][32]);
-// out: its result in shared memory.
-__device__ void scan_item_warp(const DCtx& c, const DSlot& s, int f, int side, ScanSmem* cat, int64_t* vw,
-                               DSplit& out) {
-  DSlotState* st = s.st;
-  const int lane = threadIdx.x & 31;
-  const DFeature m = c.feats[f];
-  const DParams& p = c.p;
-  const int32_t nf = c.num_features;
-  // two waves of loads, as in the block version: the slot state, then what
-  // depends on it
-  const int32_t larger_leaf = st->larger.leaf, L = st->left_leaf, s_buf = st->s_buf, l_buf = st->l_buf;
+// The scan job of leaf side `side` of the slot's running split step.
+__device__ __forceinline__ ScanJob step_job(const DCtx& c, const DSlot& s, int f, int side, int32_t& larger_leaf,
+                                            int32_t& L) {
+  const DSlotState* st = s.st;
+  ScanJob j;
+  larger_leaf = st->larger.leaf;
+  L = st->left_leaf;
+  j.s_buf = st->s_buf;
+  j.l_buf = st->l_buf;
   const bool need = st->need_find != 0 && st->done == 0;
-  const int32_t nl_cur = st->num_leaves_cur;
-  const DLeafSplits sl = st->smaller;
-  const DLeafSplits ls = side == 0 ? sl : st->larger;
-  const double gsc = st->grad_scale, hsc = st->hess_scale;
-  const bool have_larger = larger_leaf >= 0;
-  const bool live = need && (side == 0 || have_larger);
-  const int len = m.view_len;
-  const size_t sbase = (size_t)s_buf * c.total_bins + m.view_start;
-  const size_t lbase = (size_t)l_buf * c.total_bins + m.view_start;
-  const long long* hsrc = reinterpret_cast<const long long*>(s.hist);
-  int64_t v[kPer], pv[kPer];
-#pragma unroll
-  for (int j = 0; j < kPer; ++j) {
-    const int i = lane * kPer + j;
-    // histogram cells are written by other CTAs' atomics: loaded through L2
-    v[j] = (live && i < len) ? (int64_t)__ldcg(hsrc + sbase + i) : 0;
-    pv[j] = (live && side == 1 && i < len) ? (int64_t)__ldcg(hsrc + lbase + i) : 0;
-  }
-  const uint8_t in_tree = s.bytree[f];
-  const uint8_t split_ok = have_larger ? s.splittable[L * nf + f] : (uint8_t)1;
-  const double cmin = live ? s.cmin[ls.leaf] : 0.0, cmax = live ? s.cmax[ls.leaf] : 0.0;
-  if (!(live && in_tree && split_ok)) return;
-  int64_t* hdst = reinterpret_cast<int64_t*>(s.hist);
-  // the smaller leaf's view with its most frequent bin fixed (histogram.rs:42-56; exact in any order)
-  if (m.most_freq_bin > 0) {
-    uint64_t part = 0;
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-      const int i = lane * kPer + j;
-      if (i < m.num_bin && i != m.most_freq_bin) part += (uint64_t)v[j];
-    }
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    const int64_t fixed = (int64_t)((uint64_t)sl.int_sum - part);
-#pragma unroll
-    for (int j = 0; j < kPer; ++j)
-      if (lane * kPer + j == m.most_freq_bin) {
-        v[j] = fixed;
-        if (side == 0) hdst[sbase + m.most_freq_bin] = fixed;
-      }
-  }
-  if (side == 1) {  // larger = parent - smaller, in the parent's buffer (histogram.rs:59-63)
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-      const int i = lane * kPer + j;
-      if (i < len) {
-        v[j] = (int64_t)((uint64_t)pv[j] - (uint64_t)v[j]);
-        hdst[lbase + i] = v[j];
-      }
-    }
-  }
-  LeafCtx lc;
-  lc.sum_g = ls.sum_gradients;
-  lc.sum_h = ls.sum_hessians;
-  lc.int_sum = ls.int_sum;
-  lc.gs = gsc;
-  lc.hs = hsc;
-  lc.num_data = ls.num_data;
-  // learner/mod.rs:1303-1309 parent output
-  lc.parent_output = nl_cur == 1 ? root_output(ls.sum_gradients, ls.sum_hessians, p, ls.num_data) : ls.weight;
-  lc.mc = p.use_monotone != 0;
-  lc.cmin = cmin;
-  lc.cmax = cmax;
-#pragma unroll
-  for (int j = 0; j < kPer; ++j) vw[32 * j + lane] = v[j];
-  __syncwarp();
-  const bool ok = find_best_threshold_warp(vw, cat, m, p, lc, out);
-  if (lane == 0) {
-    out.feature = m.real_index;
-    out.inner = f;
-    s.feat_ok[side * nf + f] = ok ? 1 : 0;
-  }
-  __syncwarp();
-  const uint32_t* src = reinterpret_cast<const uint32_t*>(&out);
-  uint32_t* dst = reinterpret_cast<uint32_t*>(&s.feat_res[side * nf + f]);
-  for (int i = lane; i < (int)(sizeof(DSplit) / 4); i += 32) dst[i] = src[i];
-  // the partition's goes-left table for this candidate, ready if it wins
-  if (ok) build_partition_lut(m, out, s.lut_cand + ((size_t)side * nf + f) * kMaxBins, lane, 32);
+  j.root = st->num_leaves_cur == 1;
+  j.sl = st->smaller;
+  j.ls = side == 0 ? j.sl : st->larger;
+  j.gsc = st->grad_scale;
+  j.hsc = st->hess_scale;
+  // the buffers and the leaf are valid whenever this side has a leaf to search
+  j.live = need && (side == 0 || larger_leaf >= 0);
+  j.cmin = j.live ? s.cmin[j.ls.leaf] : 0.0;
+  j.cmax = j.live ? s.cmax[j.ls.leaf] : 0.0;
+  j.out = &s.feat_res[side * c.num_features + f];
+  return j;
 }
 
-// Grid (CTAs, 1, slots), kScanThreads threads: warp w of CTA b scans item
-// items[8b + w] (feature * 2 + side, or -1 for none) of slot z. The host
-// gives each CTA at most one categorical item, which uses the CTA's scratch.
-template <int kMinBlocks>
-__global__ void __launch_bounds__(kScanThreads, kMinBlocks) k_scan_warp(const __grid_constant__ DCtx c,
-                                                                        const int32_t* items) {
-  __shared__ ScanSmem cat;
-  __shared__ DSplit outs[kScanThreads / 32];
-  __shared__ int64_t views[kScanThreads / 32][kPer * 32];
-  pdl_wait();
-  pdl_trigger();
-  const DSlot& s = c.slots[blockIdx.z];
-  DSlotState* st = s.st;
-  const int warp = threadIdx.x >> 5;
-  // the partition that follows claims its row tiles from this counter
-  if (blockIdx.x == 0 && threadIdx.x == 0 && !st->done) {
-    st->part_ticket = 0;
-    st->part_done = 0;
-  }
-  const int32_t it = items[blockIdx.x * (kScanThreads / 32) + warp];
-  if (it < 0) return;
-  scan_item_warp(c, s, it >> 1, it & 1, &cat, views[warp], outs[warp]);
+// Threshold scan of feature f for one leaf side (0: smaller, 1: larger) of
+// slot s's running split step, by the whole CTA: the best threshold is
+// written to feat_res / feat_ok.
+template <bool kInt>
+__device__ void scan_item(const DCtx& c, const DSlot& s, int f, int side, ScanSmem& sm) {
+  const int tid = threadIdx.x;
+  const DFeature m = c.feats[f];
+  const int32_t nf = c.num_features;
+  // The loads run in two waves so that their latencies overlap: the slot
+  // state, then everything that depends on it (the feature's flags, both
+  // histogram views, the leaf's output bounds).
+  int32_t larger_leaf, L;
+  const ScanJob j = step_job(c, s, f, side, larger_leaf, L);
+  bool ran;
+  const bool ok = scan_block<kInt>(c, s, f, side, m, j, sm, [&] {
+    const uint8_t in_tree = s.bytree[f];
+    const uint8_t split_ok = larger_leaf >= 0 ? s.splittable[L * nf + f] : (uint8_t)1;
+    return in_tree && split_ok;
+  }, ran);
+  if (!ran) return;
+  if (tid == 0) s.feat_ok[side * nf + f] = ok ? 1 : 0;
+  // the partition's goes-left table for this candidate, ready if it wins
+  if (ok) build_partition_lut(m, sm.out, s.lut_cand + ((size_t)side * nf + f) * kMaxBins, tid, (int32_t)blockDim.x);
 }
-template __global__ void k_scan_warp<2>(const __grid_constant__ DCtx, const int32_t*);
-template __global__ void k_scan_warp<kScanWideBlocks>(const __grid_constant__ DCtx, const int32_t*);
 
 // kMinBlocks: CTAs the compiler keeps resident per SM (registers capped to
 // fit). 1 for a step of few features, where each CTA's latency is what counts;
@@ -1980,8 +1777,6 @@ template __global__ void k_scan_warp<kScanWideBlocks>(const __grid_constant__ DC
 template <bool kInt, int kMinBlocks>
 __global__ void __launch_bounds__(kScanThreads, kMinBlocks) k_scan(const __grid_constant__ DCtx c) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  pdl_wait();
-  pdl_trigger();
   const DSlot& s = c.slots[blockIdx.z];
   DSlotState* st = s.st;
   // the partition that follows claims its row tiles from this counter
@@ -2370,12 +2165,12 @@ __device__ SplitLeaf partition_prologue(const DCtx& c, const DSlot& s, const Ste
 // One partition tile after its goes-left flags are known: a block scan of
 // the per-thread left counts, the decoupled look-back for the tile's prefix,
 // then the scatter (left rows ascending from the range start, right rows
-// descending from its end). The CTA of the last tile posts the left count.
-template <int kItems>
-__device__ void tile_scatter(const DSlot& s, PartShared& ps, int32_t tile, int32_t ntiles, uint32_t epoch, int32_t t0,
-                             int32_t cnt, const uint32_t (&rows)[kItems], uint32_t flags, int32_t nleft,
-                             uint32_t* out) {
-  DSlotState* st = s.st;
+// descending from its end). stat: the look-back words of the leaf's tiles.
+// Returns the left rows up to and including this tile.
+template <int kItems, class Shared>
+__device__ int32_t tile_scatter(DSlotState* st, Shared& ps, unsigned long long* stat, int32_t tile, uint32_t epoch,
+                                int32_t t0, int32_t cnt, const uint32_t (&rows)[kItems], uint32_t flags,
+                                int32_t nleft, uint32_t* out) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // block exclusive scan of per-thread left counts
     int32_t incl = nleft;
@@ -2394,7 +2189,6 @@ __device__ void tile_scatter(const DSlot& s, PartShared& ps, int32_t tile, int32
     // decoupled look-back on the left count: warp 0 reads 32 predecessors at a
     // time and sums back to the nearest one whose inclusive prefix is posted
     if (warp == 0) {
-      unsigned long long* stat = s.tile_status;
       if (tile == 0) {
         if (lane == 0) {
           atomicExch(&stat[0], pack_status(epoch, kFlagInc, (uint64_t)tile_left));
@@ -2458,7 +2252,7 @@ __device__ void tile_scatter(const DSlot& s, PartShared& ps, int32_t tile, int32
         }
       }
     }
-    if (tile == ntiles - 1 && tid == 0) st->part_left = prefix + tile_left;
+    return prefix + tile_left;
 }
 
 // Row tiles of the split leaf L claimed in order by the CTAs (kItems rows
@@ -2514,7 +2308,8 @@ __device__ void partition_rows(const DCtx& c, const DSlot& s, PartShared& ps, co
         ++nleft;
       }
     }
-    tile_scatter<kItems>(s, ps, tile, ntiles, epoch, t0, cnt, rows, flags, nleft, out);
+    const int32_t lefts = tile_scatter<kItems>(st, ps, s.tile_status, tile, epoch, t0, cnt, rows, flags, nleft, out);
+    if (tile == ntiles - 1 && tid == 0) st->part_left = lefts;
   }
 }
 
@@ -2631,8 +2426,6 @@ __global__ void k_dp_root_apply(const __grid_constant__ DCtx c, const double* f,
 // step's split decision and the goes-left LUT, then claims row tiles; the
 // last CTA to exit ends the step.
 __global__ void __launch_bounds__(kPartThreads) k_partition(const __grid_constant__ DCtx c) {
-  pdl_wait();
-  pdl_trigger();
   const DSlot& s = c.slots[blockIdx.z];
   __shared__ PartShared ps;
   // the step's fields and this CTA's first row tile, in one round trip (a
@@ -3161,5 +2954,7 @@ cudaError_t launch_grow(int mode, int ng, int grid, size_t smem, cudaStream_t st
   void* args[] = {const_cast<DCtx*>(&c), const_cast<DTileTable*>(&tt), &sub_rows, &ntiles, &gs, &num_steps, &phase_ns};
   return cudaLaunchCooperativeKernel(grow_kernel(mode, ng), dim3(grid), dim3(kGrowThreads), args, smem, st);
 }
+
+#include "round_kernels.cuh"
 
 }  // namespace lgbm_b200
