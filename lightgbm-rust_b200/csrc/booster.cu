@@ -717,15 +717,79 @@ struct LgbmB200Forest {
 };
 
 namespace lgbm_b200 {
+// One tree in the compact layout (predict.h), appended to `out` with a leaf
+// value per node: the nodes in breadth-first order, so that the two children
+// of a node lie side by side. Returns false, for the wide layout, when the
+// tree does not fit it or its child indices are not those of a tree.
+static bool pack_tree(const LgbmB200TreeView& v, int32_t cat_base, std::vector<PNode>& out,
+                      std::vector<double>& leaf_value, std::vector<int4>& tree, int32_t& max_nodes, bool& special) {
+  // a constant tree is a node that leads to its leaf
+  const int32_t nl = v.num_leaves, nn = nl - 1, total = nl > 1 ? 2 * nl - 1 : 2, padded = (total + 1) / 2 * 2;
+  if (nl > kPNodeMaxLeaves) return false;
+  const size_t first = out.size();
+  if (first + (size_t)padded > (size_t)INT32_MAX) return false;
+  out.resize(first + (size_t)padded, PNode{NAN, 0});
+  leaf_value.resize(first + (size_t)padded, 0.0);
+  std::vector<int32_t> child((size_t)total);  // the node or ~leaf at each place
+  int32_t next = 1;
+  if (nn > 0) child[0] = 0;
+  else child[(size_t)next++] = ~0;  // place 0 keeps its NaN threshold and first child 0
+  for (int32_t i = nn > 0 ? 0 : 1; i < next; ++i) {
+    PNode& p = out[first + (size_t)i];
+    if (child[(size_t)i] < 0) {
+      const int32_t leaf = ~child[(size_t)i];
+      if (leaf >= nl) return false;
+      p = PNode{NAN, (uint32_t)(i - 1)};
+      leaf_value[first + (size_t)i] = v.leaf_value[leaf];
+      continue;
+    }
+    const int32_t nd = child[(size_t)i];
+    if (nd >= nn || next + 2 > total) return false;
+    if (v.split_feature[nd] >= (1 << kPNodeFeatureBits)) return false;
+    uint32_t meta = (uint32_t)next | (uint32_t)v.split_feature[nd] << 16;
+    const int8_t dt = v.decision_type[nd];
+    const double thr = v.threshold[nd];
+    const int mt = (dt >> 2) & 3;
+    const bool cat = dt & 1, def = (dt & 2) != 0, at_zero = 0.0 <= thr;
+    const bool nan_left = !cat && (mt == 0 || mt == 3 ? at_zero : def);
+    child[(size_t)next++] = nan_left ? v.right_child[nd] : v.left_child[nd];
+    child[(size_t)next++] = nan_left ? v.left_child[nd] : v.right_child[nd];
+    if (cat) {  // the bitset's index in the threshold's bits
+      const int32_t ci = cat_base + (int32_t)thr;
+      float bits;
+      std::memcpy(&bits, &ci, sizeof(bits));
+      p = PNode{bits, meta | kPNodeCat};
+      special = true;
+      continue;
+    }
+    if (mt == 1 && def != at_zero) {
+      meta |= kPNodeZeroFlip;
+      special = true;
+    }
+    // the largest f32 not above the threshold: v <= thr is v <= f
+    float f = (float)thr;
+    if ((double)f > thr) f = std::nextafterf(f, -INFINITY);
+    if (nan_left) {  // v > f as -v <= the f32 below -f
+      meta |= kPNodeNegate;
+      if (std::isnan(f)) f = INFINITY;             // nothing is <= NaN: every number goes right
+      else if (f == INFINITY) f = NAN;             // no number is above infinity
+      else f = std::nextafterf(-f, -INFINITY);
+    }
+    p = PNode{f, meta};
+  }
+  if (next != total) return false;
+  tree.push_back(make_int4((int32_t)first, 0, nl, padded));
+  max_nodes = std::max(max_nodes, padded);
+  return true;
+}
+
 static Status forest_create(LgbmB200Forest* F, const LgbmB200TreeView* trees, int32_t nt, int32_t ntpi,
                             int32_t device) {
   F->device = device;
   F->ntpi = std::max(1, ntpi);
-  bool wide = false;
   for (int32_t t = 0; t < nt; ++t) {
     const LgbmB200TreeView& v = trees[t];
     if (v.num_leaves < 1) return Status(LGBM_B200_ERR_INVALID_PARAMETER, "forest_create: a tree has no leaves");
-    if (v.num_leaves > 32768) wide = true;
     for (int32_t nd = 0; nd < v.num_leaves - 1; ++nd)
       if (v.split_feature[nd] < 0 || v.split_feature[nd] >= (1 << kNodeFeatureBits))
         return Status(LGBM_B200_ERR_UNSUPPORTED, "forest_create: split feature index outside [0, 2^24)");
@@ -733,38 +797,43 @@ static Status forest_create(LgbmB200Forest* F, const LgbmB200TreeView* trees, in
   CU(cudaSetDevice(device));
   CU(cudaStreamCreateWithFlags(&F->stream, cudaStreamNonBlocking));
   std::vector<int4> tree;
-  std::vector<DNode> nodes;
+  std::vector<PNode> pnodes;
   std::vector<DNodeWide> wnodes;
   std::vector<int32_t> cat_bnd{0};
   std::vector<double> leaf_value;
   std::vector<uint32_t> cat_words;
-  int32_t node_count = 0;
+  std::vector<int32_t> cat_base((size_t)nt);
+  int32_t max_nodes = 0, max_feature = 0;
+  bool compact = true, special = false;
   for (int32_t t = 0; t < nt; ++t) {
     const LgbmB200TreeView& v = trees[t];
-    tree.push_back(make_int4(node_count, (int32_t)leaf_value.size(), v.num_leaves, 0));
-    int32_t cat_base = (int32_t)cat_bnd.size() - 1;
+    for (int32_t nd = 0; nd < v.num_leaves - 1; ++nd) max_feature = std::max(max_feature, v.split_feature[nd]);
+    cat_base[(size_t)t] = (int32_t)cat_bnd.size() - 1;
     for (int32_t c = 0; c < v.num_cat; ++c) {
       int32_t b0 = v.cat_boundaries[c], b1 = v.cat_boundaries[c + 1];
       for (int32_t w = b0; w < b1; ++w) cat_words.push_back(v.cat_threshold[w]);
       cat_bnd.push_back((int32_t)cat_words.size());
     }
-    for (int32_t nd = 0; nd < v.num_leaves - 1; ++nd) {
-      double thr = v.threshold[nd];
-      if (v.decision_type[nd] & 1) {  // categorical: the bitset's index in the threshold's bits
-        const int64_t ci = cat_base + (int64_t)v.threshold[nd];
-        std::memcpy(&thr, &ci, sizeof(thr));
+  }
+  for (int32_t t = 0; t < nt && compact; ++t)
+    compact = pack_tree(trees[t], cat_base[(size_t)t], pnodes, leaf_value, tree, max_nodes, special);
+  if (!compact) {
+    tree.clear();
+    leaf_value.clear();
+    for (int32_t t = 0; t < nt; ++t) {
+      const LgbmB200TreeView& v = trees[t];
+      tree.push_back(make_int4((int32_t)wnodes.size(), (int32_t)leaf_value.size(), v.num_leaves, 0));
+      for (int32_t nd = 0; nd < v.num_leaves - 1; ++nd) {
+        double thr = v.threshold[nd];
+        if (v.decision_type[nd] & 1) {  // categorical: the bitset's index in the threshold's bits
+          const int64_t ci = cat_base[(size_t)t] + (int64_t)v.threshold[nd];
+          std::memcpy(&thr, &ci, sizeof(thr));
+        }
+        const int32_t fd = v.split_feature[nd] | ((int32_t)(uint8_t)v.decision_type[nd] << kNodeFeatureBits);
+        wnodes.push_back(DNodeWide{thr, fd, 0, v.left_child[nd], v.right_child[nd]});
       }
-      const int32_t fd = v.split_feature[nd] | ((int32_t)(uint8_t)v.decision_type[nd] << kNodeFeatureBits);
-      if (wide) {
-        DNodeWide n{thr, fd, 0, v.left_child[nd], v.right_child[nd]};
-        wnodes.push_back(n);
-      } else {
-        DNode n{thr, fd, (int16_t)v.left_child[nd], (int16_t)v.right_child[nd]};
-        nodes.push_back(n);
-      }
-      ++node_count;
+      for (int32_t l = 0; l < v.num_leaves; ++l) leaf_value.push_back(v.leaf_value[l]);
     }
-    for (int32_t l = 0; l < v.num_leaves; ++l) leaf_value.push_back(v.leaf_value[l]);
   }
   DeviceArena& A = F->arena;
   auto up = [&](auto& vec, auto** dst) -> Status {
@@ -776,10 +845,13 @@ static Status forest_create(LgbmB200Forest* F, const LgbmB200TreeView* trees, in
   DForest& f = F->f;
   f.num_trees = nt;
   f.ntpi = F->ntpi;
-  f.wide = wide;
+  f.compact = compact;
+  f.max_nodes = max_nodes;
+  f.special = special;
+  f.max_feature = max_feature;
   Status s;
   int4* tt;
-  DNode* dn = nullptr;
+  PNode* dn = nullptr;
   DNodeWide* dw = nullptr;
   int32_t* cb;
   double* lv;
@@ -787,9 +859,9 @@ static Status forest_create(LgbmB200Forest* F, const LgbmB200TreeView* trees, in
   if (!(s = up(tree, &tt)).ok() || !(s = up(cat_bnd, &cb)).ok() || !(s = up(leaf_value, &lv)).ok() ||
       !(s = up(cat_words, &cw)).ok())
     return s;
-  if (!(s = wide ? up(wnodes, &dw) : up(nodes, &dn)).ok()) return s;
+  if (!(s = compact ? up(pnodes, &dn) : up(wnodes, &dw)).ok()) return s;
   f.tree = tt;
-  f.nodes = wide ? static_cast<const void*>(dw) : static_cast<const void*>(dn);
+  f.nodes = compact ? static_cast<const void*>(dn) : static_cast<const void*>(dw);
   f.cat_bnd = cb;
   f.leaf_value = lv;
   f.cat_words = cw;
