@@ -306,7 +306,7 @@ static Status booster_iter(LgbmB200Booster* b, int32_t* stop) {
   if (b->bagging && ((b->bag_cnt < n && b->iter % b->cfg.bagging_freq == 0) || b->need_re_bagging)) {
     b->need_re_bagging = false;
     int64_t nb = (n + 1023) / 1024;
-    k_bagging<<<(unsigned)((nb + 127) / 128), 128, 0, s>>>(b->rng, n, b->cfg.bagging_fraction, b->in_bag,
+    k_bagging<<<(unsigned)((nb + 3) / 4), 128, 0, s>>>(b->rng, n, b->cfg.bagging_fraction, b->in_bag,
                                                            b->block_in);
     CU_LAUNCH();
     k_bag_scan<<<1, 1024, 0, s>>>(b->block_in, (int32_t)nb, n, b->block_base, b->counts);

@@ -611,11 +611,11 @@ Status enqueue_tree(LgbmB200Learner* h) {
   if (mode == LGBM_B200_HIST_QUANT && h->cfg.quant_train_renew_leaf) {
     k_leaf_sums<<<dim3(leaf_sum_warps(h) / 8, 1, K), 256, 16 * (size_t)L, s>>>(c, h->leaf_sums, h->leaf_rank);
     CU_LAUNCH();
-    k_leaf_renew<<<dim3(1, 1, K), 256, 0, s>>>(c, h->leaf_sums, h->leaf_rank, leaf_sum_warps(h), nullptr);
+    k_leaf_renew<<<dim3((L + 7) / 8, 1, K), 256, 0, s>>>(c, h->leaf_sums, h->leaf_rank, leaf_sum_warps(h), nullptr);
     CU_LAUNCH();
   }
   // a tree in rounds adds its rounds' launches when it is read back
-  h->last_launches = 1 + (h->rounds ? 2 : h->cfg.persistent_grow ? 1 : 2 * (L - 1) + (c.defer ? 1 : 0)) +
+  h->tree_launches = 1 + (h->rounds ? 2 : h->cfg.persistent_grow ? 1 : 2 * (L - 1) + (c.defer ? 1 : 0)) +
                      ((mode == LGBM_B200_HIST_QUANT && h->cfg.quant_train_renew_leaf) ? 2 : 0);
   return Status();
 }
@@ -691,13 +691,12 @@ static Status run_tree_dp(LgbmB200Learner* h) {
   if (mode == LGBM_B200_HIST_QUANT && h->cfg.quant_train_renew_leaf) {
     k_leaf_sums<<<dim3(leaf_sum_warps(h) / 8, 1, 1), 256, 16 * (size_t)L, s>>>(c, h->leaf_sums, h->leaf_rank);
     CU_LAUNCH();
-    k_leaf_renew<<<1, 256, 0, s>>>(c, h->leaf_sums, h->leaf_rank, leaf_sum_warps(h), h->dp_f64);
+    k_leaf_renew<<<(L + 7) / 8, 256, 0, s>>>(c, h->leaf_sums, h->leaf_rank, leaf_sum_warps(h), h->dp_f64);
     CU_LAUNCH();
     if (!(st = dp_allreduce(h, h->dp_f64, 2 * (int64_t)L, LGBM_B200_DT_FLOAT64, LGBM_B200_OP_SUM)).ok()) return st;
     k_dp_leaf_apply<<<1, 256, 0, s>>>(c, h->dp_f64);
     CU_LAUNCH();
   }
-  h->last_launches = 0;
   return Status();
 }
 
@@ -943,6 +942,7 @@ Status train_collect(LgbmB200Learner* h) {
       h->last_step_ms[(size_t)3 * step + 2] = d;
     }
   }
+  h->last_launches = h->dp ? 0 : h->tree_launches;
   if (h->rounds) {
     int rounds = 0;
     for (int k = 0; k < K; ++k) {
@@ -950,7 +950,7 @@ Status train_collect(LgbmB200Learner* h) {
       std::memcpy(&rs, h->rb_host + (size_t)k * h->rb_slot + h->rb.rs, sizeof(rs));
       rounds = std::max(rounds, rs.rounds);
     }
-    h->last_launches += 3 + 4 * rounds;
+    h->last_launches = h->tree_launches + 3 + 4 * rounds;
   }
   h->last_hist_rows = 0;
   h->last_part_rows = 0;

@@ -320,6 +320,7 @@ struct LgbmB200Learner {
   // changes (launch shape, bagging): graphs captured before it are stale
   int config_epoch = 0;
   int32_t last_launches = 0;
+  int32_t tree_launches = 0;  // of the last enqueue_tree, the rounds aside
   // growth in rounds (round_kernels.cuh)
   bool rounds = false;
   cudaStream_t body_stream = nullptr;  // captures the body of the rounds' loop

@@ -161,24 +161,53 @@ __global__ void __launch_bounds__(256) k_quant_apply(const float2* gh, int64_t n
 }
 
 // sample_strategy.rs:280-320: rows of block b draw from the LCG `state[b]`
-// (Random(bagging_seed + b)) in row order; r < fraction keeps the row.
-// One thread per 1024-row block; block_in[b] receives the block's in-bag count.
-__global__ void k_bagging(uint32_t* rng_state, int64_t n, double fraction, uint8_t* in_bag, int32_t* block_in) {
-  int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int64_t r0 = b * 1024;
+// (Random(bagging_seed + b)) in row order; r < fraction keeps the row. One
+// warp per 1024-row block, lane l on rows 32 l .. 32 l + 31 from the state
+// advanced by 32 l draws (the composition of the step with itself), so a
+// block's serial chain is 32 draws instead of 1024: 147 -> 6 us for 1.1M
+// rows. block_in[b] receives the block's in-bag count.
+__global__ void __launch_bounds__(128) k_bagging(uint32_t* rng_state, int64_t n, double fraction, uint8_t* in_bag,
+                                                 int32_t* block_in) {
+  const int lane = threadIdx.x & 31;
+  const int64_t b = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int64_t r0 = b * 1024;
   if (r0 >= n) return;
-  int64_t r1 = min(n, r0 + 1024);
+  const int32_t rows = (int32_t)min((int64_t)1024, n - r0), mine = max(0, min(32, rows - 32 * lane));
   uint32_t x = rng_state[b];
-  int32_t cnt = 0;
-  for (int64_t r = r0; r < r1; ++r) {
-    x = x * 214013u + 2531011u;
-    float f = (float)((x >> 16) & 0x7FFF) / 32768.0f;
-    const bool keep = (double)f < fraction;
-    in_bag[r] = keep ? 1 : 0;
-    cnt += keep ? 1 : 0;
+  // x -> a x + c is 32 draws; lane l applies it l times by its binary powers
+  uint32_t a = 214013u, c = 2531011u;
+  for (int i = 0; i < 5; ++i) {
+    c = a * c + c;
+    a = a * a;
   }
-  rng_state[b] = x;
-  block_in[b] = cnt;
+  for (int i = 0; i < 5; ++i) {
+    if (lane >> i & 1) x = a * x + c;
+    c = a * c + c;
+    a = a * a;
+  }
+  uint32_t keep = 0;
+  for (int k = 0; k < mine; ++k) {
+    x = x * 214013u + 2531011u;
+    const float f = (float)((x >> 16) & 0x7FFF) / 32768.0f;
+    if ((double)f < fraction) keep |= 1u << k;
+  }
+  // 32 flags as bytes: two 16-byte stores (the rows start 32-byte aligned)
+  uint8_t* out = in_bag + r0 + 32 * lane;
+  if (mine == 32) {
+    uint32_t w[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t nib = keep >> (4 * i) & 15u;
+      w[i] = (nib & 1u) | (nib & 2u) << 7 | (nib & 4u) << 14 | (nib & 8u) << 21;
+    }
+    reinterpret_cast<uint4*>(out)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    reinterpret_cast<uint4*>(out)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  } else {
+    for (int k = 0; k < mine; ++k) out[k] = (uint8_t)(keep >> k & 1u);
+  }
+  const int32_t cnt = __reduce_add_sync(0xffffffffu, __popc(keep));
+  if (lane == 0) block_in[b] = cnt;
+  if (lane == (rows - 1) / 32) rng_state[b] = x;  // the state after the block's last row
 }
 
 // Exclusive prefix of the blocks' in-bag counts (one CTA of 1024 threads,

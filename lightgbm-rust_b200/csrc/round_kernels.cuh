@@ -458,6 +458,18 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
       lg[l] = r.gain[v];
       lf[l] = r.feat[v];
     }
+    // this thread's first kOwn candidates and their rows stay in registers
+    // (more only in trees of a thousand leaves); loaded while the replay runs
+    constexpr int kOwn = 2;
+    auto listed = [&](int32_t i) { return i < st.ncand ? r.cand[i] : new0 + i - st.ncand; };
+    int32_t own_v[kOwn], own_n[kOwn];
+#pragma unroll
+    for (int j = 0; j < kOwn; ++j) {
+      const int32_t i = tid + j * kDecideThreads;
+      own_v[j] = i < total ? listed(i) : -1;
+    }
+#pragma unroll
+    for (int j = 0; j < kOwn; ++j) own_n[j] = own_v[j] >= 0 ? r.node[own_v[j]].count : 0;
     for (int b = tid; b < kRoundBins; b += kDecideThreads) {
       exps[b] = 0;
       cands[b] = 0;
@@ -491,7 +503,6 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
     if (!done) {
       const int32_t open = need - popped, spare = min(st.nfree, r.ecap - E);
       const int32_t most = max(1, min(min(r.bmax, spare - open + 1), max(kRoundMin, (open + 3) / 4)));
-      auto cand_id = [&](int32_t i) { return i < st.ncand ? r.cand[i] : new0 + i - st.ncand; };
       // 0: the node cannot be split; positive for every positive gain
       auto key_of = [&](int32_t v) {
         float k = nd.gain[v] > 0.0 ? fmaxf((float)nd.gain[v], 1.4e-45f) : 0.0f;
@@ -503,12 +514,25 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
         return __float_as_uint(k);
       };
       const uint32_t hi = key_of(top);  // no key is larger
+      uint32_t own_k[kOwn];
+      // visits this thread's candidates: fn(i, node, rows, key), for every
+      // multiple of kDecideThreads below `total` (node -1 past it)
+      auto each_cand = [&](auto fn) {
+#pragma unroll
+        for (int j = 0; j < kOwn; ++j)
+          if (j * kDecideThreads < total) fn(tid + j * kDecideThreads, own_v[j], own_n[j], own_k[j]);
+        for (int32_t i0 = kOwn * kDecideThreads; i0 < total; i0 += kDecideThreads) {
+          const int32_t i = i0 + tid, v = i < total ? listed(i) : -1;
+          fn(i, v, v >= 0 ? r.node[v].count : 0, v >= 0 ? key_of(v) : 0u);
+        }
+      };
       {
         uint32_t lo = 0xffffffffu;
-        for (int32_t i = tid; i < total; i += kDecideThreads) {
-          const uint32_t k = key_of(cand_id(i));
+#pragma unroll
+        for (int j = 0; j < kOwn; ++j) own_k[j] = own_v[j] >= 0 ? key_of(own_v[j]) : 0u;
+        each_cand([&](int32_t, int32_t, int32_t, uint32_t k) {
           if (k > 0) lo = min(lo, k);
-        }
+        });
         lo = __reduce_min_sync(0xffffffffu, lo);
         if ((tid & 31) == 0) atomicMin(&s_lo, lo);
       }
@@ -516,14 +540,13 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
       const int shift = max(0, 32 - __clz(hi - min(hi, s_lo)) - 10);
       static_assert(kRoundBins == 1 << 10, "the range of keys shifted to ten bits");
       auto bin_of = [&](uint32_t k) { return k ? min((int32_t)((hi - k) >> shift), kRoundBins - 1) : kRoundBins; };
-      for (int32_t i = tid; i < total; i += kDecideThreads) {
-        const int32_t v = cand_id(i), b = bin_of(key_of(v));
+      each_cand([&](int32_t, int32_t v, int32_t n, uint32_t k) {
+        const int32_t b = bin_of(k);
         if (b < kRoundBins) {
-          const int32_t n = r.node[v].count;
           if (n <= kRoundRows / 2 && v != top) atomicAdd(&rows[b], (unsigned long long)n);
           atomicAdd(&cands[b], 1);
         }
-      }
+      });
       for (int32_t e = tid; e < E; e += kDecideThreads) {
         const int32_t v = nd.exp_node[e];
         if (!(nd.exp[v] & kReplayed)) atomicAdd(&exps[bin_of(key_of(v))], 1);
@@ -543,7 +566,7 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
           if (kb < open && kb + k >= open) s_tau = b;  // the last bin that can still be among the splits
           if (cb < most && cb + n >= most) {           // the last bin with room this round
             s_cut = b;
-            s_room = most - cb;
+            s_room = most - cb - (b == 0 ? 1 : 0);  // the node the replay waits for is in bin 0
           }
           // the first bin that would take the round past kRoundRows rows ahead of need
           if (rb <= kRoundRows && rb + rows[b] > kRoundRows) s_rowcut = b;
@@ -575,52 +598,42 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
         r.scan_cnt[2 * at] = 0;
         r.scan_cnt[2 * at + 1] = 0;
       };
-      auto tiles_of = [&](int32_t v) { return (r.node[v].count + kPartTileRows - 1) / kPartTileRows; };
-      tiles = tiles_of(top);
+      auto tiles_of = [](int32_t n) { return (n + kPartTileRows - 1) / kPartTileRows; };
+      tiles = tiles_of(r.node[top].count);
       if (tid == 0) place(0, top, 0);
-      for (int32_t i0 = 0; i0 < total; i0 += kDecideThreads) {
-        const int32_t i = i0 + tid;
-        bool want = false, keep = false, drop = false, edge = false;
-        int32_t v = -1, nt = 0;
-        if (i < total) {
-          v = cand_id(i);
-          const int32_t b = bin_of(key_of(v));
-          if (v == top) {
-          } else if (b > tau) {
-            drop = true;
-          } else {
-            const bool fits = r.node[v].count <= kRoundRows / 2 && b < rowcut;
-            want = fits && b < cut;
-            edge = fits && b == cut;
-            keep = true;
-            nt = tiles_of(v);
-          }
+      each_cand([&](int32_t, int32_t v, int32_t n, uint32_t k) {
+        bool pick = false, keep = false, drop = false, edge = false;
+        if (v >= 0 && v != top) {
+          const int32_t b = bin_of(k);
+          drop = b > tau;
+          const bool fits = !drop && n <= kRoundRows / 2 && b < rowcut;
+          pick = fits && b < cut;
+          edge = fits && b == cut;
+          keep = !drop;
         }
         unsigned long long tot;
         const int32_t edge0 = (int32_t)block_prefix<kDecideThreads>((unsigned long long)edge, warp_sums, tot);
-        want = want || (edge && at_cut0 + edge0 < share);
+        // the cut leaves room for `most` in all, the node the replay waits for among them
+        pick = pick || (edge && at_cut0 + edge0 < share);
         at_cut0 += (int32_t)tot;
-        // expansions and their tiles; an expansion past `most` stays a candidate
-        const unsigned long long b1 = block_prefix<kDecideThreads>(want ? (1ull << 32) | (uint32_t)nt : 0ull, warp_sums, tot);
-        const int32_t at = took + (int32_t)(b1 >> 32);
-        const bool pick = want && at < most && E + at < r.ecap;
-        unsigned long long tot2;
-        block_prefix<kDecideThreads>(pick ? (1ull << 32) | (uint32_t)nt : 0ull, warp_sums, tot2);
-        if (pick) place(at, v, tiles + (int32_t)(uint32_t)b1);
-        took += (int32_t)(tot2 >> 32);
-        tiles += (int32_t)(uint32_t)tot2;
-        const bool stay = keep && !pick;
-        const unsigned long long b2 =
-            block_prefix<kDecideThreads>(((unsigned long long)stay << 32) | (uint32_t)drop, warp_sums, tot);
+        keep = keep && !pick;
+        // one sum of four counts: tiles (32 bits), picked, kept and dropped (10 bits each)
+        const int32_t nt = tiles_of(n);
+        const unsigned long long before = block_prefix<kDecideThreads>(
+            (pick ? (1ull << 32) | (uint32_t)nt : 0ull) | (unsigned long long)keep << 42 | (unsigned long long)drop << 52,
+            warp_sums, tot);
+        static_assert(kDecideThreads < 1024, "ten bits a count");
+        const int32_t at = took + (int32_t)(before >> 32 & 1023);
+        if (pick && at < r.bmax && E + at < r.ecap) place(at, v, tiles + (int32_t)(uint32_t)before);
         // the list is compacted in place: an entry moves to a place at or
         // before its own, which this pass or an earlier one has read
-        if (stay) r.cand[kept + (int32_t)(b2 >> 32)] = v;
-        if (drop) {
-          r.free_next[freed + (int32_t)(uint32_t)b2] = r.node[v].buf;
-        }
-        kept += (int32_t)(tot >> 32);
-        freed += (int32_t)(uint32_t)tot;
-      }
+        if (keep) r.cand[kept + (int32_t)(before >> 42 & 1023)] = v;
+        if (drop) r.free_next[freed + (int32_t)(before >> 52)] = r.node[v].buf;
+        took += (int32_t)(tot >> 32 & 1023);
+        tiles += (int32_t)(uint32_t)tot;
+        kept += (int32_t)(tot >> 42 & 1023);
+        freed += (int32_t)(tot >> 52);
+      });
       __syncthreads();
       // the round's buffers leave the list, the dropped candidates' join it
       for (int32_t i = tid; i < freed; i += kDecideThreads) r.free[st.nfree - took + i] = r.free_next[i];
