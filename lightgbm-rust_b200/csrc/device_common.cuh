@@ -61,6 +61,17 @@ struct DLeafSplits {  // learner/mod.rs:63-71
   double weight;
 };
 
+// Exact fixed-point form of a tree's gradients (f32) for the float histograms:
+// a value is q * 2^base with an integer q, added as limbs of `bits` bits (the
+// last one signed) in 32-bit cells.
+struct DFixed {
+  int32_t ok;             // the tree's values fit
+  int32_t rows;           // rows a cell takes before a limb could wrap
+  int32_t g_limbs, g_bits, g_base;
+  int32_t h_limbs, h_bits, h_base;  // h_limbs 1: a constant hessian, counted
+  double h_value;
+};
+
 // Control block of one tree being grown (one per tree slot).
 struct DSlotState {
   int32_t num_leaves_cur;  // tree.num_leaves
@@ -91,6 +102,7 @@ struct DSlotState {
   int32_t pd_need, pd_S, pd_G, pd_Lft, pd_R;            // the step's head
   int32_t pd_bf[2];                // the new leaves' best candidates (inner feature, -1 none)
   double pd_bg[2];                 // and their penalized gains
+  DFixed fx;
   int64_t hist_rows;       // rows histogrammed in this tree (statistics)
   int64_t part_rows;       // rows partitioned in this tree (statistics)
 };
@@ -205,6 +217,7 @@ struct DSlot {
   uint8_t* bytree;         // by-tree feature mask [num_features]
   double* root_partials;   // [2 x kRootBlocks] (g, h) partial sums
   long long* root_ipartials;
+  uint32_t* root_range;    // [5 x kRootBlocks]: smallest nonzero / largest |g|, smallest / largest / smallest nonzero h (as bits)
   int32_t* root_counter;
   DTree tree;
   DRounds r;

@@ -118,6 +118,7 @@ constexpr int kDecideThreads = 512;
 constexpr int kDecideSmemNodes = 3072;  // explored nodes the replay keeps in shared memory
 __global__ void k_round_part(const __grid_constant__ DCtx c);
 const void* round_hist_kernel(int mode, int ng);
+size_t round_hist_smem(int mode, int ng);
 cudaError_t launch_round_hist(int mode, int ng, dim3 grid, size_t smem, cudaStream_t st, const DCtx& c,
                               const DTileTable& tt, int32_t sub_rows);
 // the threshold scans of a round, on packed integer and on FP64 sums

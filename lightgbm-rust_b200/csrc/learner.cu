@@ -285,6 +285,7 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
     ALLOC(d.bytree, nf);
     ALLOC(d.root_partials, 2 * kRootBlocks);
     ALLOC(d.root_ipartials, kRootBlocks);
+    ALLOC(d.root_range, 5 * kRootBlocks);
     ALLOC(d.root_counter, 1);
     DTree& t = d.tree;
     const auto& rb = h->rb;
@@ -345,7 +346,8 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
     CU(cudaMemset(h->round_ctrl, 0, 3 * sizeof(int32_t)));
     // what is resident at once, shared by the slots (and feature tiles)
     const void* hist = round_hist_kernel(mode, h->hist_ng);
-    CU(cudaFuncSetAttribute(hist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->hist_smem));
+    h->round_hist_smem = round_hist_smem(mode, h->hist_ng);
+    CU(cudaFuncSetAttribute(hist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->round_hist_smem));
     const bool quant = mode == LGBM_B200_HIST_QUANT;
     bool cats = false;
     for (auto& f : h->feats) cats |= f.bin_type == 1;
@@ -358,7 +360,7 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
     int per_sm = 0;
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, scan, scan_threads, h->round_scan_smem));
     h->round_scan_grid = std::max(1, per_sm * h->num_sms / K);
-    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hist, kHistThreads, h->hist_smem));
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hist, kHistThreads, h->round_hist_smem));
     h->hist_grid = std::max(1, per_sm * h->num_sms / (h->ntiles * K));
     h->part_grid = std::max(1, h->part_grid / K);
     CU(cudaStreamCreateWithFlags(&h->body_stream, cudaStreamNonBlocking));
@@ -497,7 +499,7 @@ static Status enqueue_round(LgbmB200Learner* h, cudaStream_t s, bool root, cudaG
     CU_LAUNCH();
   }
   if (ev) CU(cudaEventRecord(ev[1], s));
-  CU(launch_round_hist(h->cfg.hist_precision, h->hist_ng, dim3(h->hist_grid, h->ntiles, K), h->hist_smem, s, c,
+  CU(launch_round_hist(h->cfg.hist_precision, h->hist_ng, dim3(h->hist_grid, h->ntiles, K), h->round_hist_smem, s, c,
                        h->tiles, h->sub_rows));
   if (ev) CU(cudaEventRecord(ev[2], s));
   const dim3 scan_grid(h->round_scan_grid, 1, K);

@@ -326,7 +326,7 @@ struct LgbmB200Learner {
   cudaStream_t body_stream = nullptr;  // captures the body of the rounds' loop
   int32_t* round_ctrl = nullptr;       // [3]: slots arrived, slots going on, whether another round runs
   int round_scan_grid = 0;
-  size_t round_scan_smem = 0;
+  size_t round_scan_smem = 0, round_hist_smem = 0;
   int last_rounds = 0;
   // captured tree growth
   cudaGraphExec_t graph_exec = nullptr;

@@ -62,6 +62,39 @@ __device__ bool before_find_best_split(const DCtx& c, const DSlot& s, int32_t le
   return true;
 }
 
+// The fixed-point form of one value's range: |v| < 2^(emax - 126) and its last
+// bit at or above 2^(emin - 150), from the biased exponents. Two limbs up to
+// 40 bits and a sign, three up to 60; false when it takes more.
+__device__ __forceinline__ bool fixed_form(int32_t emin, int32_t emax, int32_t& limbs, int32_t& bits, int32_t& base) {
+  const int32_t need = emax - emin + 25;
+  base = emin - 150;
+  limbs = need <= 40 ? 2 : 3;
+  bits = (need + limbs - 1) / limbs;
+  return emax < 255 && need <= 60;
+}
+
+// From the smallest nonzero and largest |g| and the smallest, largest and
+// smallest nonzero h (as bits) over the in-bag rows; one thread.
+__device__ void fixed_init(DFixed& fx, uint32_t glo, uint32_t ghi, uint32_t hlo, uint32_t hhi, uint32_t hnz) {
+  auto exponent = [](uint32_t b) { return max(1, (int32_t)(b >> 23)); };  // denormals share exponent 1
+  if (glo > ghi) glo = ghi = 0x3f800000u;                                 // every gradient is zero
+  bool ok = fixed_form(exponent(glo), exponent(ghi), fx.g_limbs, fx.g_bits, fx.g_base);
+  int32_t bits = fx.g_bits;
+  fx.h_value = (double)__uint_as_float(hlo);
+  if (hlo == hhi) {
+    fx.h_limbs = 1;
+    fx.h_bits = 1;
+    fx.h_base = 0;
+    ok = ok && (hlo >> 23 & 255) < 255;
+  } else {
+    // the reference's objectives give no negative hessian
+    ok = fixed_form(exponent(hnz), exponent(hhi), fx.h_limbs, fx.h_bits, fx.h_base) && ok && (hhi >> 31) == 0;
+    bits = max(bits, fx.h_bits);
+  }
+  fx.ok = ok;
+  fx.rows = (int32_t)min(1u << 30, (1u << (32 - bits)) - 1u);
+}
+
 // The root as node 0 of a tree grown in rounds; one thread.
 __device__ void round_init(const DCtx& c, const DSlot& s, int32_t need) {
   const DRounds& r = s.r;
@@ -120,6 +153,15 @@ __global__ void __launch_bounds__(256) k_tree_init(const __grid_constant__ DCtx 
   const int64_t b0 = min(n, (int64_t)blockIdx.x * chunk), b1 = min(n, b0 + chunk);
   double sg = 0.0, sh = 0.0;
   long long si = 0;
+  uint32_t glo = 0xffffffffu, ghi = 0, hlo = 0xffffffffu, hhi = 0, hnz = 0xffffffffu;  // of the float forms
+  auto range = [&](float2 v) {
+    const uint32_t g = __float_as_uint(v.x) & 0x7fffffffu, h = __float_as_uint(v.y);
+    if (g) glo = min(glo, g);
+    ghi = max(ghi, g);
+    hlo = min(hlo, h);
+    hhi = max(hhi, h);
+    if (h) hnz = min(hnz, h);
+  };
   if (c.hist_mode == LGBM_B200_HIST_QUANT && !bag) {
     // rows in order: eight packed values per thread and iteration
     const double gsc = s.st->grad_scale, hsc = s.st->hess_scale;
@@ -167,7 +209,10 @@ __global__ void __launch_bounds__(256) k_tree_init(const __grid_constant__ DCtx 
         const float4 b = *reinterpret_cast<const float4*>(s.gh + i + 2);
         v[0] = make_float2(a.x, a.y), v[1] = make_float2(a.z, a.w), v[2] = make_float2(b.x, b.y),
         v[3] = make_float2(b.z, b.w);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) range(v[j]);
       } else {
+        for (int64_t j = i; j < b1; ++j) range(s.gh[j]);
 #pragma unroll
         for (int j = 0; j < 4; ++j) v[j] = i + j < b1 ? s.gh[i + j] : make_float2(0.f, 0.f);
       }
@@ -180,9 +225,30 @@ __global__ void __launch_bounds__(256) k_tree_init(const __grid_constant__ DCtx 
   } else {
     for (int64_t i = b0 + tid; i < b1; i += blockDim.x) {
       float2 v = s.gh[bag ? bag[i] : (uint32_t)i];
+      range(v);
       sg += (double)v.x;
       sh += (double)v.y;
     }
+  }
+  __shared__ uint32_t red_r[5];
+  if (c.hist_mode != LGBM_B200_HIST_QUANT) {
+    if (tid < 5) red_r[tid] = tid & 1 ? 0u : 0xffffffffu;
+    __syncthreads();
+    glo = __reduce_min_sync(0xffffffffu, glo);
+    ghi = __reduce_max_sync(0xffffffffu, ghi);
+    hlo = __reduce_min_sync(0xffffffffu, hlo);
+    hhi = __reduce_max_sync(0xffffffffu, hhi);
+    hnz = __reduce_min_sync(0xffffffffu, hnz);
+    if ((tid & 31) == 0) {
+      atomicMin(&red_r[0], glo);
+      atomicMax(&red_r[1], ghi);
+      atomicMin(&red_r[2], hlo);
+      atomicMax(&red_r[3], hhi);
+      atomicMin(&red_r[4], hnz);
+    }
+    __syncthreads();
+    if (tid < 5) s.root_range[tid * kRootBlocks + blockIdx.x] = red_r[tid];
+    __threadfence();
   }
   __shared__ double red_g[8], red_h[8];
   __shared__ long long red_i[8];
@@ -243,6 +309,15 @@ __global__ void __launch_bounds__(256) k_tree_init(const __grid_constant__ DCtx 
     part[1][k] = s.root_partials[kRootBlocks + k];
     ipart[k] = s.root_ipartials[k];
   }
+  if (c.hist_mode != LGBM_B200_HIST_QUANT) {  // red_r holds this block's own range
+    for (int k = tid; k < (int)gridDim.x; k += blockDim.x) {
+      atomicMin(&red_r[0], s.root_range[k]);
+      atomicMax(&red_r[1], s.root_range[kRootBlocks + k]);
+      atomicMin(&red_r[2], s.root_range[2 * kRootBlocks + k]);
+      atomicMax(&red_r[3], s.root_range[3 * kRootBlocks + k]);
+      atomicMin(&red_r[4], s.root_range[4 * kRootBlocks + k]);
+    }
+  }
   __syncthreads();
   if (tid == 0 || tid == 32) {
     double v = 0;
@@ -258,6 +333,8 @@ __global__ void __launch_bounds__(256) k_tree_init(const __grid_constant__ DCtx 
   __syncthreads();
   if (tid != 0) return;
   *s.root_counter = 0;
+  st->fx.ok = 0;
+  if (c.hist_mode != LGBM_B200_HIST_QUANT) fixed_init(st->fx, red_r[0], red_r[1], red_r[2], red_r[3], red_r[4]);
   const double a = red_g[0], b = red_g[1];
   const long long d = red_i[0];
   s.leaf_count[0] = (int32_t)n;
@@ -818,6 +895,162 @@ __device__ void hist_body(const DCtx& c, const DSlot& s, const DTileTable& tt, i
   } else {
     __syncthreads();
   }
+}
+
+// The float forms' histogram in exact fixed point. FP64 adds to shared memory
+// are compare-and-swap loops (a load, an add and a compare-and-swap per value,
+// about 45 cycles a row of 32 features), and the compensated form's pairs of
+// FP32 atomics are no faster. A tree's f32 gradients usually span few enough
+// binary orders of magnitude (DFixed) to be integers of up to 60 bits, which
+// are added limb by limb with native 32-bit shared reductions (two or three a
+// value, one for a constant hessian) that nothing waits for. The sums of a
+// CTA are exact; they are rounded once, when the cells are flushed to the
+// FP64 histogram, so a cell carries one rounding per flush instead of one per
+// row. Trees whose gradients span more keep the adds above. Rows are staged
+// as in the tile loop above; cells: [limb][raw][lane].
+constexpr int kFixedPlanes = 6;  // three limbs of the gradient, three of the hessian
+constexpr size_t kFixedSmem =
+    (size_t)kFixedPlanes * kMaxBins * 32 * 4 + (size_t)kHistTileRows * 32 + (size_t)kHistTileRows * 24;
+
+__device__ __forceinline__ long long fixed_of(float v, int32_t base) {
+  const uint32_t b = __float_as_uint(v), e = b >> 23 & 255u;
+  const uint32_t m = (b & 0x7fffffu) | (e ? 0x800000u : 0u);
+  // m = 0 shifts nothing; otherwise the exponent is at or above the tree's smallest
+  const long long q = m ? (long long)m << (max((int32_t)e, 1) - 150 - base) : 0ll;
+  return b >> 31 ? -q : q;
+}
+
+__device__ void hist_body_fixed(const DCtx& c, const DSlot& s, const DFixed& fx, const DTileTable& tt, int tile,
+                                const LeafRows& lr, int64_t r0, int64_t r1, unsigned char* smem_raw) {
+  int f0, f1, bin0, nbins;
+  tile_of(tt, tile, f0, f1, bin0, nbins);
+  (void)nbins;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int kCells = kMaxBins * 32;
+  int32_t* cells = reinterpret_cast<int32_t*>(smem_raw);
+  uint4* sbins = reinterpret_cast<uint4*>(smem_raw + (size_t)kFixedPlanes * kCells * 4);
+  uint4* sl4 = sbins + kHistTileRows * 2;                        // limbs g0 g1 g2 h0 of each staged row
+  uint2* sl2 = reinterpret_cast<uint2*>(sl4 + kHistTileRows);    // and h1 h2
+  __shared__ int32_t s_vlen[32], s_vstart[32];
+  if (tid < 32) {
+    const int f = f0 + tid;
+    s_vlen[tid] = f < f1 ? c.feats[f].view_len : 0;
+    s_vstart[tid] = f < f1 ? c.feats[f].view_start : 0;
+  }
+  for (int i = tid; i < kFixedPlanes * kCells / 4; i += kHistThreads)
+    reinterpret_cast<uint4*>(cells)[i] = make_uint4(0u, 0u, 0u, 0u);
+  const uint32_t* idx = lr.idx + lr.begin;
+  double* out = reinterpret_cast<double*>(s.hist) + (size_t)lr.buf * c.total_bins * 2;
+  const int g_limbs = fx.g_limbs, h_limbs = fx.h_limbs, g_bits = fx.g_bits, h_bits = fx.h_bits;
+  const int32_t g_base = fx.g_base, h_base = fx.h_base;
+  const int32_t flush_rows = fx.rows;
+  // the sums of one value's limbs: exact below 2^53 in the low two, then rounded once
+  auto value_of = [&](int plane, int i, int limbs, int bits, int32_t base) {
+    const double w = ldexp(1.0, bits);
+    const double v0 = (double)(uint32_t)cells[plane * kCells + i];
+    const int32_t c1 = cells[(plane + 1) * kCells + i];
+    if (limbs == 2) return ldexp(v0 + (double)c1 * w, base);
+    const double low = v0 + (double)(uint32_t)c1 * w;
+    return ldexp((double)cells[(plane + 2) * kCells + i] * w * w + low, base);
+  };
+  auto flush = [&]() {
+    for (int i = tid; i < kCells; i += kHistThreads) {
+      const int raw = i >> 5, fl = i & 31;
+      if (raw == 0 || raw > s_vlen[fl]) continue;
+      const double g = value_of(0, i, g_limbs, g_bits, g_base);
+      const double h = h_limbs == 1 ? (double)(uint32_t)cells[3 * kCells + i] * fx.h_value
+                                    : value_of(3, i, h_limbs, h_bits, h_base);
+      double* d = out + 2 * ((size_t)s_vstart[fl] + raw - 1);
+      if (g != 0.0) atomicAdd(d, g);
+      if (h != 0.0) atomicAdd(d + 1, h);
+    }
+  };
+  // this thread's row of the next tile, its index two tiles ahead
+  auto load_idx = [&](int64_t pos) { return pos < r1 ? __ldcg(idx + pos) : 0u; };
+  float2 ngh;
+  uint4 nb[2];
+  bool nlive;
+  auto fetch = [&](int64_t pos, uint32_t row) {
+    nlive = pos < r1;
+    ngh = nlive ? s.gh[row] : make_float2(0.f, 0.f);
+    const uint4* src = reinterpret_cast<const uint4*>(c.bins + (size_t)row * c.stride + f0);
+    nb[0] = nlive ? __ldg(src) : make_uint4(0u, 0u, 0u, 0u);
+    nb[1] = nlive ? __ldg(src + 1) : make_uint4(0u, 0u, 0u, 0u);
+  };
+  uint32_t ahead;
+  {
+    const uint32_t first = load_idx(r0 + tid);
+    ahead = load_idx(r0 + kHistTileRows + tid);
+    fetch(r0 + tid, first);
+  }
+  const uint32_t cell0 = (uint32_t)__cvta_generic_to_shared(cells) + 4u * (uint32_t)lane;
+  int32_t since = 0;
+  __syncthreads();
+  for (int64_t t0 = r0; t0 < r1; t0 += kHistTileRows) {
+    const int tile_rows = (int)min((int64_t)kHistTileRows, r1 - t0);
+    {
+      const long long g = fixed_of(ngh.x, g_base);
+      const uint32_t gm = (1u << g_bits) - 1u, hm = (1u << h_bits) - 1u;
+      uint4 a;
+      uint2 b = make_uint2(0u, 0u);
+      a.x = (uint32_t)g & gm;
+      a.y = g_limbs == 2 ? (uint32_t)(g >> g_bits) : (uint32_t)(g >> g_bits) & gm;
+      a.z = (uint32_t)(g >> (2 * g_bits));
+      if (h_limbs == 1) {
+        a.w = nlive ? 1u : 0u;
+      } else {
+        const long long h = fixed_of(ngh.y, h_base);
+        a.w = (uint32_t)h & hm;
+        b.x = h_limbs == 2 ? (uint32_t)(h >> h_bits) : (uint32_t)(h >> h_bits) & hm;
+        b.y = (uint32_t)(h >> (2 * h_bits));
+      }
+      sl4[tid] = a;
+      sl2[tid] = b;
+      sbins[2 * tid] = nb[0];
+      sbins[2 * tid + 1] = nb[1];
+    }
+    __syncthreads();
+    if (t0 + kHistTileRows < r1) {
+      fetch(t0 + kHistTileRows + tid, ahead);
+      ahead = load_idx(t0 + 2 * kHistTileRows + tid);
+    }
+    const int rw0 = warp * 32;
+    if (rw0 < tile_rows) {
+      const unsigned char* rowp = reinterpret_cast<const unsigned char*>(sbins) + rw0 * 32 + lane;
+#pragma unroll 1
+      for (int jb = 0; jb < 32; jb += 8) {
+        uint32_t raw[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) raw[u] = rowp[(jb + u) * 32];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const uint4 a = sl4[rw0 + jb + u];
+          const uint32_t at = cell0 + (raw[u] << 7);
+          asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(at), "r"(a.x) : "memory");
+          asm volatile("red.shared.add.u32 [%0+32768], %1;" ::"r"(at), "r"(a.y) : "memory");
+          if (g_limbs == 3) asm volatile("red.shared.add.u32 [%0+65536], %1;" ::"r"(at), "r"(a.z) : "memory");
+          asm volatile("red.shared.add.u32 [%0+98304], %1;" ::"r"(at), "r"(a.w) : "memory");
+          if (h_limbs > 1) {
+            const uint2 b = sl2[rw0 + jb + u];
+            asm volatile("red.shared.add.u32 [%0+131072], %1;" ::"r"(at), "r"(b.x) : "memory");
+            if (h_limbs == 3) asm volatile("red.shared.add.u32 [%0+163840], %1;" ::"r"(at), "r"(b.y) : "memory");
+          }
+        }
+      }
+    }
+    since += tile_rows;
+    __syncthreads();
+    if (t0 + kHistTileRows < r1 && since + kHistTileRows > flush_rows) {
+      flush();
+      __syncthreads();
+      for (int i = tid; i < kFixedPlanes * kCells / 4; i += kHistThreads)
+        reinterpret_cast<uint4*>(cells)[i] = make_uint4(0u, 0u, 0u, 0u);
+      since = 0;
+      __syncthreads();
+    }
+  }
+  flush();
+  __syncthreads();
 }
 
 __device__ void deferred_finish(const DCtx& c, const DSlot& s, void* dec_smem);

@@ -201,6 +201,7 @@ __global__ void __launch_bounds__(kHistThreads, 2)
   const int tid = threadIdx.x;
   const bool root = r.st->root != 0;
   const int32_t nb = root ? 1 : r.st->nb, e0 = r.st->e0;
+  const DFixed fx = s.st->fx;
   long long w = 0;
   if (tid < nb) {
     int32_t id = 0;
@@ -239,8 +240,19 @@ __global__ void __launch_bounds__(kHistThreads, 2)
     lr.count = start[i + 1] - s0;
     lr.buf = buf[i] & 0x3FFFFFFF;
     lr.idx = s.idx[buf[i] >> 30 & 1];
+    if constexpr (kMode != 2) {
+      if (fx.ok) {
+        hist_body_fixed(c, s, fx, tt, blockIdx.y, lr, r0, r1, smem_raw);
+        continue;
+      }
+    }
     hist_body<kMode, kNG, 1>(c, s, tt, blockIdx.y, lr, r0, r1, sub_rows, smem_raw);
   }
+}
+
+size_t round_hist_smem(int mode, int ng) {
+  const size_t b = hist_smem_bytes(mode, ng);
+  return mode == 2 ? b : std::max(b, kFixedSmem);
 }
 
 #define LGBM_B200_ROUND_HIST_INST(M, G) \
