@@ -944,25 +944,30 @@ __device__ void hist_body_fixed(const DCtx& c, const DSlot& s, const DFixed& fx,
   const int g_limbs = fx.g_limbs, h_limbs = fx.h_limbs, g_bits = fx.g_bits, h_bits = fx.h_bits;
   const int32_t g_base = fx.g_base, h_base = fx.h_base;
   const int32_t flush_rows = fx.rows;
-  // the sums of one value's limbs: exact below 2^53 in the low two, then rounded once
-  auto value_of = [&](int plane, int i, int limbs, int bits, int32_t base) {
-    const double w = ldexp(1.0, bits);
-    const double v0 = (double)(uint32_t)cells[plane * kCells + i];
-    const int32_t c1 = cells[(plane + 1) * kCells + i];
-    if (limbs == 2) return ldexp(v0 + (double)c1 * w, base);
-    const double low = v0 + (double)(uint32_t)c1 * w;
-    return ldexp((double)cells[(plane + 2) * kCells + i] * w * w + low, base);
+  // the sums of one value's limbs: exact below 2^53 in the low two, then
+  // rounded once (the powers of two are exact)
+  const double gw = (double)(1u << g_bits), hw = (double)(1u << h_bits);
+  const double gs = ldexp(1.0, g_base), hs = h_limbs == 1 ? fx.h_value : ldexp(1.0, h_base);
+  auto value_of = [&](const int32_t* p, int limbs, double w, double scale) {
+    double v = (double)(uint32_t)p[0];
+    if (limbs == 2) v += (double)p[kCells] * w;
+    else if (limbs == 3) v = (double)p[2 * kCells] * (w * w) + (v + (double)(uint32_t)p[kCells] * w);
+    return v * scale;
   };
   auto flush = [&]() {
-    for (int i = tid; i < kCells; i += kHistThreads) {
-      const int raw = i >> 5, fl = i & 31;
-      if (raw == 0 || raw > s_vlen[fl]) continue;
-      const double g = value_of(0, i, g_limbs, g_bits, g_base);
-      const double h = h_limbs == 1 ? (double)(uint32_t)cells[3 * kCells + i] * fx.h_value
-                                    : value_of(3, i, h_limbs, h_bits, h_base);
-      double* d = out + 2 * ((size_t)s_vstart[fl] + raw - 1);
-      if (g != 0.0) atomicAdd(d, g);
-      if (h != 0.0) atomicAdd(d + 1, h);
+    const int32_t vlen = s_vlen[lane];  // cell i belongs to feature i % 32, this lane's
+    double* base = out + 2 * ((size_t)s_vstart[lane] - 1);
+#pragma unroll 4
+    for (int raw = warp; raw < kMaxBins; raw += kHistThreads / 32) {
+      const int32_t* p = cells + raw * 32 + lane;
+      const int32_t g0 = p[0], g1 = p[kCells], h0 = p[3 * kCells], h1 = h_limbs > 1 ? p[4 * kCells] : 0;
+      if (raw == 0 || raw > vlen || (g0 | g1 | h0 | h1) == 0) {
+        // a third limb alone: only where the low ones wrapped to zero together
+        if (raw == 0 || raw > vlen || !((g_limbs == 3 && p[2 * kCells]) || (h_limbs == 3 && p[5 * kCells]))) continue;
+      }
+      const double g = value_of(p, g_limbs, gw, gs), h = value_of(p + 3 * kCells, h_limbs, hw, hs);
+      if (g != 0.0) atomicAdd(base + 2 * raw, g);
+      if (h != 0.0) atomicAdd(base + 2 * raw + 1, h);
     }
   };
   // this thread's row of the next tile, its index two tiles ahead

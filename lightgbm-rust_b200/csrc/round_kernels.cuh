@@ -298,8 +298,8 @@ struct NodeFacts {
   const int32_t* exp_node;
 };
 size_t round_decide_smem(int num_leaves) {
-  // the replayed tree's leaves (gain, feature, node), then the nodes' facts
-  const size_t leaves = ((size_t)num_leaves * (sizeof(double) + 2 * sizeof(int32_t)) + 15) / 16 * 16;
+  // the replayed tree's leaves, then the nodes' facts
+  const size_t leaves = ((size_t)num_leaves * sizeof(int32_t) + 15) / 16 * 16;
   return leaves + (size_t)kDecideSmemNodes * (sizeof(double) + 2 * sizeof(int32_t)) + kDecideSmemNodes / 2 * sizeof(int32_t);
 }
 
@@ -312,13 +312,11 @@ __device__ __forceinline__ unsigned long long order_key(double v) {
 // The reference's order of splits (learner/mod.rs:653-706) replayed by one
 // warp over the gains found so far, from `popped` splits on: the leaf of
 // largest gain (then smallest feature, then smallest leaf) is split as long
-// as it has been expanded. lg / lf / ln: gain, feature and node of each leaf
-// of the replayed tree. Returns the node the replay waits for, or -1 when the
+// as it has been expanded. ln: the node of each leaf of the replayed tree. Returns the node the replay waits for, or -1 when the
 // tree is finished. Lane l owns leaves l, l + 32, ...; up to 256 leaves their
 // gains stay in registers.
 template <bool kRegs>
-__device__ int32_t replay(const DRounds& r, const NodeFacts& nd, double* lg, int32_t* lf, int32_t* ln, int32_t need,
-                          int32_t& popped) {
+__device__ int32_t replay(const DRounds& r, const NodeFacts& nd, int32_t* ln, int32_t need, int32_t& popped) {
   const int lane = threadIdx.x & 31;
   unsigned long long own[kReplaySlots];  // order keys of this lane's leaves
   unsigned long long best = 0;           // the largest, 0: none
@@ -330,15 +328,15 @@ __device__ int32_t replay(const DRounds& r, const NodeFacts& nd, double* lg, int
 #pragma unroll
       for (int k = 0; k < kReplaySlots; ++k) {
         const int32_t l = lane + 32 * k;
-        if (l < leaves && (own[k] > best || (own[k] == best && bl != INT32_MAX && better_than(0.0, lf[l], 0.0, lf[bl])))) {
+        if (l < leaves && (own[k] > best || (own[k] == best && bl != INT32_MAX && better_than(0.0, nd.feat[ln[l]], 0.0, nd.feat[ln[bl]])))) {
           best = own[k];
           bl = l;
         }
       }
     } else {
       for (int32_t l = lane; l < leaves; l += 32) {
-        const unsigned long long k = order_key(lg[l]);
-        if (k > best || (k == best && bl != INT32_MAX && better_than(0.0, lf[l], 0.0, lf[bl]))) {
+        const unsigned long long k = order_key(nd.gain[ln[l]]);
+        if (k > best || (k == best && bl != INT32_MAX && better_than(0.0, nd.feat[ln[l]], 0.0, nd.feat[ln[bl]]))) {
           best = k;
           bl = l;
         }
@@ -347,7 +345,7 @@ __device__ int32_t replay(const DRounds& r, const NodeFacts& nd, double* lg, int
   };
   if constexpr (kRegs) {
 #pragma unroll
-    for (int k = 0; k < kReplaySlots; ++k) own[k] = lane + 32 * k <= popped ? order_key(lg[lane + 32 * k]) : 0ull;
+    for (int k = 0; k < kReplaySlots; ++k) own[k] = lane + 32 * k <= popped ? order_key(nd.gain[ln[lane + 32 * k]]) : 0ull;
   }
   own_best(popped + 1);
   const unsigned long long zero = order_key(0.0);
@@ -361,7 +359,7 @@ __device__ int32_t replay(const DRounds& r, const NodeFacts& nd, double* lg, int
       in = in && (uint32_t)best == lo;
       who = __ballot_sync(0xffffffffu, in);
       if (who & (who - 1)) {  // equal gains: the smallest feature, then the smallest leaf
-        const int32_t feat = in && bl != INT32_MAX ? lf[bl] : -1;
+        const int32_t feat = in && bl != INT32_MAX ? nd.feat[ln[bl]] : -1;
         const uint32_t fe = !in ? 0xffffffffu : feat == -1 ? (uint32_t)INT32_MAX : (uint32_t)feat;
         const uint32_t mf = __reduce_min_sync(0xffffffffu, fe);
         in = in && fe == mf;
@@ -376,27 +374,19 @@ __device__ int32_t replay(const DRounds& r, const NodeFacts& nd, double* lg, int
     const int32_t v = ln[l], e = nd.exp[v];
     if (e < 0) return v;
     const int32_t R = popped + 1, a = 2 * e + 1, b = 2 * e + 2;
-    const double ga = nd.gain[a], gb = nd.gain[b];
-    const int32_t fa = nd.feat[a], fb = nd.feat[b];
+    const unsigned long long ka = order_key(nd.gain[a]), kb = order_key(nd.gain[b]);
     __syncwarp();
     if (lane == 0) {
       nd.exp[v] = e | kReplayed;
       r.exp[v] = e | kReplayed;
       r.pop_node[popped] = v;
       r.pop_leaf[popped] = l;
-      lf[l] = fa;
       ln[l] = a;
-      lf[R] = fb;
       ln[R] = b;
-      if (!kRegs) {
-        lg[l] = ga;
-        lg[R] = gb;
-      }
     }
     __syncwarp();
     ++popped;
     if constexpr (kRegs) {
-      const unsigned long long ka = order_key(ga), kb = order_key(gb);
 #pragma unroll
       for (int k = 0; k < kReplaySlots; ++k) {
         if (l == lane + 32 * k) own[k] = ka;
@@ -434,8 +424,9 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
   __shared__ int32_t exps[kRoundBins], cands[kRoundBins];
   __shared__ unsigned long long rows[kRoundBins];
   __shared__ unsigned long long warp_sums[kDecideThreads / 32];
+  __shared__ int32_t fresh[kMaxRoundItems];
   __shared__ uint32_t s_lo;
-  __shared__ int32_t s_popped, s_top, s_tau, s_cut, s_room, s_rowcut;
+  __shared__ int32_t s_popped, s_top, s_tau, s_cut, s_room, s_rowcut, s_tiles;
   const DSlot& s = c.slots[blockIdx.z];
   const DRounds& r = s.r;
   RoundState* rs = r.st;
@@ -447,12 +438,10 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
     const int32_t E = st.e0 + st.nb, N = 2 * E + 1;
     const int32_t new0 = st.root ? 0 : 2 * st.e0 + 1, nnew = N - new0;
     const int32_t total = st.ncand + nnew;  // the candidates: those kept, then the new nodes
-    double* lg = reinterpret_cast<double*>(smem_raw);
-    int32_t* lf = reinterpret_cast<int32_t*>(lg + L);
-    int32_t* ln = lf + L;
+    int32_t* ln = reinterpret_cast<int32_t*>(smem_raw);
     NodeFacts nd{r.gain, r.feat, r.exp, r.exp_node};
     if (N <= kDecideSmemNodes) {
-      double* a = reinterpret_cast<double*>(smem_raw + ((size_t)L * (sizeof(double) + 2 * sizeof(int32_t)) + 15) / 16 * 16);
+      double* a = reinterpret_cast<double*>(smem_raw + ((size_t)L * sizeof(int32_t) + 15) / 16 * 16);
       int32_t* b = reinterpret_cast<int32_t*>(a + N);
       int32_t* d = b + N;
       int32_t* e = d + N;
@@ -464,24 +453,28 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
       for (int32_t i = tid; i < E; i += kDecideThreads) e[i] = r.exp_node[i];
       nd = NodeFacts{a, b, d, e};
     }
-    for (int32_t l = tid; l <= st.popped; l += kDecideThreads) {
-      const int32_t v = r.leaf_node[l];
-      ln[l] = v;
-      lg[l] = r.gain[v];
-      lf[l] = r.feat[v];
-    }
+    for (int32_t l = tid; l <= st.popped; l += kDecideThreads) ln[l] = r.leaf_node[l];
     // this thread's first kOwn candidates and their rows stay in registers
     // (more only in trees of a thousand leaves); loaded while the replay runs
     constexpr int kOwn = 2;
     auto listed = [&](int32_t i) { return i < st.ncand ? r.cand[i] : new0 + i - st.ncand; };
-    int32_t own_v[kOwn], own_n[kOwn];
+    int32_t own_v[kOwn], own_n[kOwn], own_begin[kOwn], own_side[kOwn], own_buf[kOwn], own_inner[kOwn];
 #pragma unroll
     for (int j = 0; j < kOwn; ++j) {
       const int32_t i = tid + j * kDecideThreads;
       own_v[j] = i < total ? listed(i) : -1;
     }
 #pragma unroll
-    for (int j = 0; j < kOwn; ++j) own_n[j] = own_v[j] >= 0 ? r.node[own_v[j]].count : 0;
+    for (int j = 0; j < kOwn; ++j) {
+      const RNode& nv = r.node[max(own_v[j], 0)];
+      own_n[j] = own_v[j] >= 0 ? nv.count : 0;
+      own_begin[j] = nv.begin;
+      own_side[j] = nv.side;
+      own_buf[j] = nv.buf;
+      own_inner[j] = r.best[max(own_v[j], 0)].inner;
+    }
+    // the buffers the round may take, from the end of the list
+    for (int i = tid; i < min(r.bmax, st.nfree); i += kDecideThreads) fresh[i] = r.free[st.nfree - 1 - i];
     for (int b = tid; b < kRoundBins; b += kDecideThreads) {
       exps[b] = 0;
       cands[b] = 0;
@@ -497,8 +490,8 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
     __syncthreads();
     if (tid < 32) {
       int32_t popped = st.popped;
-      const int32_t top = L <= 32 * kReplaySlots ? replay<true>(r, nd, lg, lf, ln, need, popped)
-                                                 : replay<false>(r, nd, lg, lf, ln, need, popped);
+      const int32_t top = L <= 32 * kReplaySlots ? replay<true>(r, nd, ln, need, popped)
+                                                 : replay<false>(r, nd, ln, need, popped);
       if (tid == 0) {
         s_popped = popped;
         s_top = top;
@@ -525,25 +518,32 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
         }
         return __float_as_uint(k);
       };
+      auto tiles_of = [](int32_t n) { return (n + kPartTileRows - 1) / kPartTileRows; };
       const uint32_t hi = key_of(top);  // no key is larger
       uint32_t own_k[kOwn];
-      // visits this thread's candidates: fn(i, node, rows, key), for every
-      // multiple of kDecideThreads below `total` (node -1 past it)
+      // visits this thread's candidates: fn(candidate), for every multiple of
+      // kDecideThreads below `total` (node -1 past it)
+      struct Cand {
+        int32_t v, n, begin, side, buf, inner;
+        uint32_t key;
+      };
       auto each_cand = [&](auto fn) {
 #pragma unroll
         for (int j = 0; j < kOwn; ++j)
-          if (j * kDecideThreads < total) fn(tid + j * kDecideThreads, own_v[j], own_n[j], own_k[j]);
+          if (j * kDecideThreads < total)
+            fn(Cand{own_v[j], own_n[j], own_begin[j], own_side[j], own_buf[j], own_inner[j], own_k[j]});
         for (int32_t i0 = kOwn * kDecideThreads; i0 < total; i0 += kDecideThreads) {
           const int32_t i = i0 + tid, v = i < total ? listed(i) : -1;
-          fn(i, v, v >= 0 ? r.node[v].count : 0, v >= 0 ? key_of(v) : 0u);
+          const RNode& nv = r.node[max(v, 0)];
+          fn(Cand{v, nv.count, nv.begin, nv.side, nv.buf, r.best[max(v, 0)].inner, v >= 0 ? key_of(v) : 0u});
         }
       };
       {
         uint32_t lo = 0xffffffffu;
 #pragma unroll
         for (int j = 0; j < kOwn; ++j) own_k[j] = own_v[j] >= 0 ? key_of(own_v[j]) : 0u;
-        each_cand([&](int32_t, int32_t, int32_t, uint32_t k) {
-          if (k > 0) lo = min(lo, k);
+        each_cand([&](const Cand& x) {
+          if (x.key > 0) lo = min(lo, x.key);
         });
         lo = __reduce_min_sync(0xffffffffu, lo);
         if ((tid & 31) == 0) atomicMin(&s_lo, lo);
@@ -552,12 +552,13 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
       const int shift = max(0, 32 - __clz(hi - min(hi, s_lo)) - 10);
       static_assert(kRoundBins == 1 << 10, "the range of keys shifted to ten bits");
       auto bin_of = [&](uint32_t k) { return k ? min((int32_t)((hi - k) >> shift), kRoundBins - 1) : kRoundBins; };
-      each_cand([&](int32_t, int32_t v, int32_t n, uint32_t k) {
-        const int32_t b = bin_of(k);
+      each_cand([&](const Cand& x) {
+        const int32_t b = bin_of(x.key);
         if (b < kRoundBins) {
-          if (n <= kRoundRows / 2 && v != top) atomicAdd(&rows[b], (unsigned long long)n);
+          if (x.n <= kRoundRows / 2 && x.v != top) atomicAdd(&rows[b], (unsigned long long)x.n);
           atomicAdd(&cands[b], 1);
         }
+        if (x.v == top) s_tiles = tiles_of(x.n);
       });
       for (int32_t e = tid; e < E; e += kDecideThreads) {
         const int32_t v = nd.exp_node[e];
@@ -593,32 +594,21 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
       // node the replay waits for is always the first), the ones kept, and the
       // buffers of the ones dropped
       int32_t took = 1, kept = 0, freed = 0, tiles = 0, at_cut0 = 0;
-      auto place = [&](int32_t at, int32_t v, int32_t tile0) {
-        const RNode& nd = r.node[v];
-        RItem it;
-        it.node = v;
-        it.begin = nd.begin;
-        it.count = nd.count;
-        it.side = nd.side;
-        it.inner = r.best[v].inner;
-        it.tile0 = tile0;
-        it.buf = r.free[st.nfree - 1 - at];
-        it.pad = 0;
-        r.item[at] = it;
-        r.exp_node[E + at] = v;
-        r.exp[v] = E + at;
+      auto place = [&](int32_t at, const Cand& x, int32_t tile0) {
+        r.item[at] = RItem{x.v, x.begin, x.n, x.side, x.inner, tile0, fresh[at], 0};
+        r.exp_node[E + at] = x.v;
+        r.exp[x.v] = E + at;
         r.scan_cnt[2 * at] = 0;
         r.scan_cnt[2 * at + 1] = 0;
       };
-      auto tiles_of = [](int32_t n) { return (n + kPartTileRows - 1) / kPartTileRows; };
-      tiles = tiles_of(r.node[top].count);
-      if (tid == 0) place(0, top, 0);
-      each_cand([&](int32_t, int32_t v, int32_t n, uint32_t k) {
+      tiles = s_tiles;
+      each_cand([&](const Cand& x) {
         bool pick = false, keep = false, drop = false, edge = false;
-        if (v >= 0 && v != top) {
-          const int32_t b = bin_of(k);
+        if (x.v == top) place(0, x, 0);
+        if (x.v >= 0 && x.v != top) {
+          const int32_t b = bin_of(x.key);
           drop = b > tau;
-          const bool fits = !drop && n <= kRoundRows / 2 && b < rowcut;
+          const bool fits = !drop && x.n <= kRoundRows / 2 && b < rowcut;
           pick = fits && b < cut;
           edge = fits && b == cut;
           keep = !drop;
@@ -630,17 +620,17 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
         at_cut0 += (int32_t)tot;
         keep = keep && !pick;
         // one sum of four counts: tiles (32 bits), picked, kept and dropped (10 bits each)
-        const int32_t nt = tiles_of(n);
+        const int32_t nt = tiles_of(x.n);
         const unsigned long long before = block_prefix<kDecideThreads>(
             (pick ? (1ull << 32) | (uint32_t)nt : 0ull) | (unsigned long long)keep << 42 | (unsigned long long)drop << 52,
             warp_sums, tot);
         static_assert(kDecideThreads < 1024, "ten bits a count");
         const int32_t at = took + (int32_t)(before >> 32 & 1023);
-        if (pick && at < r.bmax && E + at < r.ecap) place(at, v, tiles + (int32_t)(uint32_t)before);
+        if (pick && at < r.bmax && E + at < r.ecap) place(at, x, tiles + (int32_t)(uint32_t)before);
         // the list is compacted in place: an entry moves to a place at or
         // before its own, which this pass or an earlier one has read
-        if (keep) r.cand[kept + (int32_t)(before >> 42 & 1023)] = v;
-        if (drop) r.free_next[freed + (int32_t)(before >> 52)] = r.node[v].buf;
+        if (keep) r.cand[kept + (int32_t)(before >> 42 & 1023)] = x.v;
+        if (drop) r.free_next[freed + (int32_t)(before >> 52)] = x.buf;
         took += (int32_t)(tot >> 32 & 1023);
         tiles += (int32_t)(uint32_t)tot;
         kept += (int32_t)(tot >> 42 & 1023);
@@ -671,7 +661,10 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
     }
   }
   // whether any slot goes on: by the last slot's CTA
-  if (tid == 0) {
+  if (tid == 0 && gridDim.z == 1) {
+    ctrl[2] = active;
+    if (use_cond) cudaGraphSetConditional(cond, (unsigned)active);
+  } else if (tid == 0) {
     if (active) atomicAdd(&ctrl[1], 1);
     __threadfence();
     if (atomicAdd(&ctrl[0], 1) == (int)gridDim.z - 1) {

@@ -500,56 +500,74 @@ __device__ __forceinline__ ScanSpan scan_span(const DFeature& m, bool reverse, b
   return v;
 }
 
+// A serial chain of adds (sign 1) or subtractions (-1) over `segs` chunks of
+// kPer values of x, in order, each replaced by its running value if `store`.
+// Values that take no part are zeros (a running sum here is never -0.0, so
+// adding zero changes nothing), which leaves a load, an add and a store per
+// value: with the visited tests in the loop a chain took 45 cycles a value.
+// The next chunk is loaded while this one is added.
+__device__ __noinline__ double f64_chain(double a, double* x, int segs, double sign, bool store) {
+  double v[kPer], next[kPer];
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) v[i] = x[i];
+  for (int k = 0; k < segs; ++k, x += kPer + 1) {
+    if (k + 1 < segs) {
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) next[i] = x[kPer + 1 + i];
+    }
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) v[i] = a = a + sign * v[i];
+    if (store) {
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) x[i] = v[i];
+    }
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) v[i] = next[i];
+  }
+  return a;
+}
+
 // The cumulative sums of both directions in the reference's order
 // (split.rs:676-891), four serial chains side by side: lane 0 adds the
 // gradients in reverse, lane 1 the hessians, lanes 2 and 3 the same forward
 // (two: both directions are scanned). The forward chain starts, for a feature
 // with NaN missing and no stored bin 0, from the leaf's sums minus every
-// stored bin (split.rs:787-800), which `base` returns.
+// stored bin (split.rs:787-800), which base_g / base_h return. Past its length
+// the view holds zeros. The reverse sums of bin t lie at place 8 * segs - 1 - t,
+// so that all lanes run forward.
 __device__ __forceinline__ void f64_chains(F64Scratch& sm, const LeafCtx& lc, const ScanSpan& rev, const ScanSpan& fwd,
                                            int len, bool two, bool first_extra, double& base_g, double& base_h) {
   const int lane = threadIdx.x & 31;
-  const bool forward = lane >= 2, hess = lane & 1;
-  const double* x = sm.view[hess];
-  double* cum = sm.cum[lane & 3];
+  const bool forward = (lane & 3) >= 2 && two, hess = lane & 1;
+  const int segs = (len + kPer - 1) / kPer, last = kPer * segs - 1;
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int t = 32 * k + lane;
+    if (t > last) continue;
+    const double g = sm.view[0][view_at(t)], h = sm.view[1][view_at(t)];
+    sm.cum[0][view_at(last - t)] = rev.has(t) ? g : 0.0;
+    sm.cum[1][view_at(last - t)] = rev.has(t) ? h : 0.0;
+    if (two) {
+      sm.cum[2][view_at(t)] = fwd.has(t) ? g : 0.0;
+      sm.cum[3][view_at(t)] = fwd.has(t) ? h : 0.0;
+    }
+  }
   double a = hess ? kEpsilon : 0.0;
   if (first_extra) {
-    double b = hess ? lc.sum_h - kEpsilon : lc.sum_g;
-    for (int t0 = 0; t0 < len; t0 += kPer) {
-      double v[kPer];
-#pragma unroll
-      for (int k = 0; k < kPer; ++k) v[k] = x[view_at(t0 + k)];
-#pragma unroll
-      for (int k = 0; k < kPer; ++k)
-        if (t0 + k < len) b -= v[k];
-    }
+    const double b = f64_chain(hess ? lc.sum_h - kEpsilon : lc.sum_g, sm.view[hess], segs, -1.0, false);
     if (forward) a = b;
     base_g = __shfl_sync(0xffffffffu, b, 2);
     base_h = __shfl_sync(0xffffffffu, b, 3);
   }
-  const ScanSpan span = forward ? fwd : rev;
-  const int segs = (len + kPer - 1) / kPer, step = forward ? 1 : -1;
-  const bool mine = lane < (two ? 4 : 2);
-  for (int k = 0; k < segs; ++k) {
-    const int t0 = forward ? k * kPer : (segs - 1 - k) * kPer + kPer - 1;
-    double v[kPer];
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) v[i] = x[view_at(t0 + step * i)];
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-      if (span.has(t0 + step * i)) a += v[i];
-      v[i] = a;
-    }
-    if (mine) {
-#pragma unroll
-      for (int i = 0; i < kPer; ++i) cum[view_at(t0 + step * i)] = v[i];
-    }
-  }
+  __syncwarp();
+  // lanes past the chains repeat them without storing
+  f64_chain(a, sm.cum[(forward ? 2 : 0) + hess], segs, 1.0, lane < (two ? 4 : 2));
   __syncwarp();
 }
 
 // One direction of FindBestThresholdSequentially (split.rs:676-891) by one
-// warp, lane l on bins 8l .. 8l + 7, over the cumulative sums in cg / ch.
+// warp, lane l on bins 8l .. 8l + 7, over the cumulative sums in cg / ch
+// (f64_chains).
 __device__ __forceinline__ bool scan_direction_f64(const double* cg, const double* ch, const double* view_h,
                                                    const ScanSpan& span, const DFeature& m, const DParams& p,
                                                    const LeafCtx& lc, double min_gain_shift, double cnt_factor,
@@ -610,13 +628,15 @@ __device__ __forceinline__ bool scan_direction_f64(const double* cg, const doubl
   auto estimate = [&](double a, double b) {
     return gain_estimate((float)a, (float)b, (float)(lc.sum_g - a), (float)(lc.sum_h - b), l2f);
   };
+  const int last = (len + kPer - 1) / kPer * kPer - 1;
   double a[kPer], b[kPer];
   float est[kPer];
   uint32_t pend = 0, stop = 0;
 #pragma unroll
   for (int j = 0; j < kPer; ++j) {
-    a[j] = cg[view_at(lane * kPer + j)];
-    b[j] = ch[view_at(lane * kPer + j)];
+    const int t = lane * kPer + j, at = view_at(reverse ? max(0, last - t) : t);
+    a[j] = cg[at];
+    b[j] = ch[at];
     est[j] = estimate(a[j], b[j]);
     if ((visited >> j & 1) && !low(b[j], n[j])) (ends(b[j], n[j]) ? stop : pend) |= 1u << j;
   }
@@ -787,20 +807,13 @@ __global__ void __launch_bounds__(kF64ScanThreads, kScanF64Blocks) k_round_scan_
       if (m.most_freq_bin > 0) {
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
-          sm.view[0][view_at(32 * k + lane)] = v[k].x;
-          sm.view[1][view_at(32 * k + lane)] = v[k].y;
+          const bool own = 32 * k + lane != m.most_freq_bin;
+          sm.view[0][view_at(32 * k + lane)] = own ? v[k].x : 0.0;
+          sm.view[1][view_at(32 * k + lane)] = own ? v[k].y : 0.0;
         }
         __syncwarp();
-        const double* x = sm.view[lane & 1];
-        double a = (lane & 1) ? j.sl.sum_hessians : j.sl.sum_gradients;
-        for (int t0 = 0; t0 < m.num_bin; t0 += kPer) {
-          double u[kPer];
-#pragma unroll
-          for (int k = 0; k < kPer; ++k) u[k] = x[view_at(t0 + k)];
-#pragma unroll
-          for (int k = 0; k < kPer; ++k)
-            if (t0 + k < m.num_bin && t0 + k != m.most_freq_bin) a -= u[k];
-        }
+        const double a = f64_chain((lane & 1) ? j.sl.sum_hessians : j.sl.sum_gradients, sm.view[lane & 1],
+                                   (len + kPer - 1) / kPer, -1.0, false);
         const double2 fixed = make_double2(__shfl_sync(0xffffffffu, a, 0), __shfl_sync(0xffffffffu, a, 1));
 #pragma unroll
         for (int k = 0; k < kPer; ++k)
