@@ -187,6 +187,7 @@ struct DRounds {
   RCopy* copy;           // [ecap + 1]
   unsigned long long* status;  // look-back words of a round's row tiles
   int32_t ecap, bmax, pool;
+  int32_t share, least;  // a round expands at most 1 / share of the splits to come, but may take `least`
 };
 constexpr int kRoundBins = 1024;
 constexpr int32_t kReplayed = 1 << 30;
@@ -242,6 +243,7 @@ struct DCtx {
   int32_t bagging;     // 1 when the in-bag rows are a strict subset
   const DFeature* feats;
   DParams p;
+  DParams p_cat;           // p with cat_l2 added to lambda_l2, for categorical splits of several bins
   DSlot slots[kMaxSlots];  // by value: read from the constant bank
   int32_t num_slots;
   int32_t rows_per_block;  // histogram rows per CTA (minimum)

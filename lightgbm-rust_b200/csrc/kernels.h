@@ -109,10 +109,9 @@ __global__ void k_partition(const __grid_constant__ DCtx c);
 __global__ void k_finish(const __grid_constant__ DCtx c);
 // Growth in rounds (round_kernels.cuh).
 constexpr int kMaxRoundItems = 256;     // expansions per round at most
-constexpr int kRoundMin = 24;           // and the least a round may take when that many are worth it
 constexpr int kF64ScanThreads = 128;
 constexpr int kScanF64Blocks = 4;       // CTAs of the FP64 scan per SM
-constexpr int kScanIntBlocks = 3;       // CTAs of the quantized scan per SM
+constexpr int kScanIntBlocks = 2;       // CTAs of the quantized scan per SM
 constexpr unsigned long long kRoundRows = 8000000;  // rows a round expands on speculation at most
 constexpr int kDecideThreads = 512;
 constexpr int kDecideSmemNodes = 3072;  // explored nodes the replay keeps in shared memory

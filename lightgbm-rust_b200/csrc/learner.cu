@@ -197,21 +197,31 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
   const size_t max_tiles = ((size_t)n + kPartTileRows - 1) / kPartTileRows + 1;
   // Growth in rounds, unless a launch strategy that goes step by step is
   // asked for (data-parallel growth also does, set after this). The explored
-  // tree may hold up to 16 times the splits of the finished one: 1.6 times is
-  // usual, 3 to 5 times on late trees of a run, whose gains hardly fall with
+  // tree may hold up to 16 times the splits of the finished one: 1.4 times is
+  // usual, 2 to 3 times on late trees of a run, whose gains hardly fall with
   // depth. Only the nodes that may still be split hold a histogram, so three
   // times the splits suffice there, less when that would take more than an
   // eighth of the free memory (with none to spare, the rounds shrink to the
   // one node the replay waits for).
   h->rounds = !cfg->persistent_grow && !h->scan_part;
-  int32_t ecap = 0, bmax = 0, pool = 0;
+  int32_t ecap = 0, bmax = 0, pool = 0, share = 6, least = 16;
   if (h->rounds) {
     const int32_t need = L - 1;
     size_t free_b = 0, total_b = 0;
     CU(cudaMemGetInfo(&free_b, &total_b));
     const size_t hist_b = cells * 8 * (size_t)K + 1;
     const size_t node_b = 2 * (sizeof(RNode) + sizeof(DSplit) + (size_t)nf + 64) * (size_t)K;
-    bmax = std::max(1, std::min(kMaxRoundItems, std::max(kRoundMin, (need + 3) / 4)));
+    // A round costs about 50 us however few nodes it expands; an expansion
+    // costs two scans per feature and slot, of which the GPU does about 200 a
+    // microsecond. Many slots and features make a wasted expansion dear:
+    // multiclass K=10 x 200 features 7.7 ms an iteration at a quarter (at least
+    // 24), 6.9 at a sixth (12), 6.5 at a tenth (8); binary x 28 1.24, 1.20 and
+    // 1.4 ms.
+    if (2 * (int64_t)nf * K > 1000) {
+      share = 10;
+      least = 8;
+    }
+    bmax = std::max(1, std::min(kMaxRoundItems, std::max(least, (need + share - 1) / share)));
     ecap = need + (int32_t)std::min<size_t>(15 * (size_t)need, free_b / 16 / node_b);
     pool = need + 1 + (int32_t)std::min<size_t>(2 * (size_t)need + 2 * (size_t)bmax, free_b / 8 / hist_b);
   }
@@ -312,6 +322,8 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
       r.ecap = ecap;
       r.bmax = bmax;
       r.pool = pool;
+      r.share = share;
+      r.least = least;
       r.st = reinterpret_cast<RoundState*>(rbk + rb.rs);
       ALLOC(r.node, nodes);
       ALLOC(r.best, nodes);
@@ -441,6 +453,8 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
   p.max_depth = cfg->max_depth;
   p.monotone_penalty = cfg->monotone_penalty;
   p.use_monotone = use_monotone ? 1 : 0;
+  c.p_cat = p;
+  c.p_cat.lambda_l2 += p.cat_l2;
   for (int k = 0; k < K; ++k) c.slots[k] = h->slots_h[k];
   c.num_slots = K;
   c.rows_per_block = rpb;

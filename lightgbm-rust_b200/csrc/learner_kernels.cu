@@ -1152,12 +1152,16 @@ __device__ __forceinline__ int32_t warp_min_i(int32_t v) {
   return v;
 }
 
-// split.rs:448-670 / :1194-1400 categorical threshold search, in lane 0
-// (the candidate lists are at most a few dozen bins; the stable sort is a
-// rank sort done by the whole warp).
+// split.rs:448-670 / :1194-1400 categorical threshold search, by one warp.
+// The bins are sorted by a rank sort; in each direction lane i takes the split
+// after sorted position i: the sums up to it (in the reference's order; packed
+// ones exact in any), whether it is skipped or ends the direction, and, where
+// the running group is large enough, its gain. (One lane did all of it before,
+// with two FP64 divides per position one after another.) One-hot splits, of a
+// few bins, stay in lane 0.
 template <bool kInt, class Scratch>
-__device__ __noinline__ bool scan_categorical(Scratch& sm, const DFeature& m, const DParams& p, const LeafCtx& lc,
-                                              DSplit& out) {
+__device__ __noinline__ bool scan_categorical(Scratch& sm, const DFeature m, const DParams& p, const DParams& p_cat,
+                                              const LeafCtx lc, DSplit& out) {
   const int lane = threadIdx.x & 31;
   const int offset = m.offset;
   const int bin_start = 1 - offset, bin_end = m.num_bin - offset;
@@ -1185,11 +1189,13 @@ __device__ __noinline__ bool scan_categorical(Scratch& sm, const DFeature& m, co
   int32_t used_bin = 0;
   if (!use_onehot) {
     // bins with enough data, then a stable sort by sum_grad / (sum_hess + cat_smooth)
-    if (lane == 0) {
-      for (int i = bin_start; i < bin_end; ++i)
-        if ((double)CNT(i) >= p.cat_smooth) sm.tpos[used_bin++] = i;
+    for (int i0 = bin_start; i0 < bin_end; i0 += 32) {
+      const int i = i0 + lane;
+      const bool in = i < bin_end && (double)CNT(i) >= p.cat_smooth;
+      const unsigned mask = __ballot_sync(0xffffffffu, in);
+      if (in) sm.tpos[used_bin + __popc(mask & ((1u << lane) - 1u))] = i;
+      used_bin += __popc(mask);
     }
-    used_bin = __shfl_sync(0xffffffffu, used_bin, 0);
     __syncwarp();
     for (int k = lane; k < used_bin; k += 32) {
       int i = sm.tpos[k];
@@ -1208,16 +1214,106 @@ __device__ __noinline__ bool scan_categorical(Scratch& sm, const DFeature& m, co
     __syncwarp();
   }
   bool is_splittable = false;
+  const double gain_shift = use_smoothing(p) ? leaf_gain_given_output(sum_gradient, sum_hessian, p, lc.parent_output)
+                                             : leaf_gain(sum_gradient, sum_hessian, p, lc.num_data, 0.0);
+  const double min_gain_shift = gain_shift + p.min_gain_to_split;
+  const DParams& pc = use_onehot ? p : p_cat;
+  double best_gain = -INFINITY;
+  int32_t best_left_count = 0, best_threshold = -1, best_dir = 1;
+  double best_slg = 0.0, best_slh = 0.0;
+  int64_t best_left_int = 0;
+  if (!use_onehot) {
+    const int32_t steps = min(used_bin, min(p.max_cat_threshold, (used_bin + 1) / 2));
+    for (int d = 0; d < 2; ++d) {
+      const int32_t dir = d == 0 ? 1 : -1;
+      // state before position i0: the running group, and the sums so far
+      int32_t group = 0, left_count = 0;
+      double slg = 0.0, slh = kEpsilon;
+      int64_t sl_int = 0;
+      for (int32_t i0 = 0; i0 < steps; i0 += 32) {
+        const int32_t i = i0 + lane, valid = min(32, steps - i0);
+        const bool in = lane < valid;
+        const int t = in ? sm.sorted[d == 0 ? i : used_bin - 1 - i] : 0;
+        const int32_t cnt = in ? CNT(t) : 0;
+        int32_t n = cnt;
+        uint64_t q = in ? (uint64_t)Q(t) : 0ull;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int32_t on = __shfl_up_sync(0xffffffffu, n, o);
+          const uint64_t oq = kInt ? __shfl_up_sync(0xffffffffu, q, o) : 0ull;
+          if (lane >= o) {
+            n += on;
+            q += oq;
+          }
+        }
+        n += left_count;
+        q += (uint64_t)sl_int;
+        double g = slg, h = slh;
+        if constexpr (!kInt) {  // in order: lane i adds the bins up to its own
+          for (int k = 0; k < valid; ++k) {
+            const int tk = __shfl_sync(0xffffffffu, t, k);
+            const double gk = G(tk), hk = H(tk);
+            if (k <= lane) {
+              g += gk;
+              h += hk;
+            }
+          }
+        }
+        double lg, lh, rg, rh;
+        if (kInt) {
+          const int64_t rest = (int64_t)((uint64_t)lc.int_sum - q);
+          lg = (double)int_grad((int64_t)q) * gs;
+          lh = (double)int_hess((int64_t)q) * hs;
+          rg = (double)int_grad(rest) * gs;
+          rh = (double)int_hess(rest) * hs;
+        } else {
+          lg = g;
+          lh = h;
+          rg = sum_gradient - g;
+          rh = sum_hessian - h;
+        }
+        const int32_t right_count = lc.num_data - n;
+        const bool low = n < p.min_data_in_leaf || lh < p.min_sum_hessian_in_leaf;
+        const bool end = right_count < p.min_data_in_leaf || right_count < p.min_data_per_group ||
+                         rh < p.min_sum_hessian_in_leaf;
+        const unsigned lows = __ballot_sync(0xffffffffu, in && low);
+        const unsigned ends = __ballot_sync(0xffffffffu, in && !low && end);
+        const int32_t stop = ends ? __ffs(ends) - 1 : valid;
+        unsigned take = 0;
+        for (int k = 0; k < stop; ++k) {
+          group += __shfl_sync(0xffffffffu, cnt, k);
+          if ((lows >> k & 1) || group < p.min_data_per_group) continue;
+          group = 0;
+          take |= 1u << k;
+        }
+        double gain = -INFINITY;
+        if (take >> lane & 1)
+          gain = split_gain(lg, lh, rg, rh, pc, n, right_count, lc.parent_output, lc.mc, lc.cmin, lc.cmax, 0);
+        const bool good = (take >> lane & 1) && !(gain <= min_gain_shift);
+        if (__any_sync(0xffffffffu, good)) {
+          is_splittable = true;
+          double bg = good ? gain : -INFINITY;
+          int32_t bi = good && gain > -INFINITY ? lane : INT32_MAX;  // the first of equal gains
+          warp_best(bg, bi);
+          if (bi != INT32_MAX && bg > best_gain) {
+            best_gain = bg;
+            best_threshold = i0 + bi;
+            best_dir = dir;
+            best_left_count = __shfl_sync(0xffffffffu, n, bi);
+            best_slg = __shfl_sync(0xffffffffu, g, bi);
+            best_slh = __shfl_sync(0xffffffffu, h, bi);
+            best_left_int = (int64_t)__shfl_sync(0xffffffffu, q, bi);
+          }
+        }
+        if (ends) break;
+        left_count = __shfl_sync(0xffffffffu, n, 31);
+        sl_int = (int64_t)__shfl_sync(0xffffffffu, q, 31);
+        slg = __shfl_sync(0xffffffffu, g, 31);
+        slh = __shfl_sync(0xffffffffu, h, 31);
+      }
+    }
+  }
   if (lane == 0) {
     out.default_left = 0;
-    double gain_shift = use_smoothing(p) ? leaf_gain_given_output(sum_gradient, sum_hessian, p, lc.parent_output)
-                                         : leaf_gain(sum_gradient, sum_hessian, p, lc.num_data, 0.0);
-    double min_gain_shift = gain_shift + p.min_gain_to_split;
-    DParams pc = p;
-    double best_gain = -INFINITY;
-    int32_t best_left_count = 0, best_threshold = -1, best_dir = 1;
-    double best_slg = 0.0, best_slh = 0.0;
-    int64_t best_left_int = 0;
     if (use_onehot) {
       for (int t = bin_start; t < bin_end; ++t) {
         int32_t cnt = CNT(t);
@@ -1247,73 +1343,6 @@ __device__ __noinline__ bool scan_categorical(Scratch& sm, const DFeature& m, co
           best_left_count = cnt;
           best_left_int = Q(t);
           best_gain = gain;
-        }
-      }
-    } else {
-      pc.lambda_l2 += p.cat_l2;
-      int32_t max_num_cat = min(p.max_cat_threshold, (used_bin + 1) / 2);
-      for (int d = 0; d < 2; ++d) {
-        int32_t dir = d == 0 ? 1 : -1;
-        int32_t start_pos = d == 0 ? 0 : used_bin - 1;
-        int32_t cnt_cur_group = 0, left_count = 0;
-        double slg = 0.0, slh = kEpsilon;
-        int64_t sl_int = 0;
-        for (int32_t i = 0; i < used_bin && i < max_num_cat; ++i) {
-          int t = sm.sorted[start_pos];
-          start_pos += dir;
-          int32_t cnt = CNT(t);
-          double srh, srg, slh_eff;
-          if (kInt) {
-            sl_int = (int64_t)((uint64_t)sl_int + (uint64_t)Q(t));
-            left_count += cnt;
-            cnt_cur_group += cnt;
-            slh_eff = (double)int_hess(sl_int) * hs;
-            if (left_count < p.min_data_in_leaf || slh_eff < p.min_sum_hessian_in_leaf) continue;
-            int32_t right_count = lc.num_data - left_count;
-            if (right_count < p.min_data_in_leaf || right_count < p.min_data_per_group) break;
-            int64_t sr_int = (int64_t)((uint64_t)lc.int_sum - (uint64_t)sl_int);
-            srh = (double)int_hess(sr_int) * hs;
-            if (srh < p.min_sum_hessian_in_leaf) break;
-            if (cnt_cur_group < p.min_data_per_group) continue;
-            cnt_cur_group = 0;
-            double slg_i = (double)int_grad(sl_int) * gs;
-            srg = (double)int_grad(sr_int) * gs;
-            double gain = split_gain(slg_i, slh_eff, srg, srh, pc, left_count, right_count, lc.parent_output, lc.mc,
-                                     lc.cmin, lc.cmax, 0);
-            if (gain <= min_gain_shift) continue;
-            is_splittable = true;
-            if (gain > best_gain) {
-              best_left_int = sl_int;
-              best_threshold = i;
-              best_gain = gain;
-              best_dir = dir;
-            }
-          } else {
-            slg += G(t);
-            slh += H(t);
-            left_count += cnt;
-            cnt_cur_group += cnt;
-            if (left_count < p.min_data_in_leaf || slh < p.min_sum_hessian_in_leaf) continue;
-            int32_t right_count = lc.num_data - left_count;
-            if (right_count < p.min_data_in_leaf || right_count < p.min_data_per_group) break;
-            srh = sum_hessian - slh;
-            if (srh < p.min_sum_hessian_in_leaf) break;
-            if (cnt_cur_group < p.min_data_per_group) continue;
-            cnt_cur_group = 0;
-            srg = sum_gradient - slg;
-            double gain = split_gain(slg, slh, srg, srh, pc, left_count, right_count, lc.parent_output, lc.mc, lc.cmin,
-                                     lc.cmax, 0);
-            if (gain <= min_gain_shift) continue;
-            is_splittable = true;
-            if (gain > best_gain) {
-              best_left_count = left_count;
-              best_slg = slg;
-              best_slh = slh;
-              best_threshold = i;
-              best_gain = gain;
-              best_dir = dir;
-            }
-          }
         }
       }
     }
@@ -1643,7 +1672,8 @@ __device__ bool scan_direction_block(ScanSmem& sm, const DFeature& m, const DPar
 // find_best_threshold (split.rs:246-271, :930-950) for one leaf and feature,
 // by the whole CTA; the view is in `sm` (g/h, or ig for the quantized form).
 template <bool kInt>
-__device__ bool find_best_threshold_block(ScanSmem& sm, const DFeature& m, const DParams& p, LeafCtx lc, DSplit& out) {
+__device__ bool find_best_threshold_block(ScanSmem& sm, const DFeature& m, const DParams& p, const DParams& p_cat,
+                                          LeafCtx lc, DSplit& out) {
   const int tid = threadIdx.x;
   if (tid == 0) {
     out.default_left = 1;
@@ -1656,7 +1686,7 @@ __device__ bool find_best_threshold_block(ScanSmem& sm, const DFeature& m, const
   if (m.bin_type == 1) {
     __syncthreads();
     if (tid < 32) {
-      bool r = scan_categorical<kInt>(sm, m, p, lc, out);
+      bool r = scan_categorical<kInt>(sm, m, p, p_cat, lc, out);
       if (tid == 0) sm.ok = r ? 1 : 0;
     }
     __syncthreads();
@@ -1962,7 +1992,7 @@ __device__ __forceinline__ bool scan_block(const DCtx& c, const DSlot& s, int f,
     const LeafCtx lc = leaf_ctx(c, j);
     // the result is built in shared memory and stored once
     DSplit& out = sm.out;
-    const bool ok = find_best_threshold_block<kInt>(sm, m, p, lc, out);
+    const bool ok = find_best_threshold_block<kInt>(sm, m, p, c.p_cat, lc, out);
     if (tid == 0) {
       out.feature = m.real_index;
       out.inner = f;

@@ -409,10 +409,10 @@ __device__ int32_t replay(const DRounds& r, const NodeFacts& nd, int32_t* ln, in
 //   - A candidate ranked past as many known nodes as there are splits to come
 //     can never be split. It is dropped and its histogram buffer is free again.
 //   - Expanded next are the node the replay waits for and the best-ranked
-//     candidates, at most a quarter of the splits still to come, at least
-//     kRoundMin: fewer take more rounds, more expand what is not needed (on
-//     late trees of a run, whose gains hardly fall with depth, 3 to 7 times
-//     the splits; 1.6 times on early ones). Nodes of many rows are expanded
+//     candidates, at most a share of the splits still to come (DRounds): fewer
+//     take more rounds, more expand what is not needed (at a quarter 1.6 times
+//     the splits on early trees, 2 to 3 times on late ones, whose gains hardly
+//     fall with depth). Nodes of many rows are expanded
 //     ahead of need only up to kRoundRows rows a round, whose partition and
 //     histogram take as long as a few rounds.
 //   - A split needs one buffer and one expansion, and as many as there are
@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
     }
     if (!done) {
       const int32_t open = need - popped, spare = min(st.nfree, r.ecap - E);
-      const int32_t most = max(1, min(min(r.bmax, spare - open + 1), max(kRoundMin, (open + 3) / 4)));
+      const int32_t most = max(1, min(min(r.bmax, spare - open + 1), max(r.least, (open + r.share - 1) / r.share)));
       // 0: the node cannot be split; positive for every positive gain
       auto key_of = [&](int32_t v) {
         float k = nd.gain[v] > 0.0 ? fmaxf((float)nd.gain[v], 1.4e-45f) : 0.0f;

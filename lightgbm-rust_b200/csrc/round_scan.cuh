@@ -340,7 +340,8 @@ __device__ __forceinline__ bool scan_direction_packed(const int64_t* view, const
 // find_best_threshold (split.rs:246-271, :930-950) of the quantized form for
 // one leaf and feature, by one warp.
 __device__ __forceinline__ bool find_best_threshold_packed(const int64_t* view, CatScratch* cat, const DFeature& m,
-                                                           const DParams& p, const LeafCtx& lc, DSplit& out) {
+                                                           const DParams& p, const DParams& p_cat, const LeafCtx& lc,
+                                                           DSplit& out) {
   const int lane = threadIdx.x & 31;
   if (lane == 0) {
     out.default_left = 1;
@@ -353,7 +354,7 @@ __device__ __forceinline__ bool find_best_threshold_packed(const int64_t* view, 
   if (m.bin_type == 1) {
     for (int t = lane; t < m.view_len; t += 32) cat->ig[t] = view[view_at(t)];
     __syncwarp();
-    ok = scan_categorical<true>(*cat, m, p, lc, out);
+    ok = scan_categorical<true>(*cat, m, p, p_cat, lc, out);
   } else {
     const double sg = (double)int_grad(lc.int_sum) * lc.gs;
     const double sh = (double)int_hess(lc.int_sum) * lc.hs;
@@ -446,7 +447,7 @@ __global__ void __launch_bounds__(kScanThreads, kScanIntBlocks) k_round_scan_int
         view[view_at(t)] = (int64_t)v[k];
       }
       __syncwarp();
-      ok = find_best_threshold_packed(view, cat, m, c.p, leaf_ctx(c, j), out);
+      ok = find_best_threshold_packed(view, cat, m, c.p, c.p_cat, leaf_ctx(c, j), out);
       if (lane == 0) {
         out.feature = m.real_index;
         out.inner = f;
@@ -722,8 +723,8 @@ __device__ __forceinline__ bool scan_direction_f64(const double* cg, const doubl
 
 // find_best_threshold (split.rs:246-271, :402-441) for one leaf and feature,
 // by one warp; the view is in sm.view.
-__device__ __forceinline__ bool find_best_threshold_f64(F64Scratch& sm, const DFeature& m, const DParams& p, LeafCtx lc,
-                                                        DSplit& out) {
+__device__ __forceinline__ bool find_best_threshold_f64(F64Scratch& sm, const DFeature& m, const DParams& p,
+                                                        const DParams& p_cat, LeafCtx lc, DSplit& out) {
   const int lane = threadIdx.x & 31;
   if (lane == 0) {
     out.default_left = 1;
@@ -741,7 +742,7 @@ __device__ __forceinline__ bool find_best_threshold_f64(F64Scratch& sm, const DF
       cat.h[t] = sm.view[1][view_at(t)];
     }
     __syncwarp();
-    ok = scan_categorical<false>(cat, m, p, lc, out);
+    ok = scan_categorical<false>(cat, m, p, p_cat, lc, out);
   } else {
     const double min_gain_shift =
         leaf_gain_hot(plain_split(p, lc.mc), lc.sum_g, lc.sum_h, p, lc.num_data, lc.parent_output) +
@@ -834,7 +835,7 @@ __global__ void __launch_bounds__(kF64ScanThreads, kScanF64Blocks) k_round_scan_
         sm.view[1][view_at(t)] = v[k].y;
       }
       __syncwarp();
-      ok = find_best_threshold_f64(sm, m, c.p, leaf_ctx(c, j), out);
+      ok = find_best_threshold_f64(sm, m, c.p, c.p_cat, leaf_ctx(c, j), out);
       if (lane == 0) {
         out.feature = m.real_index;
         out.inner = f;
