@@ -43,7 +43,7 @@ static Status launch_gradients(const LgbmB200ObjectiveConfig& o, const float* la
   switch (o.objective) {
     case LGBM_B200_OBJ_LAMBDARANK:
       if (!rank) return Status(LGBM_B200_ERR_INVALID_PARAMETER, "lambdarank needs query boundaries");
-      return launch_lambdarank(*rank, label, score, g, h, gh, sms, s);
+      return launch_lambdarank(*rank, label, score, g, h, gh, s);
     case LGBM_B200_OBJ_BINARY: k_grad_binary<<<blocks, 256, 0, s>>>(label, score, n, o.sigmoid, gh, g, h); break;
     case LGBM_B200_OBJ_REGRESSION: k_grad_l2<<<blocks, 256, 0, s>>>(label, score, n, gh, g, h); break;
     case LGBM_B200_OBJ_MULTICLASS:

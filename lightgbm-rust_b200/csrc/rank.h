@@ -17,7 +17,8 @@ struct DRank {
   const double* label_gain;    // [31]
   const double* discount;      // [kRankMaxQuery]
   uint32_t* sorted;            // [n] per query: positions in descending score order
-  double* sorted_score;        // [n] the query's scores in that order
+  double* sorted_score;        // [n] the query's scores in that order (queries too large for shared memory)
+  double* sorted_gain;         // [n] and its label gains
   float* sorted_label;         // [n] the query's labels in that order
   double sigmoid, min_in, max_in, idx_factor;
   int32_t truncation_level;
@@ -34,7 +35,7 @@ struct RankTables {
 };
 
 Status launch_lambdarank(const DRank& r, const float* label, const double* score, float* g, float* h, float2* gh,
-                         int sms, cudaStream_t s);
+                         cudaStream_t s);
 // NDCG@ks[j] of every query into out[q * nk + j] (device buffers).
 Status launch_ndcg(const DRank& r, const float* label, const double* score, const int32_t* ks, int32_t nk,
                    double* out, int sms, cudaStream_t s);

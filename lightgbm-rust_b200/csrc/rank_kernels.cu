@@ -1,23 +1,23 @@
 // LambdarankNDCG gradients (crates/lgbm-core/src/objective/rank.rs:119-262,
-// RankingBase::gradients :63-111) on the device.
-//
-// Two launches per call:
-//   k_rank_sort    one CTA per query (grid-stride): the stable descending
-//                  order of the query's scores (dcg.rs:167-179) by rank
-//                  counting in shared memory, with the scores and labels
-//                  written out in that order
-//   k_lambdarank   one warp per query. The reference's pair loop (outer
-//                  position i below the truncation level, inner j > i) adds
-//                  to the row at position p first the pairs (i, p) for
-//                  i < p in order of i, then, when p itself is an outer
-//                  position, the pairs (p, j) in order of j. Lane l takes
-//                  the positions l, l + 32, ... and adds exactly those pairs
-//                  in that order in registers, so every f32 lambda and
-//                  hessian is formed as on the CPU. The FP64 sum of the
-//                  lambdas (for the normalisation) is one sequential chain
-//                  in the loop's order: the lanes compute 32 consecutive
-//                  pair values at a time and lane 0 subtracts them in order
-//                  (a skipped pair adds +0.0, which changes no sum).
+// RankingBase::gradients :63-111) on the device, in one launch:
+//   k_lambdarank   one CTA of 4 warps per query.
+//     order   the stable descending order of the query's scores
+//             (dcg.rs:167-179) by rank counting; the sorted scores, gains
+//             and labels stay in shared memory (queries above kRankRows
+//             rows: in global memory)
+//     pairs   the reference's pair loop (outer position i below the
+//             truncation level, inner j > i) as one sequence, in tiles of
+//             kRankTile pairs: each pair's lambda and hessian are evaluated
+//             once, by any thread, into shared memory
+//     sums    the row at position p adds first the pairs (i, p), i < p, in
+//             order of i, then, when p itself is an outer position, the
+//             pairs (p, j) in order of j, one thread per row, so every f32
+//             lambda and hessian is formed as on the CPU. The FP64 sum of
+//             the lambdas (for the normalisation) is one sequential chain in
+//             the sequence's order; it runs in one thread beside the rows'
+//             sums (a pair that is skipped would add 0.0, which changes no
+//             sum, and is left out of the chain).
+// k_ndcg's order comes from k_rank_sort, the same rank counting on its own.
 // The tables the reference builds in its constructor (label gains,
 // discounts, inverse max DCG per query, the 2^20-entry sigmoid table) are
 // built on the host by the same arithmetic and uploaded once.
@@ -26,81 +26,93 @@
 namespace lgbm_b200 {
 
 constexpr double kMinScoreD = -INFINITY;  // consts.rs kMinScore
-constexpr int kRankSortThreads = 128;
-constexpr int kRankSmemScores = 2048;  // queries up to this size sort from shared memory
+constexpr int kRankThreads = 128;
+constexpr int kRankTile = 1024;  // pairs evaluated between two barriers
+constexpr int kRankRows = 256;   // rows of a query whose sorted order stays in shared memory
+constexpr int kRankHold = 4;     // rows ranked at once by a thread of a larger query
 
-// Strict total order of the sort: larger score first, equal scores by
-// position (a stable sort); a NaN score orders after every number.
-__device__ __forceinline__ bool precedes(double sj, int j, double si, int i) {
-  const bool nj = isnan(sj), ni = isnan(si);
-  if (nj != ni) return ni;  // the number precedes the NaN
-  if (!nj && sj != si) return sj > si;
-  return j < i;
+// Monotone map of a score onto uint64: larger score, larger key; -0 and +0
+// are equal, and a NaN orders after every number.
+__device__ __forceinline__ uint64_t rank_key(double s) {
+  if (isnan(s)) return 0;
+  const uint64_t b = (uint64_t)__double_as_longlong(s == 0.0 ? 0.0 : s);
+  return (b & 0x8000000000000000ull) ? ~b : (b | 0x8000000000000000ull);
 }
 
-__global__ void __launch_bounds__(kRankSortThreads) k_rank_sort(DRank r, const double* score, const float* label) {
-  __shared__ double s[kRankSmemScores];
+// Position i's place in the stable descending order of key[0, cnt). (No key
+// is the largest uint64, so the key after it is one too.)
+__device__ __forceinline__ int32_t rank_of(const uint64_t* key, int32_t cnt, int32_t i) {
+  const uint64_t ki = key[i];
+  int32_t rank = 0;
+#pragma unroll 4
+  for (int32_t j = 0; j < cnt; ++j) rank += key[j] >= (j < i ? ki : ki + 1) ? 1 : 0;
+  return rank;
+}
+
+// The same for every row of a query too large for shared memory: a thread
+// keeps the places of kRankHold of its rows while the keys pass through
+// `key` (kRankTile of them at a time); place(i, rank) takes each result.
+// All threads of the CTA call it.
+template <class F>
+__device__ __forceinline__ void rank_large(const double* score, int32_t cnt, uint64_t* key, F place) {
+  for (int32_t i0 = 0; i0 < cnt; i0 += kRankHold * blockDim.x) {
+    uint64_t mine[kRankHold];
+    int32_t rank[kRankHold], row[kRankHold];
+#pragma unroll
+    for (int k = 0; k < kRankHold; ++k) {
+      row[k] = i0 + k * (int32_t)blockDim.x + (int32_t)threadIdx.x;
+      mine[k] = row[k] < cnt ? rank_key(score[row[k]]) : 0;
+      rank[k] = 0;
+    }
+    for (int32_t j0 = 0; j0 < cnt; j0 += kRankTile) {
+      const int32_t here = min(kRankTile, cnt - j0);
+      __syncthreads();
+      for (int32_t j = threadIdx.x; j < here; j += blockDim.x) key[j] = rank_key(score[j0 + j]);
+      __syncthreads();
+      for (int32_t j = 0; j < here; ++j) {
+        const uint64_t kj = key[j];
+#pragma unroll
+        for (int k = 0; k < kRankHold; ++k) rank[k] += kj >= (j0 + j < row[k] ? mine[k] : mine[k] + 1) ? 1 : 0;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kRankHold; ++k)
+      if (row[k] < cnt) place(row[k], rank[k]);
+  }
+}
+
+__global__ void __launch_bounds__(kRankThreads) k_rank_sort(DRank r, const double* score) {
+  __shared__ uint64_t key[kRankTile];
   for (int32_t q = blockIdx.x; q < r.nq; q += gridDim.x) {
     const int32_t b0 = r.bnd[q], cnt = r.bnd[q + 1] - b0;
-    const double* sc = score + b0;
-    const bool in_smem = cnt <= kRankSmemScores;
-    __syncthreads();
-    if (in_smem)
-      for (int i = threadIdx.x; i < cnt; i += blockDim.x) s[i] = sc[i];
-    __syncthreads();
-    const double* src = in_smem ? s : sc;
-    for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
-      const double si = src[i];
-      int32_t rank = 0;
-      for (int j = 0; j < cnt; ++j) rank += precedes(src[j], j, si, i) ? 1 : 0;
-      r.sorted[b0 + rank] = (uint32_t)i;
-      r.sorted_score[b0 + rank] = si;
-      r.sorted_label[b0 + rank] = label[b0 + i];
-    }
+    rank_large(score + b0, cnt, key, [&](int32_t i, int32_t at) { r.sorted[b0 + at] = (uint32_t)i; });
   }
 }
 
 __device__ __forceinline__ double rank_sigmoid(const DRank& r, double score) {  // rank.rs:178-186
-  if (score <= r.min_in) return r.sigmoid_table[0];
+  if (!(score > r.min_in)) return r.sigmoid_table[0];  // a NaN too, as its cast to an index
   if (score >= r.max_in) return r.sigmoid_table[kRankSigmoidBins - 1];
   return r.sigmoid_table[(size_t)((score - r.min_in) * r.idx_factor)];
 }
 
-// One query's sorted scores and labels and the values its pairs share.
+// One query's rows in sorted order and the values its pairs share.
 struct QueryView {
-  const double* ssc;
-  const float* slb;
+  const double* score;
+  const double* gain;  // of the label
+  const float* label;
   double inverse_max_dcg;
   bool scale_by_score;  // norm and best_score != worst_score (rank.rs:231-233)
 };
 
-__device__ __forceinline__ QueryView query_view(const DRank& r, int32_t q, int32_t b0, int32_t cnt) {
-  QueryView v;
-  v.ssc = r.sorted_score + b0;
-  v.slb = r.sorted_label + b0;
-  v.inverse_max_dcg = r.inv_max_dcg[q];
-  const double best_score = v.ssc[0];
-  int32_t worst_idx = cnt - 1;
-  if (worst_idx > 0 && v.ssc[worst_idx] == kMinScoreD) worst_idx -= 1;
-  v.scale_by_score = r.norm && best_score != v.ssc[worst_idx];
-  return v;
-}
-
-// The pair of sorted positions a < b (labels la != lb, neither score the
+// The pair of sorted positions a < b (labels differ, neither score the
 // minimum): its lambda and hessian by the reference's FP64 operations
-// (rank.rs:217-252), and whether a is the higher-labelled of the two. Both
-// rows of a pair evaluate the same operations, so they get the same values.
-__device__ __forceinline__ void pair_value(const DRank& r, const QueryView& v, int32_t a, int32_t b, float la,
-                                           float lb, double& p_lambda, double& p_hessian, bool& a_high) {
-  a_high = la > lb;
+// (rank.rs:217-252); a_high: a is the higher-labelled of the two.
+__device__ __forceinline__ void pair_value(const DRank& r, const QueryView& v, int32_t a, int32_t b, bool a_high,
+                                           double& p_lambda, double& p_hessian) {
   const int32_t high_rank = a_high ? a : b, low_rank = a_high ? b : a;
-  const double high_score = v.ssc[high_rank], low_score = v.ssc[low_rank];
-  const double high_label_gain = r.label_gain[(int32_t)(a_high ? la : lb)];
-  const double low_label_gain = r.label_gain[(int32_t)(a_high ? lb : la)];
-  const double high_discount = r.discount[high_rank], low_discount = r.discount[low_rank];
-  const double delta_score = high_score - low_score;
-  const double dcg_gap = high_label_gain - low_label_gain;
-  const double paired_discount = fabs(high_discount - low_discount);
+  const double delta_score = v.score[high_rank] - v.score[low_rank];
+  const double dcg_gap = v.gain[high_rank] - v.gain[low_rank];
+  const double paired_discount = fabs(r.discount[high_rank] - r.discount[low_rank]);
   double delta_pair_ndcg = dcg_gap * paired_discount * v.inverse_max_dcg;
   if (v.scale_by_score) delta_pair_ndcg /= (double)0.01f + fabs(delta_score);
   double pl = rank_sigmoid(r, delta_score);
@@ -111,99 +123,173 @@ __device__ __forceinline__ void pair_value(const DRank& r, const QueryView& v, i
   p_hessian = ph;
 }
 
-constexpr int kRankWarps = 8;  // queries per CTA (one warp each)
-
-// LambdarankNDCG::one_query (rank.rs:192-262) for every query, one warp
-// each. Writes g/h (class-major float arrays) and/or the interleaved pairs.
-__global__ void __launch_bounds__(kRankWarps * 32) k_lambdarank(DRank r, float* g, float* h, float2* gh) {
-  __shared__ __align__(16) double chain[kRankWarps][32];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int32_t T = r.truncation_level;
-  for (int64_t q = (int64_t)blockIdx.x * kRankWarps + wib; q < r.nq; q += (int64_t)gridDim.x * kRankWarps) {
+// LambdarankNDCG::one_query (rank.rs:192-262), a CTA per query. Writes g/h
+// (class-major float arrays) or the interleaved pairs.
+//
+// What bounds it: issue slots (2.2 instructions a cycle) and the barriers
+// between the parts, since a pair costs an FP64 divide, index arithmetic and
+// a load from the 8 MB sigmoid table, and one thread has the FP64 chain. A
+// pair is evaluated once (each of its two rows and the chain read it from
+// shared memory; a warp per query that evaluated it in all three places had
+// no barriers and three times the work), and the whole CTA is on one query's
+// pairs, so the largest query does not run on alone. Order and gradients,
+// two launches -> this one, on B200 with 5 labels and truncation 30: 800k
+// rows in queries of 40 rows (geometric) 1130 -> 455 us; of 400 rows 13.2
+// -> 3.8 ms; 20k rows of 40 670 -> 160 us; one query of 10000 rows 81 -> 17
+// ms. CTAs of 64, 96 and 256 threads take 1.25, 1.07 and 1.2 times as long
+// at 40 rows a query (256 would win above 400).
+__global__ void __launch_bounds__(kRankThreads, 9) k_lambdarank(DRank r, const double* score, const float* label,
+                                                             float* g, float* h, float2* gh) {
+  __shared__ __align__(16) double t_chain[kRankTile];  // 2 * lambda of the pairs that count, in order, by 32 slots
+  __shared__ float t_lambda[kRankTile];  // what the pair adds to its outer row (its inner row takes the negative)
+  __shared__ float t_hess[kRankTile];
+  __shared__ double s_score[kRankRows], s_gain[kRankRows];
+  __shared__ float s_label[kRankRows];
+  __shared__ uint16_t s_row[kRankRows];
+  __shared__ int32_t t_count[kRankTile / 32];
+  __shared__ double s_sum;
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (int64_t q = blockIdx.x; q < r.nq; q += gridDim.x) {
     const int32_t b0 = r.bnd[q], cnt = r.bnd[q + 1] - b0;
-    if (cnt == 0) continue;
-    const QueryView v = query_view(r, (int32_t)q, b0, cnt);
-    // every row's lambda and hessian, the pairs added in the reference's order
-    for (int32_t p = lane; p < cnt; p += 32) {
-      float acc_l = 0.0f, acc_h = 0.0f;
-      const double sp = v.ssc[p];
-      const float lp = v.slb[p];
-      if (sp != kMinScoreD) {
-        // as the inner position: the outer positions i < p (all i + 1 < cnt)
-        const int32_t imax = min(p, T);
-        for (int32_t i = 0; i < imax; ++i) {
-          if (v.ssc[i] == kMinScoreD) continue;
-          const float li = v.slb[i];
-          if (li == lp) continue;
-          double pl, ph;
-          bool i_high;
-          pair_value(r, v, i, p, li, lp, pl, ph, i_high);
-          acc_l += i_high ? -(float)pl : (float)pl;  // the lower-labelled row takes -lambda
-          acc_h += (float)ph;
+    if (cnt == 0) continue;  // uniform over the CTA
+    const bool small = cnt <= kRankRows;
+    QueryView v;
+    v.score = small ? s_score : r.sorted_score + b0;
+    v.gain = small ? s_gain : r.sorted_gain + b0;
+    v.label = small ? s_label : r.sorted_label + b0;
+    v.inverse_max_dcg = r.inv_max_dcg[q];
+    __syncthreads();  // the query before is done with shared memory
+    if (small) {
+      uint64_t* key = reinterpret_cast<uint64_t*>(t_chain);
+      for (int32_t i = tid; i < cnt; i += kRankThreads) key[i] = rank_key(score[b0 + i]);
+      __syncthreads();
+      for (int32_t i = tid; i < cnt; i += kRankThreads) {
+        const int32_t at = rank_of(key, cnt, i);
+        const float l = label[b0 + i];
+        s_score[at] = score[b0 + i];
+        s_gain[at] = r.label_gain[(int32_t)l];
+        s_label[at] = l;
+        s_row[at] = (uint16_t)i;
+      }
+    } else {
+      rank_large(score + b0, cnt, reinterpret_cast<uint64_t*>(t_chain), [&](int32_t i, int32_t rank) {
+        const int32_t at = b0 + rank;
+        const float l = label[b0 + i];
+        r.sorted_score[at] = score[b0 + i];
+        r.sorted_gain[at] = r.label_gain[(int32_t)l];
+        r.sorted_label[at] = l;
+        r.sorted[at] = (uint32_t)i;
+      });
+    }
+    __syncthreads();
+    int32_t worst_idx = cnt - 1;
+    if (worst_idx > 0 && v.score[worst_idx] == kMinScoreD) worst_idx -= 1;
+    v.scale_by_score = r.norm && v.score[0] != v.score[worst_idx];
+    // the sequence of pairs: rows i = 0 .. outer - 1, row i the pairs (i, i + 1 .. cnt - 1), from `start(i)` on
+    const int32_t outer = max(0, min(r.truncation_level, cnt - 1));
+    const int32_t pairs = outer * (cnt - 1) - (int32_t)((int64_t)outer * (outer - 1) / 2);
+    auto start = [&](int32_t i) { return i * (cnt - 1) - (int32_t)((int64_t)i * (i - 1) / 2); };
+    double sum_lambdas = 0.0;  // thread 0's chain
+    int32_t i = 0, j = 1 + tid;                   // this thread's next pair
+    int32_t first = 0;                            // the row that holds the tile's first pair
+    for (int32_t base = 0; base == 0 || base < pairs; base += kRankTile) {
+      const int32_t here = min(kRankTile, pairs - base);  // 0 for a query of one row
+      for (int32_t t = tid; t < kRankTile; t += kRankThreads) {
+        while (i < outer && j >= cnt) {
+          ++i;
+          j = j - cnt + i + 1;
         }
-        // as the outer position
-        if (p < T && p + 1 < cnt) {
-          for (int32_t j = p + 1; j < cnt; ++j) {
-            if (v.ssc[j] == kMinScoreD) continue;
-            const float lj = v.slb[j];
-            if (lj == lp) continue;
-            double pl, ph;
-            bool p_high;
-            pair_value(r, v, p, j, lp, lj, pl, ph, p_high);
-            acc_l += p_high ? (float)pl : -(float)pl;
-            acc_h += (float)ph;
+        double pl = 0.0, ph = 0.0;
+        bool counts = false, i_high = false;
+        if (i < outer) {
+          const float li = v.label[i], lj = v.label[j];
+          i_high = li > lj;
+          counts = li != lj && v.score[i] != kMinScoreD && v.score[j] != kMinScoreD;
+          if (counts) pair_value(r, v, i, j, i_high, pl, ph);
+        }
+        t_lambda[t] = i_high ? (float)pl : -(float)pl;
+        t_hess[t] = (float)ph;
+        const uint32_t m = __ballot_sync(0xffffffffu, counts);
+        const int32_t n = max(__popc(m), 1);  // one zero where no pair counts
+        if (counts) t_chain[(t & ~31) + __popc(m & ((1u << lane) - 1))] = 2.0 * pl;
+        if (lane >= __popc(m) && lane < ((n + 3) & ~3)) t_chain[(t & ~31) + lane] = 0.0;
+        if (lane == 0) t_count[t >> 5] = n;
+        j += kRankThreads;
+        if (base + t - tid + kRankThreads >= pairs) break;  // uniform: no pair is left
+      }
+      __syncthreads();
+      const int32_t last = base + here;  // pairs of the tile: [base, last)
+      while (first + 1 < outer && start(first + 1) <= base) ++first;
+      if (tid == 0 && r.norm) {
+        double2 x = *reinterpret_cast<const double2*>(&t_chain[0]), y = *reinterpret_cast<const double2*>(&t_chain[2]);
+        int32_t n = here > 0 ? t_count[0] : 0;
+        for (int32_t w = 0; w * 32 < here; ++w) {
+          const int32_t after = (w + 1) * 32 < here ? t_count[w + 1] : 0;
+          for (int32_t k = 0; k < n; k += 4) {
+            // the next four: of this group, or the first of the group after it
+            const int32_t at = min(w * 32 + (k + 4 < n ? k + 4 : 32), kRankTile - 4);
+            const double2 nx = *reinterpret_cast<const double2*>(&t_chain[at]);
+            const double2 ny = *reinterpret_cast<const double2*>(&t_chain[at + 2]);
+            sum_lambdas -= x.x;
+            sum_lambdas -= x.y;
+            sum_lambdas -= y.x;
+            sum_lambdas -= y.y;
+            x = nx;
+            y = ny;
+          }
+          n = after;
+        }
+      }
+      // the rows' sums; warp 0 keeps to the chain when there is one
+      const int32_t skip = r.norm ? 32 : 0;
+      for (int32_t p = (base == 0 ? 0 : first) + tid - skip; tid >= skip && p < cnt; p += kRankThreads - skip) {
+        // as the inner position of rows first ..: pair (i, p) is slot start(i) + p - i - 1
+        const int32_t inner = min(p, outer);
+        int32_t o = first, slot = start(first) + p - first - 1 - base;
+        if (slot < 0 && o < inner) slot += cnt - 2 - o++;  // row `first` began in the tile before
+        const int32_t from = max(base, start(p)), to = min(last, start(p) + cnt - 1 - p);
+        if (base > 0 && !(o < inner && slot < here) && !(p < outer && from < to)) continue;  // none of its pairs
+        const uint32_t row = b0 + (small ? (uint32_t)s_row[p] : r.sorted[b0 + p]);
+        float acc_l = 0.0f, acc_h = 0.0f;
+        if (base > 0) {
+          acc_l = g ? g[row] : gh[row].x;
+          acc_h = g ? h[row] : gh[row].y;
+        }
+#pragma unroll 4
+        for (; o < inner && slot < here; slot += cnt - 2 - o++) {
+          acc_l -= t_lambda[slot];
+          acc_h += t_hess[slot];
+        }
+        // as the outer position: its row's pairs inside the tile
+        if (p < outer) {
+#pragma unroll 8
+          for (int32_t t = from; t < to; ++t) {
+            acc_l += t_lambda[t - base];
+            acc_h += t_hess[t - base];
           }
         }
+        if (g) {
+          g[row] = acc_l;
+          h[row] = acc_h;
+        } else {
+          gh[row] = make_float2(acc_l, acc_h);
+        }
       }
-      const uint32_t row = r.sorted[b0 + p];
-      if (g) {
-        g[b0 + row] = acc_l;
-        h[b0 + row] = acc_h;
-      } else {
-        gh[b0 + row] = make_float2(acc_l, acc_h);
-      }
+      __syncthreads();  // the sums are written, and the tile is free
     }
     if (!r.norm) continue;
-    // sum_lambdas -= 2 p_lambda over the pairs in the loop's order (lane 0's chain)
-    double sum_lambdas = 0.0;
-    for (int32_t i = 0; i + 1 < cnt && i < T; ++i) {
-      if (v.ssc[i] == kMinScoreD) continue;  // uniform over the warp
-      const float li = v.slb[i];
-      for (int32_t jb = i + 1; jb < cnt; jb += 32) {
-        const int32_t j = jb + lane;
-        double val = 0.0;
-        if (j < cnt && v.ssc[j] != kMinScoreD && v.slb[j] != li) {
-          double pl, ph;
-          bool i_high;
-          pair_value(r, v, i, j, li, v.slb[j], pl, ph, i_high);
-          val = 2.0 * pl;
-        }
-        chain[wib][lane] = val;
-        __syncwarp();
-        if (lane == 0) {
-          // all 32 in order: the slots past the query hold +0.0, which
-          // changes no sum; unrolled, the loads go in pairs
-#pragma unroll
-          for (int32_t k = 0; k < 32; k += 2) {
-            const double2 two = *reinterpret_cast<const double2*>(&chain[wib][k]);
-            sum_lambdas -= two.x;
-            sum_lambdas -= two.y;
-          }
-        }
-        __syncwarp();
-      }
-    }
-    sum_lambdas = __shfl_sync(0xffffffffu, sum_lambdas, 0);
-    if (sum_lambdas > 0.0) {  // every lane's rows are written (the warp's stores are ordered by __syncwarp)
-      __syncwarp();
+    if (tid == 0) s_sum = sum_lambdas;
+    __syncthreads();
+    sum_lambdas = s_sum;
+    if (sum_lambdas > 0.0) {
       const double norm_factor = log2(1.0 + sum_lambdas) / sum_lambdas;
-      for (int32_t x = lane; x < cnt; x += 32) {
+      for (int32_t x = tid; x < cnt; x += kRankThreads) {
         if (g) {
           g[b0 + x] = (float)((double)g[b0 + x] * norm_factor);
           h[b0 + x] = (float)((double)h[b0 + x] * norm_factor);
         } else {
-          gh[b0 + x].x = (float)((double)gh[b0 + x].x * norm_factor);
-          gh[b0 + x].y = (float)((double)gh[b0 + x].y * norm_factor);
+          const float2 a = gh[b0 + x];
+          gh[b0 + x] = make_float2((float)((double)a.x * norm_factor), (float)((double)a.y * norm_factor));
         }
       }
     }
@@ -257,7 +343,7 @@ Status launch_ndcg(const DRank& r, const float* label, const double* score, cons
                    double* out, int sms, cudaStream_t s) {
   if (r.nq == 0) return Status();
   const int sort_grid = (int)std::min<int64_t>(r.nq, (int64_t)sms * 16);
-  k_rank_sort<<<sort_grid, kRankSortThreads, 0, s>>>(r, score, label);
+  k_rank_sort<<<sort_grid, kRankThreads, 0, s>>>(r, score);
   CU_LAUNCH();
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((r.nq + 127) / 128, (int64_t)sms * 16));
   k_ndcg<<<grid, 128, 0, s>>>(r, label, ks, nk, out);
@@ -315,12 +401,14 @@ Status RankTables::build(const float* label_h, const int32_t* bnd_h, int32_t nq_
   double *inv_d, *table_d, *gain_d, *disc_d;
   uint32_t* sorted_d;
   double* sorted_score_d;
+  double* sorted_gain_d;
   float* sorted_label_d;
   const size_t n1 = (size_t)std::max<int64_t>(1, n);
   if (!(s = arena.alloc_n(&bnd_d, (size_t)nq + 1)).ok() || !(s = arena.alloc_n(&inv_d, std::max<size_t>(1, nq))).ok() ||
       !(s = arena.alloc_n(&table_d, table.size())).ok() || !(s = arena.alloc_n(&gain_d, label_gain.size())).ok() ||
       !(s = arena.alloc_n(&disc_d, discount.size())).ok() || !(s = arena.alloc_n(&sorted_d, n1)).ok() ||
-      !(s = arena.alloc_n(&sorted_score_d, n1)).ok() || !(s = arena.alloc_n(&sorted_label_d, n1)).ok())
+      !(s = arena.alloc_n(&sorted_score_d, n1)).ok() || !(s = arena.alloc_n(&sorted_gain_d, n1)).ok() ||
+      !(s = arena.alloc_n(&sorted_label_d, n1)).ok())
     return s;
   CU(cudaMemcpy(bnd_d, bnd_h, sizeof(int32_t) * ((size_t)nq + 1), cudaMemcpyHostToDevice));
   if (nq > 0) CU(cudaMemcpy(inv_d, inv.data(), sizeof(double) * nq, cudaMemcpyHostToDevice));
@@ -335,6 +423,7 @@ Status RankTables::build(const float* label_h, const int32_t* bnd_h, int32_t nq_
   d.discount = disc_d;
   d.sorted = sorted_d;
   d.sorted_score = sorted_score_d;
+  d.sorted_gain = sorted_gain_d;
   d.sorted_label = sorted_label_d;
   d.sigmoid = sigmoid;
   d.min_in = min_in;
@@ -346,13 +435,9 @@ Status RankTables::build(const float* label_h, const int32_t* bnd_h, int32_t nq_
 }
 
 Status launch_lambdarank(const DRank& r, const float* label, const double* score, float* g, float* h, float2* gh,
-                         int sms, cudaStream_t s) {
+                         cudaStream_t s) {
   if (r.nq == 0) return Status();
-  const int sort_grid = (int)std::min<int64_t>(r.nq, (int64_t)sms * 16);
-  k_rank_sort<<<sort_grid, kRankSortThreads, 0, s>>>(r, score, label);
-  CU_LAUNCH();
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((r.nq + kRankWarps - 1) / kRankWarps, (int64_t)sms * 32));
-  k_lambdarank<<<grid, kRankWarps * 32, 0, s>>>(r, g, h, gh);
+  k_lambdarank<<<(unsigned)r.nq, kRankThreads, 0, s>>>(r, score, label, g, h, gh);
   CU_LAUNCH();
   return Status();
 }

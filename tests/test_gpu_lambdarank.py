@@ -49,3 +49,24 @@ def test_normalised_gradients_within_one_ulp(lgb, orc):
     obj = lgb.Objective(params, label, group=group)
     g2, h2 = obj.gradients(score)
     assert np.array_equal(g2, g) and np.array_equal(h2, h)
+
+
+@pytest.mark.parametrize("size", [35, 36, 45, 46, 47, 255, 256, 257, 511, 512, 513, 1024, 1025, 2500])
+@pytest.mark.parametrize("trunc", [30, 1023])
+def test_one_query_at_tile_edges(lgb, orc, size, trunc):
+    """Queries around one and two tiles of 1024 pairs, the largest ordered in
+    shared memory and the passes of larger ones: unnormalised sums bit for
+    bit, normalised ones within an ulp (the order of every sum is fixed)."""
+    rng = np.random.default_rng(size)
+    label = rng.integers(0, 5, size).astype(np.float32)
+    score = np.round(rng.standard_normal(size), 1)
+    score[rng.random(size) < 0.02] = -np.inf
+    group = np.array([3, size - 3], np.int32) if size % 2 else np.array([size], np.int32)
+    for norm in (False, True):
+        params = {"objective": "lambdarank", "lambdarank_norm": norm, "lambdarank_truncation_level": trunc}
+        g, h = lgb.gradients(params, label, score, group=group)
+        og, oh = orc.gradients(lgb.resolve_params(params), label, score, group)
+        if norm:
+            assert _ulps(g, og).max() <= 1 and _ulps(h, oh).max() <= 1
+        else:
+            assert np.array_equal(g, og) and np.array_equal(h, oh)
