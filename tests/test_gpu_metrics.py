@@ -79,3 +79,20 @@ def test_ndcg_matches_oracle(lgb, orc):
         got = lgb.ndcg(label, score, group, ks)
         want = orc.ndcg(label, score, group, ks)
         assert np.array_equal(got, want), (ks, got, want)
+
+
+@pytest.mark.parametrize("n", [1, 31, 255, 257, 1024, 1025, 24576, 24577, 26624, 26625, 262144 + 5])
+@pytest.mark.parametrize("scores", ["distinct", "few", "one", "special"])
+def test_auc_sort_at_tile_edges(lgb, orc, n, scores):
+    """The counted pairs' blocks (256) and slices (1024), the largest counted
+    and the smallest sorted, whole and broken tiles of the sort (2048), with
+    scores that stand alone, large tied groups across tiles, a single group,
+    and signed zeros, infinities and subnormals. Equal bit for bit: every sum
+    is a multiple of 1/2 below 2^52."""
+    rng = np.random.default_rng(n)
+    label = rng.integers(0, 2, n).astype(np.float32)
+    s = {"distinct": lambda: rng.permutation(n) * 1.25 - n / 2,
+         "few": lambda: rng.integers(-2, 3, n).astype(np.float64),
+         "one": lambda: np.full(n, 0.75),
+         "special": lambda: rng.choice([0.0, -0.0, np.inf, -np.inf, 5e-324, -5e-324, 1e308, -1.0], n)}[scores]()
+    assert lgb.metric("auc", label, s) == orc.auc(label, s)
