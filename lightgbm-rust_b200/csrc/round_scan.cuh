@@ -109,10 +109,15 @@ __device__ __forceinline__ void scans_stored(const DCtx& c, const DSlot& s, int 
   int last = 0;
   __syncwarp();
   if ((threadIdx.x & 31) == 0) {
-    __threadfence();
-    last = atomicAdd(&s.r.scan_cnt[q], count) + count == c.num_features;
-    __threadfence();
+    // releases this warp's results, and acquires the others' for the last
+    int32_t before;
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;"
+                 : "=r"(before)
+                 : "l"(&s.r.scan_cnt[q]), "r"(count)
+                 : "memory");
+    last = before + count == c.num_features;
   }
+  __syncwarp();
   last = __shfl_sync(0xffffffffu, last, 0);
   if (last) round_best(c, s, q, child, depth);
   __syncwarp();
@@ -468,11 +473,31 @@ __global__ void __launch_bounds__(kScanThreads, kScanIntBlocks) k_round_scan_int
 // ---- FP64: one warp per scan ------------------------------------------------------------
 
 // A warp's shared memory: the view's gradients and hessians, and the
-// cumulative sums of both directions (reverse g, h, forward g, h).
-struct F64Scratch {
-  double view[2][kViewPad];
-  double cum[4][kViewPad];
+// cumulative sums of both directions (reverse g, h, forward g, h). Values
+// move in 16-byte pairs. A pair of padding after every 16 values lets lanes
+// on consecutive groups of 8 meet different banks and leaves a chain's
+// addresses constant offsets (pairs permuted by their chunk took 15.5 cycles
+// a value, this 9.9); one more after the last lets the four lanes that walk
+// the four sums side by side meet different banks too.
+constexpr int kF64Chunk = 16;  // values of a chain's step
+constexpr int kF64Pad = kMaxBins + 2 * (kMaxBins / kF64Chunk) + 2;
+static_assert(kF64Pad % 16 == 2, "the arrays start one 16-byte bank apart");
+struct __align__(16) F64Scratch {
+  double view[2][kF64Pad];
+  double cum[4][kF64Pad];
 };
+__device__ __forceinline__ int f64_at(int t) { return t + 2 * (t >> 4); }
+// Values 8 * seg .. 8 * seg + 7.
+__device__ __forceinline__ void f64_load8(const double* x, int seg, double (&v)[kPer]) {
+  static_assert(kPer == 8 && kF64Chunk == 16, "two groups a chunk");
+  const double2* q = reinterpret_cast<const double2*>(x + f64_at(kPer * seg));
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const double2 two = q[i];
+    v[2 * i] = two.x;
+    v[2 * i + 1] = two.y;
+  }
+}
 // A categorical scan's scratch, in the place of the cumulative sums.
 struct CatScratchF64 {
   double g[kMaxBins], h[kMaxBins], key[kMaxBins];
@@ -501,29 +526,50 @@ __device__ __forceinline__ ScanSpan scan_span(const DFeature& m, bool reverse, b
   return v;
 }
 
-// A serial chain of adds (sign 1) or subtractions (-1) over `segs` chunks of
-// kPer values of x, in order, each replaced by its running value if `store`.
-// Values that take no part are zeros (a running sum here is never -0.0, so
-// adding zero changes nothing), which leaves a load, an add and a store per
-// value: with the visited tests in the loop a chain took 45 cycles a value.
-// The next chunk is loaded while this one is added.
-__device__ __noinline__ double f64_chain(double a, double* x, int segs, double sign, bool store) {
-  double v[kPer], next[kPer];
+// Chunks of kF64Chunk values that hold a view.
+__device__ __forceinline__ int f64_chunks(int len) { return (len + kF64Chunk - 1) / kF64Chunk; }
+
+// A serial chain of adds (kMinus: subtractions) over `chunks` chunks of
+// kF64Chunk values of x, in order, each replaced by its running value if
+// kStore. Values that take no part are zeros (a running sum here is never
+// -0.0, so adding zero changes nothing), which leaves an add and half a
+// 16-byte load and store per value: with the visited tests in the loop a
+// chain took 45 cycles a value. Half a chunk is loaded while the other half
+// is added. Only the lanes with a chain of their own come here: a 16-byte
+// access of 32 lanes is four wavefronts even when they name the same four
+// addresses, and the shared-memory pipe is what a full round is bound by (60%
+// of its peak with scalar accesses of arrays whose starts shared a bank). An
+// FP64 add takes 8.2 cycles to its result, a value of the chain 9.5. Scans of
+// an iteration of 1M x 100 with 255 leaves 1238 -> 710 us, the iteration 3.04
+// -> 2.44 ms.
+template <bool kMinus, bool kStore>
+__device__ __noinline__ double f64_chain(double a, double* x, int chunks) {
+  double2* q = reinterpret_cast<double2*>(x);
+  double2 lo[4], hi[4];
 #pragma unroll
-  for (int i = 0; i < kPer; ++i) v[i] = x[i];
-  for (int k = 0; k < segs; ++k, x += kPer + 1) {
-    if (k + 1 < segs) {
+  for (int i = 0; i < 4; ++i) lo[i] = q[i];
+  auto add = [&](double2& two) {
+    two.x = a = kMinus ? a - two.x : a + two.x;
+    two.y = a = kMinus ? a - two.y : a + two.y;
+  };
+  for (int k = 0; k < chunks; ++k, q += kF64Chunk / 2 + 1) {
 #pragma unroll
-      for (int i = 0; i < kPer; ++i) next[i] = x[kPer + 1 + i];
+    for (int i = 0; i < 4; ++i) hi[i] = q[4 + i];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) add(lo[i]);
+    if constexpr (kStore) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) q[i] = lo[i];
     }
+    // past the last chunk: the array, the split records or the warp after, not used
 #pragma unroll
-    for (int i = 0; i < kPer; ++i) v[i] = a = a + sign * v[i];
-    if (store) {
+    for (int i = 0; i < 4; ++i) lo[i] = q[kF64Chunk / 2 + 1 + i];
 #pragma unroll
-      for (int i = 0; i < kPer; ++i) x[i] = v[i];
+    for (int i = 0; i < 4; ++i) add(hi[i]);
+    if constexpr (kStore) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) q[4 + i] = hi[i];
     }
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) v[i] = next[i];
   }
   return a;
 }
@@ -534,35 +580,35 @@ __device__ __noinline__ double f64_chain(double a, double* x, int segs, double s
 // (two: both directions are scanned). The forward chain starts, for a feature
 // with NaN missing and no stored bin 0, from the leaf's sums minus every
 // stored bin (split.rs:787-800), which base_g / base_h return. Past its length
-// the view holds zeros. The reverse sums of bin t lie at place 8 * segs - 1 - t,
-// so that all lanes run forward.
+// the view holds zeros. The reverse sums of bin t lie at place
+// kF64Chunk * chunks - 1 - t, so that all lanes run forward.
 __device__ __forceinline__ void f64_chains(F64Scratch& sm, const LeafCtx& lc, const ScanSpan& rev, const ScanSpan& fwd,
                                            int len, bool two, bool first_extra, double& base_g, double& base_h) {
   const int lane = threadIdx.x & 31;
   const bool forward = (lane & 3) >= 2 && two, hess = lane & 1;
-  const int segs = (len + kPer - 1) / kPer, last = kPer * segs - 1;
+  const int chunks = f64_chunks(len), last = kF64Chunk * chunks - 1;
 #pragma unroll
   for (int k = 0; k < kPer; ++k) {
     const int t = 32 * k + lane;
     if (t > last) continue;
-    const double g = sm.view[0][view_at(t)], h = sm.view[1][view_at(t)];
-    sm.cum[0][view_at(last - t)] = rev.has(t) ? g : 0.0;
-    sm.cum[1][view_at(last - t)] = rev.has(t) ? h : 0.0;
+    const double g = sm.view[0][f64_at(t)], h = sm.view[1][f64_at(t)];
+    sm.cum[0][f64_at(last - t)] = rev.has(t) ? g : 0.0;
+    sm.cum[1][f64_at(last - t)] = rev.has(t) ? h : 0.0;
     if (two) {
-      sm.cum[2][view_at(t)] = fwd.has(t) ? g : 0.0;
-      sm.cum[3][view_at(t)] = fwd.has(t) ? h : 0.0;
+      sm.cum[2][f64_at(t)] = fwd.has(t) ? g : 0.0;
+      sm.cum[3][f64_at(t)] = fwd.has(t) ? h : 0.0;
     }
   }
   double a = hess ? kEpsilon : 0.0;
   if (first_extra) {
-    const double b = f64_chain(hess ? lc.sum_h - kEpsilon : lc.sum_g, sm.view[hess], segs, -1.0, false);
+    double b = 0.0;
+    if (lane < 4) b = f64_chain<true, false>(hess ? lc.sum_h - kEpsilon : lc.sum_g, sm.view[hess], chunks);
     if (forward) a = b;
     base_g = __shfl_sync(0xffffffffu, b, 2);
     base_h = __shfl_sync(0xffffffffu, b, 3);
   }
   __syncwarp();
-  // lanes past the chains repeat them without storing
-  f64_chain(a, sm.cum[(forward ? 2 : 0) + hess], segs, 1.0, lane < (two ? 4 : 2));
+  if (lane < (two ? 4 : 2)) f64_chain<false, true>(a, sm.cum[(forward ? 2 : 0) + hess], chunks);
   __syncwarp();
 }
 
@@ -583,10 +629,12 @@ __device__ __forceinline__ bool scan_direction_f64(const double* cg, const doubl
   // count estimates: each bin's rounded on its own, their sums exact in any order
   int32_t n[kPer], pre = 0, all = 0;
   uint32_t visited = 0;
+  double a[kPer], b[kPer];
+  f64_load8(view_h, lane, b);
 #pragma unroll
   for (int j = 0; j < kPer; ++j) {
     const int t = lane * kPer + j;
-    const int32_t ce = t < len ? round_int(view_h[view_at(t)] * cnt_factor) : 0;
+    const int32_t ce = t < len ? round_int(b[j] * cnt_factor) : 0;
     if (first_extra) all += ce;
     n[j] = 0;
     if (span.has(t)) {
@@ -629,15 +677,26 @@ __device__ __forceinline__ bool scan_direction_f64(const double* cg, const doubl
   auto estimate = [&](double a, double b) {
     return gain_estimate((float)a, (float)b, (float)(lc.sum_g - a), (float)(lc.sum_h - b), l2f);
   };
-  const int last = (len + kPer - 1) / kPer * kPer - 1;
-  double a[kPer], b[kPer];
+  {  // the reverse sums lie mirrored (f64_chains)
+    const int segs = f64_chunks(len) * (kF64Chunk / kPer);
+    const int seg = reverse ? max(0, segs - 1 - lane) : lane;
+    f64_load8(cg, seg, a);
+    f64_load8(ch, seg, b);
+    if (reverse) {
+#pragma unroll
+      for (int j = 0; j < kPer / 2; ++j) {
+        const double x = a[j], y = b[j];
+        a[j] = a[kPer - 1 - j];
+        b[j] = b[kPer - 1 - j];
+        a[kPer - 1 - j] = x;
+        b[kPer - 1 - j] = y;
+      }
+    }
+  }
   float est[kPer];
   uint32_t pend = 0, stop = 0;
 #pragma unroll
   for (int j = 0; j < kPer; ++j) {
-    const int t = lane * kPer + j, at = view_at(reverse ? max(0, last - t) : t);
-    a[j] = cg[at];
-    b[j] = ch[at];
     est[j] = estimate(a[j], b[j]);
     if ((visited >> j & 1) && !low(b[j], n[j])) (ends(b[j], n[j]) ? stop : pend) |= 1u << j;
   }
@@ -738,8 +797,8 @@ __device__ __forceinline__ bool find_best_threshold_f64(F64Scratch& sm, const DF
   if (m.bin_type == 1) {
     CatScratchF64& cat = *reinterpret_cast<CatScratchF64*>(sm.cum);
     for (int t = lane; t < m.view_len; t += 32) {
-      cat.g[t] = sm.view[0][view_at(t)];
-      cat.h[t] = sm.view[1][view_at(t)];
+      cat.g[t] = sm.view[0][f64_at(t)];
+      cat.h[t] = sm.view[1][f64_at(t)];
     }
     __syncwarp();
     ok = scan_categorical<false>(cat, m, p, p_cat, lc, out);
@@ -809,12 +868,13 @@ __global__ void __launch_bounds__(kF64ScanThreads, kScanF64Blocks) k_round_scan_
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
           const bool own = 32 * k + lane != m.most_freq_bin;
-          sm.view[0][view_at(32 * k + lane)] = own ? v[k].x : 0.0;
-          sm.view[1][view_at(32 * k + lane)] = own ? v[k].y : 0.0;
+          sm.view[0][f64_at(32 * k + lane)] = own ? v[k].x : 0.0;
+          sm.view[1][f64_at(32 * k + lane)] = own ? v[k].y : 0.0;
         }
         __syncwarp();
-        const double a = f64_chain((lane & 1) ? j.sl.sum_hessians : j.sl.sum_gradients, sm.view[lane & 1],
-                                   (len + kPer - 1) / kPer, -1.0, false);
+        double a = 0.0;
+        if (lane < 2)
+          a = f64_chain<true, false>(lane ? j.sl.sum_hessians : j.sl.sum_gradients, sm.view[lane], f64_chunks(len));
         const double2 fixed = make_double2(__shfl_sync(0xffffffffu, a, 0), __shfl_sync(0xffffffffu, a, 1));
 #pragma unroll
         for (int k = 0; k < kPer; ++k)
@@ -831,8 +891,8 @@ __global__ void __launch_bounds__(kF64ScanThreads, kScanF64Blocks) k_round_scan_
           v[k] = make_double2(pv[k].x - v[k].x, pv[k].y - v[k].y);
           if (t < len) hp[t] = v[k];
         }
-        sm.view[0][view_at(t)] = v[k].x;
-        sm.view[1][view_at(t)] = v[k].y;
+        sm.view[0][f64_at(t)] = v[k].x;
+        sm.view[1][f64_at(t)] = v[k].y;
       }
       __syncwarp();
       ok = find_best_threshold_f64(sm, m, c.p, c.p_cat, leaf_ctx(c, j), out);
