@@ -142,40 +142,6 @@ def hist_bytes_per_row(nf, form):
     return nf * 1 + (4 if form == "quantized" else 8) + 4
 
 
-def hist_rows_by_step(t):
-    """Rows each split step's histogram launch reads: step 0 the root (every
-    row of the tree), step s the smaller child of split s - 1 (the split
-    order is the node order)."""
-    def count(c):
-        return int(t["internal_count"][c]) if c >= 0 else int(t["leaf_count"][~c])
-
-    nl = int(t["num_leaves"])
-    if nl < 2:
-        return []
-    out = [int(np.sum(t["leaf_count"]))]
-    for k in range(nl - 2):
-        out.append(min(count(int(t["left_child"][k])), count(int(t["right_child"][k]))))
-    return out
-
-
-def hist_by_rows(step_rows, step_ms, bytes_per_row):
-    """Histogram launches binned by the rows they read: launches, mean us per
-    launch, and GB/s of algorithmic bytes (rows x bytes per row) per bin."""
-    edges = [0, 1_000, 10_000, 100_000, 1_000_000, 10**12]
-    out = []
-    r = np.asarray(step_rows, np.float64)
-    ms = np.asarray(step_ms, np.float64)
-    for lo, hi in zip(edges[:-1], edges[1:]):
-        sel = (r >= lo) & (r < hi)
-        if not np.any(sel):
-            continue
-        t = float(ms[sel].sum()) / 1000.0
-        out.append({"rows_from": lo, "rows_to": hi if hi < 10**12 else None, "launches": int(sel.sum()),
-                    "us_per_launch": 1e6 * t / int(sel.sum()),
-                    "gbs": float(r[sel].sum()) * bytes_per_row / t / 1e9 if t > 0 else None})
-    return out
-
-
 def _shape_key(args, form):
     """Key of a workload's tuned launch shape: workload, scale, histogram form."""
     return f"{args.workload}{'' if args.scale == 1.0 else '@' + format(args.scale, 'g')}/{form}"
@@ -239,8 +205,7 @@ def run_form(lgb, data, ds, dv, form, args, device):
     L.set_timing(True)
     hist_ms = scan_ms = part_ms = 0.0
     rows = prows = 0
-    launches = 0
-    step_rows, step_hist_ms = [], []
+    launches = rounds = 0
     for _ in range(args.steps):
         bst.update()
         t, r, nl = L.last_timing()
@@ -251,10 +216,7 @@ def run_form(lgb, data, ds, dv, form, args, device):
         rows += r
         prows += pr
         launches = nl
-        st = L.step_times()
-        rr = hist_rows_by_step(bst.trees[-1])
-        step_rows.extend(rr)
-        step_hist_ms.extend(st[: len(rr), 0])
+        rounds += len(L.step_times())  # a round's launches: partition, histogram, scan
     L.set_timing(False)
     done = args.warmup + extra + 2 * args.steps
     for _ in range(max(0, args.rounds - done)):
@@ -270,8 +232,6 @@ def run_form(lgb, data, ds, dv, form, args, device):
     auc_device = lgb.metric("auc", data["y_valid"], sv, device=device)
     auc_device_ms = 1000 * (time.perf_counter() - t0)
     nf = ds.binned()["num_features"]
-    steps_per_tree = int(params["num_leaves"]) - 1
-    hist_launches = args.steps * steps_per_tree
     hist_bytes = rows * hist_bytes_per_row(nf, form)
     # the partition moves each row of the split leaf: index in, its byte of the
     # split feature (column copy), index out
@@ -279,16 +239,15 @@ def run_form(lgb, data, ds, dv, form, args, device):
     return {
         "ms_per_step": ms, "wall_ms_per_step": 1000 * wall / args.steps, "s_per_500": ms * ROUNDS / 1000.0,
         "auc": auc, "auc_device": auc_device, "auc_device_ms": auc_device_ms, "auc_numpy_ms": auc_numpy_ms,
-        "hist_ms_per_launch": hist_ms / hist_launches, "hist_gbs": hist_bytes / (hist_ms / 1000) / 1e9,
-        "hist_bytes_per_launch": hist_bytes / hist_launches, "hist_rows_per_tree": rows / args.steps,
+        "hist_ms_per_launch": hist_ms / rounds, "hist_gbs": hist_bytes / (hist_ms / 1000) / 1e9,
+        "hist_bytes_per_launch": hist_bytes / rounds, "hist_rows_per_tree": rows / args.steps,
         "scan_ms_per_step": scan_ms / args.steps, "partition_ms_per_step": part_ms / args.steps,
         "part_rows_per_tree": prows / args.steps,
         "part_gbs": part_bytes / (part_ms / 1000) / 1e9 if part_ms > 0 else None,
-        "part_bytes_per_launch": part_bytes / (args.steps * steps_per_tree),
-        "part_ms_per_launch": part_ms / (args.steps * steps_per_tree),
+        "part_bytes_per_launch": part_bytes / rounds, "part_ms_per_launch": part_ms / rounds,
+        "rounds_per_iteration": rounds / args.steps,
         "hist_ms_per_step": hist_ms / args.steps, "kernel_launches_per_tree": launches, "clocks": clk,
         "num_trees": bst.num_trees(), "nf": nf, "launch_shape": shape, "launch_shape_source": shape_src,
-        "hist_by_rows": hist_by_rows(step_rows, step_hist_ms, hist_bytes_per_row(nf, form)),
     }
 
 
@@ -828,35 +787,33 @@ def main():
                       "scan_ms_per_step": v["scan_ms_per_step"], "partition_ms_per_step": v["partition_ms_per_step"],
                       "hist_rows_per_tree": v["hist_rows_per_tree"], "part_gbs": v["part_gbs"],
                       "part_rows_per_tree": v["part_rows_per_tree"], "launch_shape": v["launch_shape"],
-                      "launch_shape_source": v["launch_shape_source"], "hist_by_rows": v["hist_by_rows"]}
+                      "launch_shape_source": v["launch_shape_source"],
+                      "rounds_per_iteration": v["rounds_per_iteration"]}
                   for k, v in res.items()},
-        "roofline": {"bound": "hbm", "kernel": f"k_hist ({head})", "achieved": achieved, "peak": peak,
+        "roofline": {"bound": "hbm", "kernel": f"k_round_hist ({head})", "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,
                      "traffic": ((HIST_DRAM_BYTES_PER_ROW_ROOT * len(data["y"]) + HIST_DRAM_BYTES_PER_ROW_SCATTERED *
                                   (r["hist_rows_per_tree"] - len(data["y"]))) /
-                                 (int(data["params"]["num_leaves"]) - 1) if head == "quantized" else None),
+                                 r["rounds_per_iteration"] if head == "quantized" else None),
                      "traffic_note": ("ncu DRAM bytes per row of a 5M-row run (root launch: rows in order; next "
                                       "launch: scattered rows) x the rows of an average launch"),
-                     "bytes_per_launch": r["hist_bytes_per_launch"], "ms_per_launch": r["hist_ms_per_launch"],
-                     # the histogram's achieved fraction of the HBM roofline by leaf size
-                     "by_rows": [dict(b, frac=(b["gbs"] / peak if b["gbs"] else None)) for b in r["hist_by_rows"]]},
+                     "bytes_per_launch": r["hist_bytes_per_launch"], "ms_per_launch": r["hist_ms_per_launch"]},
         "cpu_baseline": cpu, "e2e": e2e,
-        # per iteration: the tree's launches (init, 3 per split, leaf renewal), then the
+        # per iteration: the tree's launches (init, 4 per round, the tree's arrays, leaf renewal), then the
         # gradients, the quantization (max-abs, packing), the leaf shrinkage, the training
         # rows' score update and the held-out rows' scoring
         "gpu_launches": args.steps * (r["kernel_launches_per_tree"] + 1 + (2 if head == "quantized" else 0) + 3),
-        # device-time shares of the three split-step kernels (events around every launch)
+        # device-time shares of a round's three kernels (events around every launch)
         "kernel_share": {k: r[f"{k}_ms_per_step"] / (r["hist_ms_per_step"] + r["scan_ms_per_step"] +
                                                      r["partition_ms_per_step"])
                          for k in ("hist", "scan", "partition")},
         "clocks": r["clocks"],
     }
-    # the row partition, the largest share of device time (its launches are
-    # latency-bound: most leaves are small)
+    # the row partition, the other kernel whose time is its rows
     line["roofline_partition"] = {
-        "bound": "hbm", "kernel": "k_partition", "achieved": r["part_gbs"], "peak": peak, "unit": "GB/s",
+        "bound": "hbm", "kernel": "k_round_part", "achieved": r["part_gbs"], "peak": peak, "unit": "GB/s",
         "frac": r["part_gbs"] / peak, "peak_kind": peak_kind,
-        "traffic": PART_DRAM_BYTES_PER_ROW * r["part_rows_per_tree"] / (int(data["params"]["num_leaves"]) - 1),
+        "traffic": PART_DRAM_BYTES_PER_ROW * r["part_rows_per_tree"] / r["rounds_per_iteration"],
         "traffic_note": "ncu DRAM bytes per row of the 5M-row root split x rows per launch (average)",
         "bytes_per_row": 9, "bytes_per_launch": r["part_bytes_per_launch"],
         "ms_per_launch": r["part_ms_per_launch"]}

@@ -282,8 +282,10 @@ typedef int32_t (*LgbmB200AllReduceFn)(void* device_buf, int64_t count, int32_t 
 int lgbm_b200_learner_set_data_parallel(LgbmB200Learner* h, int64_t row_offset, int64_t global_num_data,
                                         LgbmB200AllReduceFn fn, void* user);
 
-/* Launch shape of the per-split-step kernels (the default launch strategy;
- * the persistent one has none). No field changes a result: the shapes differ
+/* Launch shape of the growth kernels (the default launch strategy;
+ * the persistent one has none). A round of the default growth divides
+ * its rows evenly over the histogram's CTAs; hist_rows_per_block counts where
+ * trees grow split by split. No field changes a result: the shapes differ
  * only in speed. No counterpart in the reference, whose CPU learner has a
  * thread count instead. */
 typedef struct {
@@ -305,8 +307,8 @@ int lgbm_b200_learner_set_launch_shape(LgbmB200Learner* h, const LgbmB200LaunchS
 int lgbm_b200_learner_autotune(LgbmB200Learner* h, const LgbmB200LaunchShape* candidates, int32_t num_candidates,
                                int32_t reps, int32_t* chosen, double* ms_per_tree);
 
-/* Per-kernel timing: when enabled, every split step of the next train calls
- * is bracketed by CUDA events on the learner's stream (no extra syncs). */
+/* Per-kernel timing: when enabled, every round (or, where trees grow split by
+ * split, every split step) of the next train calls is bracketed by CUDA events on the learner's stream (no extra syncs). */
 int lgbm_b200_learner_set_timing(LgbmB200Learner* h, int32_t enabled);
 /* Timing marks: record event `mark` (0..15) on the learner's stream; the
  * elapsed device time between two recorded marks, in ms. */
@@ -316,10 +318,11 @@ int lgbm_b200_learner_elapsed(LgbmB200Learner* h, int32_t a, int32_t b, double* 
  * [histogram, scan, partition, other]; rows histogrammed; kernels launched. */
 int lgbm_b200_learner_last_timing(LgbmB200Learner* h, double* ms, int64_t* hist_rows, int32_t* launches);
 /* With timing on (lgbm_b200_learner_set_timing), the device time of the
- * histogram, scan and partition launches of every split step of the last
- * train call: ms[3 * step + {0, 1, 2}] for step < min(*steps, capacity).
- * Histogram step s builds the smaller child of split s - 1 (step 0: the
- * root). A diagnostic with no counterpart in the reference. */
+ * histogram, scan and partition launches of every round of the last train
+ * call (of every split step where trees grow split by split):
+ * ms[3 * step + {0, 1, 2}] for step < min(*steps, capacity). Step 0's
+ * histogram is the root's, a later one's the smaller child of every node
+ * whose rows the step partitioned. A diagnostic with no counterpart in the reference. */
 int lgbm_b200_learner_step_times(LgbmB200Learner* h, float* ms, int32_t capacity, int32_t* steps);
 /* Rows of the last train call: histogrammed by the histogram kernel, and
  * moved by the partition. For the bench's bandwidth figures; no

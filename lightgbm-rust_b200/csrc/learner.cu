@@ -2,10 +2,11 @@
 //
 // A learner handle owns the uploaded bin matrix and, per tree slot, every
 // device buffer the grow loop touches. One train call enqueues the whole
-// tree (init, then num_leaves-1 steps of histogram / scan / partition) on
-// the handle's stream without reading anything back until the tree is done
-// (optionally replayed from a captured CUDA graph), then copies the tree
-// arrays back and rebuilds the reference's Tree layout on the host.
+// tree (init, then rounds of partition / histogram / scan / decision, repeated
+// by a conditional node of a captured CUDA graph) on the handle's stream
+// without reading anything back until the tree is done, then copies the tree
+// arrays back and rebuilds the reference's Tree layout on the host. Without
+// the graph, or with timing on, the host reads one word a round.
 #include <cstdlib>
 #include <algorithm>
 #include <functional>

@@ -1,10 +1,13 @@
 // The tree learner's sm_100a kernels. One tree (or one tree per class slot,
-// grown in lockstep) is grown entirely on the device: every kernel reads
-// the current leaf, counts and split from the slot's control block, so the
-// per-split launches need no host round trip and can be captured in a CUDA
-// graph.
+// grown together) is grown entirely on the device: every kernel reads what it
+// works on from the slot's control block, so no launch needs a host round
+// trip and all of them can be captured in a CUDA graph.
 //
-// Per split step (learner/mod.rs:653-666):
+// Trees grow in rounds of many splits (round_kernels.cuh, included at the
+// end), whose kernels share the histogram, scan and partition bodies below.
+// The data-parallel learner, the persistent launch and the cooperative scan
+// and partition grow them one split at a time; per split step
+// (learner/mod.rs:653-666):
 //   k_hist       histogram of the smaller leaf      (multi_val_bin.rs:556-703)
 //   k_scan       fix / subtract / threshold scan per feature, then in the
 //                last CTA: best split per leaf, best leaf, Tree::split
