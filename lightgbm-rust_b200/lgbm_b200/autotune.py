@@ -1,14 +1,15 @@
-"""Launch-shape autotuner for the tree learner's per-step kernels.
+"""Launch-shape autotuner for the tree learner's growth kernels.
 
-A split step launches the histogram of the smaller leaf, the threshold scans
-and the row partition. Three knobs of those launches change their speed and
-nothing else (every shape grows the same trees):
+A growth round launches the row partition of the nodes it expands, the
+histograms of their smaller children and the threshold scans. Three knobs of
+those launches change their speed and nothing else (every shape grows the
+same trees):
 
 - ``partition_ctas``: CTAs of the row partition per tree slot;
 - ``hist_ctas``: histogram CTAs per tree slot and feature tile (a multiple of
   the histogram cluster size);
 - ``hist_rows_per_block``: the least rows a histogram CTA takes, which sets
-  how many CTAs a small leaf spreads over.
+  how many CTAs a round's rows spread over.
 
 ``tune`` searches them one knob at a time around the learner's built-in
 shape, then confirms the winner against that shape in one more pass. Each
@@ -18,7 +19,8 @@ gradients and quantization offsets, so the same trees, and the random
 streams of later trees untouched). The learner keeps the fastest shape.
 ``record`` and ``lookup`` keep the choices per workload in
 ``launch_shapes.json`` beside this module, keyed by workload and histogram
-form, with the device they were measured on.
+form, with the device they were measured on. A record holds for the kernels it was
+measured on and is taken out when those change.
 """
 import json
 import os
@@ -32,12 +34,11 @@ def candidates(base, knob):
     """The values of one knob to try, around the built-in shape ``base``
     (ascending, duplicates removed, ``base[knob]`` included).
 
-    The partition's default is 3 CTAs per SM, which the kernel's registers
-    allow resident at once; the candidates go down to one CTA per 16 SMs
-    (tree slots batched in one launch share the SMs: K = 10 class trees
-    measured fastest at the lowest candidates). The histogram's default is
-    every cluster resident at once; the candidates are an eighth, a quarter,
-    a half and all of it."""
+    The partition's default is 6 CTAs per SM, shared by the tree slots (3 for
+    growth step by step); the candidates go down to a forty-eighth of it. The
+    histogram's default is every CTA resident at once, shared by the slots
+    and feature tiles; the candidates are an eighth, a quarter, a half and
+    all of it."""
     if knob not in KNOBS:
         raise ValueError(f"unknown launch-shape knob {knob!r}")
     d = int(base[knob])
