@@ -25,15 +25,38 @@ void set_last_error(const std::string& msg) { g_last_error = msg; }
 
 namespace lgbm_b200 {
 
+constexpr int kMaxLeaves = 8192;
+
+// Opt the kernels whose dynamic shared memory depends on a learner's
+// configuration in to the most any accepted one takes. The limit belongs to
+// the device's context, not to a learner: set to each new learner's own need,
+// it would refuse the launches of the larger learners created before.
+static Status shared_memory_limits() {
+  cudaError_t e = cudaSuccess;
+  auto limit = [&](const void* k, size_t bytes) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  // the per-position leaf kernels hold a 16-byte table entry per leaf
+  for (const void* k : {(const void*)k_leaf_sums, (const void*)k_add_leaf_outputs, (const void*)k_leaf_of_row})
+    limit(k, 16 * (size_t)kMaxLeaves);
+  limit((const void*)k_round_decide, round_decide_smem(kMaxLeaves));
+  limit((const void*)k_round_scan_int, round_scan_int_smem(true));
+  limit((const void*)k_round_scan_f64, round_scan_f64_smem());
+  CU(e);
+  return Status();
+}
+
 static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg, const uint8_t* bins, int64_t n,
                             int32_t nf, const LgbmB200FeatureMeta* metas) {
   h->cfg = *cfg;
   if (n <= 0 || n > INT32_MAX) return Status(LGBM_B200_ERR_INVALID_DATA, "num_data must be in [1, 2^31-1]");
   if (nf <= 0) return Status(LGBM_B200_ERR_INVALID_DATA, "no features");
-  if (cfg->num_leaves > 8192)
+  if (cfg->num_leaves > kMaxLeaves)
     return Status(LGBM_B200_ERR_UNSUPPORTED, "num_leaves above 8192 on the device learner");
   h->device = cfg->device;
   CU(cudaSetDevice(h->device));
+  Status s = shared_memory_limits();
+  if (!s.ok()) return s;
   cudaDeviceProp prop;
   CU(cudaGetDeviceProperties(&prop, h->device));
   h->num_sms = prop.multiProcessorCount;
@@ -115,10 +138,6 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
   // clusters above 8 CTAs are a non-portable size the kernel must opt into
   if (hist_cluster(mode) > 8) CU(cudaFuncSetAttribute(hk, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   h->scan_smem = sizeof(ScanSmem);
-  // the per-position leaf kernels hold a 16-byte table entry per leaf
-  CU(cudaFuncSetAttribute(k_leaf_sums, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * h->L));
-  CU(cudaFuncSetAttribute(k_add_leaf_outputs, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * h->L));
-  CU(cudaFuncSetAttribute(k_leaf_of_row, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * h->L));
   CU(cudaFuncSetAttribute(k_scan<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->scan_smem));
   CU(cudaFuncSetAttribute(k_scan<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->scan_smem));
   CU(cudaFuncSetAttribute(k_scan<false, kScanWideBlocks>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -177,7 +196,7 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
   // device buffers
   DeviceArena& A = h->arena;
   uint8_t* bins_d;
-  Status s = A.alloc_n(&bins_d, (size_t)n * h->stride);
+  s = A.alloc_n(&bins_d, (size_t)n * h->stride);
   if (!s.ok()) return s;
   {
     // host copy with the padded row stride, uploaded once
@@ -367,9 +386,6 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
     const void* scan = quant ? (const void*)k_round_scan_int : (const void*)k_round_scan_f64;
     const int scan_threads = quant ? kScanThreads : kF64ScanThreads;
     h->round_scan_smem = quant ? round_scan_int_smem(cats) : round_scan_f64_smem();
-    CU(cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->round_scan_smem));
-    CU(cudaFuncSetAttribute(k_round_decide, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)round_decide_smem(L)));
     int per_sm = 0;
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, scan, scan_threads, h->round_scan_smem));
     h->round_scan_grid = std::max(1, per_sm * h->num_sms / K);
