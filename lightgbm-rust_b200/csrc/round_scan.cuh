@@ -138,9 +138,12 @@ struct CatScratch {
 };
 
 // The accumulated hessian integers a threshold may have: [lo, hi], hi < lo
-// when there are none. Counts and hessian sums only grow in scan order, so a
-// threshold passes the reference's data and hessian minima on both sides
-// exactly within a range, which depends on the leaf alone.
+// when there are none. Where counts and hessian sums only grow in scan order,
+// a threshold passes the reference's data and hessian minima on both sides
+// exactly within a range, which depends on the leaf alone. They need not grow:
+// the reference sums the root's packed values by position when it bags
+// (quant.rs:452-477), so the most frequent bin, which takes what the other
+// bins leave of that sum, can hold a negative hessian.
 struct HessRange {
   uint32_t lo, hi;
 };
@@ -261,24 +264,61 @@ __device__ __forceinline__ bool scan_direction_packed(const int64_t* view, const
     return gain_estimate((float)int_grad((int64_t)a) * gsf, (float)int_hess((int64_t)a) * hsf,
                          (float)int_grad((int64_t)rest) * gsf, (float)int_hess((int64_t)rest) * hsf, l2f);
   };
-  auto admissible = [&](uint64_t a) {
-    const uint32_t h = int_hess((int64_t)a);
-    return h >= range.lo && h <= range.hi;
-  };
-  // which thresholds are admissible, and their estimates
+  // which thresholds are admissible (extra: the candidate t = -1, lane 0's)
   uint32_t pend = 0;
+  bool extra = first_extra && lane == 0;
+  bool falls = (base >> 31 & 1) != 0;  // a negative hessian: the sums do not only grow
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) falls |= (x[j] >> 31 & 1) != 0;
+  if (!__any_sync(0xffffffffu, falls)) {
+    auto admissible = [&](uint64_t a) {
+      const uint32_t h = int_hess((int64_t)a);
+      return h >= range.lo && h <= range.hi;
+    };
+#pragma unroll
+    for (int j = 0; j < kPer; ++j)
+      if ((visited >> j & 1) && admissible(q[j])) pend |= 1u << j;
+    extra = extra && admissible(base);
+  } else {
+    // the reference's tests one by one: too little on the accumulated side
+    // passes over a threshold, on the other side it ends the scan
+    uint32_t stop = 0;
+    auto test = [&](uint64_t a, bool& end) {
+      const double h = (double)int_hess((int64_t)a);
+      const int32_t ac = round_int(h * cnt_factor);
+      if (ac < p.min_data_in_leaf || h * lc.hs < p.min_sum_hessian_in_leaf) return false;
+      end = lc.num_data - ac < p.min_data_in_leaf ||
+            (double)int_hess((int64_t)(sum - a)) * lc.hs < p.min_sum_hessian_in_leaf;
+      return !end;
+    };
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      bool end = false;
+      if ((visited >> j & 1) && test(q[j], end)) pend |= 1u << j;
+      if (end) stop |= 1u << j;
+    }
+    int32_t brk = reverse ? INT32_MIN : INT32_MAX;
+    if (stop) brk = lane * kPer + (reverse ? 31 - __clz(stop) : __ffs(stop) - 1);
+    if (extra) {
+      bool end = false;
+      extra = test(base, end);
+      if (end) brk = -1;
+    }
+    brk = reverse ? __reduce_max_sync(0xffffffffu, brk) : __reduce_min_sync(0xffffffffu, brk);
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const int t = lane * kPer + j;
+      if (reverse ? t <= brk : t >= brk) pend &= ~(1u << j);
+    }
+  }
+  // their estimates
   float est[kPer];
   float most = -INFINITY;
 #pragma unroll
   for (int j = 0; j < kPer; ++j) {
     est[j] = estimate(q[j]);
-    if ((visited >> j & 1) && admissible(q[j])) {
-      pend |= 1u << j;
-      most = fmaxf(most, est[j]);
-    }
+    if (pend >> j & 1) most = fmaxf(most, est[j]);
   }
-  // the extra candidate t = -1 (lane 0)
-  const bool extra = first_extra && lane == 0 && admissible(base);
   if (extra) most = fmaxf(most, estimate(base));
   if (!__any_sync(0xffffffffu, pend != 0 || extra)) return false;
 #pragma unroll
