@@ -137,7 +137,7 @@ struct RNode {
   int32_t side, depth;
   int32_t buf;           // histogram buffer
   int32_t need;          // before_find_best_split of this node and its sibling
-  int32_t pad;
+  int32_t desc;          // 1: its rows lie in the reverse of the root's order
   DLeafSplits ls;
   double cmin, cmax;     // basic monotone constraint
 };
@@ -156,13 +156,19 @@ struct RoundState {
   int32_t done;
   int32_t root;          // 1: the first round, which only searches the root
   int32_t rounds;        // rounds run
-  int32_t ncopy;         // row pieces k_round_restore moves
+  int32_t npiece;        // row pieces of the leaves that lost their lists (k_round_restore, k_round_order)
+  int32_t disorder;      // 1: some piece is not ascending or descending (k_round_order leaves the pieces as they are)
   int32_t ncand, nfree;  // lengths of cand and free
   double root_value;     // the root's output
 };
-// A run of rows to copy into the other index buffer (k_round_restore).
-struct RCopy {
-  int32_t begin, count, side, pad;
+// A run of rows of a leaf that lost its list to its descendants'
+// (k_round_restore, k_round_order).
+struct RPiece {
+  int32_t begin, count, side;  // in index buffer `side`
+  int32_t desc;                // 1: descending rows
+  int32_t leaf;
+  int32_t first, num;          // the leaf's pieces
+  int32_t leaf_desc;           // 1: the leaf's own list is descending
 };
 struct DRounds {
   RoundState* st;
@@ -180,11 +186,11 @@ struct DRounds {
   int32_t* free;         // [pool]: unused histogram buffers
   int32_t* free_next;    // [pool]: scratch, the buffers a round gives back
   int32_t* leaf_node;    // [num_leaves]: the node of each leaf of the replayed tree
-  int32_t* pop_node;     // [num_leaves]: the node and leaf of each split of the replayed tree
-  int32_t* pop_leaf;
+  int32_t* pop_node;     // [num_leaves]: the node of each split of the replayed tree
   int32_t* pop_time;     // [node] scratch of k_round_emit: split index, -1
   int32_t* node_leaf;    // [node] scratch of k_round_emit: leaf index, -1
-  RCopy* copy;           // [ecap + 1]
+  RPiece* piece;         // [ecap + 1]
+  int32_t* piece_num;    // [2][num_leaves] scratch of k_round_emit: each leaf's pieces, and those placed so far
   unsigned long long* status;  // look-back words of a round's row tiles
   int32_t ecap, bmax, pool;
   int32_t share, least;  // a round expands at most 1 / share of the splits to come, but may take `least`

@@ -360,10 +360,10 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
       ALLOC(r.free_next, pool);
       ALLOC(r.leaf_node, L);
       ALLOC(r.pop_node, L);
-      ALLOC(r.pop_leaf, L);
       ALLOC(r.pop_time, nodes);
       ALLOC(r.node_leaf, nodes);
-      ALLOC(r.copy, (size_t)ecap + 1);
+      ALLOC(r.piece, (size_t)ecap + 1);
+      ALLOC(r.piece_num, 2 * (size_t)L);
       ALLOC(r.status, max_tiles + bmax);
       CU(cudaMemset(r.st, 0, sizeof(RoundState)));
       CU(cudaMemset(r.status, 0, (max_tiles + bmax) * sizeof(unsigned long long)));
@@ -549,6 +549,10 @@ static Status enqueue_round(LgbmB200Learner* h, cudaStream_t s, bool root, cudaG
   return Status();
 }
 
+static bool renews_leaves(const LgbmB200Learner* h) {
+  return h->cfg.hist_precision == LGBM_B200_HIST_QUANT && h->cfg.quant_train_renew_leaf;
+}
+
 // The rounds of one tree set. Under capture they are a conditional loop of
 // the graph, which the decision kernel ends; otherwise the host reads back
 // after every round whether another one runs.
@@ -604,6 +608,10 @@ static Status enqueue_rounds(LgbmB200Learner* h) {
   CU_LAUNCH();
   k_round_restore<<<dim3(std::max(1, 2 * h->num_sms / h->K), 1, h->K), 256, 0, s>>>(h->ctx);
   CU_LAUNCH();
+  if (renews_leaves(h)) {  // the renewal's sums follow the lists' order
+    k_round_order<<<dim3(std::max(1, 2 * h->num_sms / h->K), 1, h->K), 256, 0, s>>>(h->ctx);
+    CU_LAUNCH();
+  }
   return Status();
 }
 
@@ -645,15 +653,15 @@ Status enqueue_tree(LgbmB200Learner* h) {
       CU_LAUNCH();
     }
   }
-  if (mode == LGBM_B200_HIST_QUANT && h->cfg.quant_train_renew_leaf) {
+  if (renews_leaves(h)) {
     k_leaf_sums<<<dim3(leaf_sum_warps(h) / 8, 1, K), 256, 16 * (size_t)L, s>>>(c, h->leaf_sums, h->leaf_rank);
     CU_LAUNCH();
     k_leaf_renew<<<dim3((L + 7) / 8, 1, K), 256, 0, s>>>(c, h->leaf_sums, h->leaf_rank, leaf_sum_warps(h), nullptr);
     CU_LAUNCH();
   }
   // a tree in rounds adds its rounds' launches when it is read back
-  h->tree_launches = 1 + (h->rounds ? 2 : h->cfg.persistent_grow ? 1 : 2 * (L - 1) + (c.defer ? 1 : 0)) +
-                     ((mode == LGBM_B200_HIST_QUANT && h->cfg.quant_train_renew_leaf) ? 2 : 0);
+  h->tree_launches = 1 + (h->rounds ? 2 + renews_leaves(h) : h->cfg.persistent_grow ? 1 : 2 * (L - 1) + (c.defer ? 1 : 0)) +
+                     (renews_leaves(h) ? 2 : 0);
   return Status();
 }
 
@@ -1350,6 +1358,12 @@ int lgbm_b200_learner_get_partition(LgbmB200Learner* h, int32_t slot, int32_t* l
   const int nl = std::max(1, h->st_h[slot].num_leaves_cur);
   std::vector<int32_t> side((size_t)nl), beg((size_t)nl), cnt((size_t)nl);
   cudaStream_t s = h->stream;
+  if (h->rounds && h->trained) {  // leaves that lost their lists in the lists' order
+    DCtx c = h->ctx;
+    c.slots[0] = h->ctx.slots[slot];
+    k_round_order<<<2 * h->num_sms, 256, 0, s>>>(c);
+    if (cudaGetLastError() != cudaSuccess) return fail(Status(LGBM_B200_ERR_CUDA, "launch"));
+  }
   cudaMemcpyAsync(beg.data(), d.leaf_begin, sizeof(int32_t) * nl, cudaMemcpyDeviceToHost, s);
   cudaMemcpyAsync(cnt.data(), d.leaf_count, sizeof(int32_t) * nl, cudaMemcpyDeviceToHost, s);
   cudaMemcpyAsync(side.data(), d.leaf_side, sizeof(int32_t) * nl, cudaMemcpyDeviceToHost, s);

@@ -110,7 +110,7 @@ __device__ void round_init(const DCtx& c, const DSlot& s, int32_t need) {
   nd.depth = 0;
   nd.buf = 0;
   nd.need = need;
-  nd.pad = 0;
+  nd.desc = 0;
   nd.ls = st->smaller;
   nd.ls.weight = 0.0;
   nd.cmin = s.cmin[0];
@@ -130,7 +130,7 @@ __device__ void round_init(const DCtx& c, const DSlot& s, int32_t need) {
   rs->done = 0;
   rs->root = 1;
   rs->rounds = 0;
-  rs->ncopy = 0;
+  rs->npiece = 0;
   rs->ncand = 0;
   rs->nfree = r.pool - 1;
   rs->root_value = s.tree.leaf_value[0];

@@ -54,6 +54,7 @@ __device__ void round_children(const DCtx& c, const DSlot& s, int32_t e, const R
   b.count = nr;
   a.side = b.side = 1 - up.side;
   a.depth = b.depth = up.depth + 1;
+  b.desc = 1 - up.desc;
   const bool left_smaller = nl < nr;
   a.buf = left_smaller ? it.buf : up.buf;
   b.buf = left_smaller ? up.buf : it.buf;
@@ -380,7 +381,6 @@ __device__ int32_t replay(const DRounds& r, const NodeFacts& nd, int32_t* ln, in
       nd.exp[v] = e | kReplayed;
       r.exp[v] = e | kReplayed;
       r.pop_node[popped] = v;
-      r.pop_leaf[popped] = l;
       ln[l] = a;
       ln[R] = b;
     }
@@ -683,11 +683,11 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
 // reference's tree arrays (Tree::split, tree.rs:254-297) and leaf ranges. A
 // leaf that was expanded past its children has lost its own row list to its
 // grandchildren's; its rows then lie in the ranges of the unexpanded nodes
-// under it, and the ones in the wrong index buffer are listed for
-// k_round_restore.
+// under it, which are listed leaf by leaf for k_round_restore and
+// k_round_order.
 __global__ void __launch_bounds__(kDecideThreads) k_round_emit(const __grid_constant__ DCtx c) {
   __shared__ unsigned long long warp_sums[kDecideThreads / 32];
-  __shared__ int32_t s_bad, s_copies;
+  __shared__ int32_t s_bad;
   const DSlot& s = c.slots[blockIdx.z];
   const DRounds& r = s.r;
   RoundState* rs = r.st;
@@ -699,10 +699,10 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_emit(const __grid_cons
     r.pop_time[v] = -1;
     r.node_leaf[v] = -1;
   }
-  if (tid == 0) {
-    s_bad = 0;
-    s_copies = 0;
-  }
+  int32_t* piece_num = r.piece_num;
+  int32_t* placed = r.piece_num + c.p.num_leaves;
+  for (int32_t l = tid; l <= P; l += kDecideThreads) piece_num[l] = placed[l] = 0;
+  if (tid == 0) s_bad = 0;
   __syncthreads();
   for (int32_t i = tid; i < P; i += kDecideThreads) r.pop_time[r.pop_node[i]] = i;
   for (int32_t l = tid; l <= P; l += kDecideThreads) r.node_leaf[r.leaf_node[l]] = l;
@@ -770,25 +770,41 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_emit(const __grid_cons
       t.leaf_depth[l] = nd.depth;
     }
   }
-  // unexpanded nodes under a leaf that lost its list
-  for (int32_t v = tid; v < N; v += kDecideThreads) {
-    if (r.exp[v] >= 0 || r.node_leaf[v] >= 0) continue;
-    int32_t up = r.node[v].parent, depth = 1;
-    while (r.node_leaf[up] < 0) {
-      up = r.node[up].parent;
-      ++depth;
+  // unexpanded nodes under a leaf that lost its list: visit(node, leaf, the leaf's node)
+  auto each_piece = [&](auto visit) {
+    for (int32_t v = tid; v < N; v += kDecideThreads) {
+      if (r.exp[v] >= 0 || r.node_leaf[v] >= 0 || r.node[v].count == 0) continue;
+      int32_t up = r.node[v].parent;
+      while (r.node_leaf[up] < 0) up = r.node[up].parent;
+      const int32_t e = r.exp[up];
+      if (r.exp[2 * e + 1] >= 0 || r.exp[2 * e + 2] >= 0) visit(v, r.node_leaf[up], up);
     }
-    const int32_t e = r.exp[up];
-    const bool lost = r.exp[2 * e + 1] >= 0 || r.exp[2 * e + 2] >= 0;
-    const RNode& nd = r.node[v];
-    if (lost && (depth & 1) == 0 && nd.count > 0) {
-      const int32_t at = atomicAdd(&s_copies, 1);
-      r.copy[at] = RCopy{nd.begin, nd.count, nd.side, 0};
-    }
+  };
+  each_piece([&](int32_t, int32_t l, int32_t) { atomicAdd(&piece_num[l], 1); });
+  __syncthreads();
+  int32_t pieces = 0;
+  for (int32_t l0 = 0; l0 <= P; l0 += kDecideThreads) {
+    const int32_t l = l0 + tid;
+    const int32_t num = l <= P ? piece_num[l] : 0;
+    unsigned long long tot;
+    const int32_t first = (int32_t)block_prefix<kDecideThreads>((unsigned long long)num, warp_sums, tot);
+    if (l <= P) placed[l] = pieces + first;
+    pieces += (int32_t)tot;
   }
   __syncthreads();
+  each_piece([&](int32_t v, int32_t l, int32_t up) {
+    const RNode& nd = r.node[v];
+    const int32_t at = atomicAdd(&placed[l], 1);
+    r.piece[at] = RPiece{nd.begin, nd.count, nd.side, nd.desc, l, 0, piece_num[l], r.node[up].desc};
+  });
+  __syncthreads();
+  for (int32_t i = tid; i < pieces; i += kDecideThreads) {
+    const int32_t l = r.piece[i].leaf;
+    r.piece[i].first = placed[l] - piece_num[l];
+  }
   if (tid == 0) {
-    rs->ncopy = s_copies;
+    rs->npiece = pieces;
+    rs->disorder = 0;
     st->num_leaves_cur = P + 1;
     st->num_cat = cats;
     if (s_bad && st->status == kStatusOk) st->status = kStatusEmptyChild;
@@ -796,24 +812,75 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_emit(const __grid_cons
   }
 }
 
-// The listed row pieces copied into the other index buffer, at the same
-// positions (every piece owns its positions in both). Grid (G, 1, slots).
+// The listed row pieces that lie in the leaf's own buffer copied into the
+// other one, at the same positions (every piece owns its positions in both),
+// and every piece's order checked. Grid (G, 1, slots).
 __global__ void __launch_bounds__(256) k_round_restore(const __grid_constant__ DCtx c) {
-  __shared__ RCopy piece[256];
+  __shared__ RPiece piece[256];
   const DSlot& s = c.slots[blockIdx.z];
-  const int32_t n = s.r.st->ncopy;
+  const int32_t n = s.r.st->npiece;
+  bool disorder = false;
   for (int32_t i0 = 0; i0 < n; i0 += 256) {
     const int32_t m = min(256, n - i0);
     __syncthreads();
-    if ((int)threadIdx.x < m) piece[threadIdx.x] = s.r.copy[i0 + threadIdx.x];
+    if ((int)threadIdx.x < m) piece[threadIdx.x] = s.r.piece[i0 + threadIdx.x];
     __syncthreads();
     for (int32_t i = 0; i < m; ++i) {
-      const RCopy p = piece[i];
+      const RPiece p = piece[i];
+      const int32_t target = s.leaf_side[p.leaf];
       const uint32_t* from = s.idx[p.side] + p.begin;
-      uint32_t* to = s.idx[1 - p.side] + p.begin;
+      uint32_t* to = s.idx[target] + p.begin;
       // small pieces start at different CTAs
       const uint32_t b = (blockIdx.x + (uint32_t)i * 37u) % gridDim.x;
-      for (uint32_t k = b * 256u + threadIdx.x; k < (uint32_t)p.count; k += gridDim.x * 256u) to[k] = from[k];
+      for (uint32_t k = b * 256u + threadIdx.x; k < (uint32_t)p.count; k += gridDim.x * 256u) {
+        const uint32_t row = from[k];
+        if (k + 1 < (uint32_t)p.count) disorder |= (from[k + 1] < row) != (p.desc != 0);
+        if (p.side != target) to[k] = row;
+      }
     }
+  }
+  if (disorder) s.r.st->disorder = 1;
+}
+
+// Rows of the list x[0, n) below `row`.
+__device__ __forceinline__ int32_t rows_below(const uint32_t* x, int32_t n, bool desc, uint32_t row) {
+  int32_t lo = 0, hi = n;  // the first place on the other side of `row`
+  while (lo < hi) {
+    const int32_t mid = (lo + hi) >> 1;
+    if ((x[mid] < row) != desc) lo = mid + 1;
+    else hi = mid;
+  }
+  return desc ? n - lo : lo;
+}
+
+// The rows of the leaves that lost their lists in the lists' own order, that
+// of growth split by split: a split keeps its left rows' order and reverses
+// its right rows', so every list of the tree is ascending or descending and a
+// row's place is its rank among the leaf's pieces, found by bisection. The
+// pieces lie in the children's buffer (k_round_restore); the leaf's own takes
+// the result. Without this, sums in list order (k_leaf_sums) would depend on
+// how far the rounds had expanded a leaf, and so on the memory that was free
+// for the explored nodes. Grid (G, 1, slots); a second run changes nothing.
+__global__ void __launch_bounds__(256) k_round_order(const __grid_constant__ DCtx c) {
+  const DSlot& s = c.slots[blockIdx.z];
+  const DRounds& r = s.r;
+  const int32_t n = r.st->npiece;
+  if (r.st->disorder) return;
+  for (int32_t i = 0; i < n; ++i) {
+    const RPiece p = r.piece[i];
+    const int32_t own = r.node[r.leaf_node[p.leaf]].side, lb = s.leaf_begin[p.leaf], lc = s.leaf_count[p.leaf];
+    const uint32_t* from = s.idx[1 - own];
+    const uint32_t b = (blockIdx.x + (uint32_t)i * 37u) % gridDim.x;
+    for (uint32_t k = b * 256u + threadIdx.x; k < (uint32_t)p.count; k += gridDim.x * 256u) {
+      const uint32_t row = from[p.begin + k];
+      int32_t rank = p.desc ? p.count - 1 - (int32_t)k : (int32_t)k;
+      for (int32_t q = p.first; q < p.first + p.num; ++q) {
+        if (q == i) continue;
+        const RPiece& o = r.piece[q];
+        rank += rows_below(from + o.begin, o.count, o.desc != 0, row);
+      }
+      s.idx[own][lb + (p.leaf_desc ? lc - 1 - rank : rank)] = row;
+    }
+    if (i == p.first && b == 0 && threadIdx.x == 0) s.leaf_side[p.leaf] = own;
   }
 }
