@@ -1205,12 +1205,15 @@ __device__ __noinline__ bool scan_categorical(Scratch& sm, const DFeature m, con
       sm.key[k] = G(i) / (H(i) + p.cat_smooth);
     }
     __syncwarp();
+    // NaN keys (an empty bin without smoothing, NaN gradients) come after the
+    // numbers, in bin order: the ranks are a permutation whatever the keys
+    auto before = [](double a, double b) { return a < b || (b != b && a == a); };
     for (int k = lane; k < used_bin; k += 32) {
       double kk = sm.key[k];
       int rank = 0;
       for (int j = 0; j < used_bin; ++j) {
         double kj = sm.key[j];
-        if (kj < kk || (j < k && !(kk < kj) && !(kj < kk))) ++rank;
+        if (before(kj, kk) || (j < k && !before(kk, kj))) ++rank;
       }
       sm.sorted[rank] = sm.tpos[k];
     }
@@ -1387,9 +1390,11 @@ __device__ __noinline__ bool scan_categorical(Scratch& sm, const DFeature m, con
       for (int w = 0; w < kCatWords; ++w) out.cat_bits[w] = 0;
       int32_t ncat = 0;
       if (use_onehot) {
-        uint32_t b = (uint32_t)(best_threshold + offset);
-        out.cat_bits[b >> 5] |= 1u << (b & 31);
-        ncat = 1;
+        if (best_threshold >= 0) {  // -1 where every gain is NaN
+          uint32_t b = (uint32_t)(best_threshold + offset);
+          out.cat_bits[b >> 5] |= 1u << (b & 31);
+          ncat = 1;
+        }
       } else {
         for (int32_t i = 0; i <= best_threshold; ++i) {
           uint32_t b = (uint32_t)((best_dir == 1 ? sm.sorted[i] : sm.sorted[used_bin - 1 - i]) + offset);
