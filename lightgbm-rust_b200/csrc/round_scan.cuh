@@ -17,13 +17,21 @@
 // value's relative error is below 1e-6 (four roundings and an approximate
 // divide), so the FP64 maximum and its ties are always among those, and the
 // result is the FP64 search's bit for bit. (Only the largest gain decides
-// whether a feature is splittable.) Parameters that change the gain's formula
-// (L1, max_delta_step, path smoothing, monotone bounds) evaluate all in FP64.
+// whether a feature is splittable.) The bound needs divisors well inside
+// FP32's range and a largest gain above 1e-30: a square below FP32's normal
+// numbers is off by up to 2^-150, and over a divisor of 1e-8 or more by 7e-38,
+// which 1e-5 of such a gain covers; the approximate divide returns 0 from a
+// divisor of 2^126 on. Thresholds outside are evaluated in FP64. Parameters
+// that change the gain's formula (L1, max_delta_step, path smoothing, monotone
+// bounds) evaluate all in FP64.
 #pragma once
 
-// FP32 estimate of the plain gain of a threshold.
+// FP32 estimate of the plain gain of a threshold; NaN, which no floor leaves
+// out, where it could be too far off.
 __device__ __forceinline__ float gain_estimate(float lg, float lh, float rg, float rh, float l2) {
-  return __fdividef(lg * lg, lh + l2) + __fdividef(rg * rg, rh + l2);
+  const float ld = lh + l2, rd = rh + l2;
+  const bool safe = fminf(ld, rd) >= 1e-8f && fmaxf(ld, rd) <= 1e37f;
+  return safe ? __fdividef(lg * lg, ld) + __fdividef(rg * rg, rd) : NAN;
 }
 // The estimates from which a threshold is evaluated in FP64, given the
 // largest: all of them when it is outside FP32's comfortable range.
