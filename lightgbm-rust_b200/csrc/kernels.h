@@ -122,6 +122,7 @@ cudaError_t launch_round_hist(int mode, int ng, dim3 grid, size_t smem, cudaStre
                               const DTileTable& tt, int32_t sub_rows);
 // the threshold scans of a round, on packed integer and on FP64 sums
 __global__ void k_round_scan_int(const __grid_constant__ DCtx c);
+__global__ void k_scan_warp(const __grid_constant__ DCtx c);
 __global__ void k_round_scan_f64(const __grid_constant__ DCtx c);
 size_t round_scan_int_smem(bool cat);
 size_t round_scan_f64_smem();

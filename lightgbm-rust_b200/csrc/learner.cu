@@ -41,6 +41,7 @@ static Status shared_memory_limits() {
     limit(k, 16 * (size_t)kMaxLeaves);
   limit((const void*)k_round_decide, round_decide_smem(kMaxLeaves));
   limit((const void*)k_round_scan_int, round_scan_int_smem(true));
+  limit((const void*)k_scan_warp, round_scan_int_smem(true));
   limit((const void*)k_round_scan_f64, round_scan_f64_smem());
   CU(e);
   return Status();
@@ -142,10 +143,9 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
   CU(cudaFuncSetAttribute(k_scan<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->scan_smem));
   CU(cudaFuncSetAttribute(k_scan<false, kScanWideBlocks>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                           (int)h->scan_smem));
-  CU(cudaFuncSetAttribute(k_scan<true, kScanWideBlocks>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                          (int)h->scan_smem));
-  // a step's scans are (feature, side, slot) CTAs: beyond two CTAs per SM they
-  // run in waves, and the register-capped variant keeps more of them resident
+  // a split step's scans are (feature, side, slot) CTAs: beyond two CTAs per SM
+  // they run in waves, where the quantized form takes a warp a scan instead and
+  // the FP64 form the register-capped variant that keeps more CTAs resident
   // (LGBM_B200_SCAN_WIDE=0/1 forces either)
   h->scan_wide = (int64_t)nf * 2 * std::max(1, cfg->num_tree_slots) > 2 * (int64_t)h->num_sms;
   if (const char* e = std::getenv("LGBM_B200_SCAN_WIDE")) h->scan_wide = std::atoi(e) != 0;
@@ -165,6 +165,8 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
   h->part_grid = h->num_sms * 3;  // of a split step: 3 CTAs per SM measured best with 1024-row tiles (2 and 2.5 per SM are slower)
   // LGBM_B200_PART_GRID sets the partition's CTA count (launch-shape sweeps)
   if (const char* e = std::getenv("LGBM_B200_PART_GRID")) h->part_grid = std::max(1, std::atoi(e));
+  h->step_hist_grid = h->hist_grid;
+  h->step_part_grid = h->part_grid;
   // LGBM_B200_SCANPART=1: the threshold scans and the partition of a step run
   // as one cooperative launch (one kernel boundary less per split); the
   // grid is what stays resident at once, shared by the tree slots
@@ -373,6 +375,17 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
     CU(cudaMemset(d.root_counter, 0, sizeof(int32_t)));
     CU(cudaMemset(d.bytree, 1, nf));
   }
+  {  // one scan a warp: what is resident at once, shared by the slots
+    const bool quant = mode == LGBM_B200_HIST_QUANT;
+    bool cats = false;
+    for (auto& f : h->feats) cats |= f.bin_type == 1;
+    h->scan_warp_smem = quant ? round_scan_int_smem(cats) : round_scan_f64_smem();
+    int per_sm = 0;
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &per_sm, quant ? (const void*)k_round_scan_int : (const void*)k_round_scan_f64,
+        quant ? kScanThreads : kF64ScanThreads, h->scan_warp_smem));
+    h->scan_warp_grid = std::max(1, per_sm * h->num_sms / K);
+  }
   if (h->rounds) {
     if (!(s = A.alloc_n(&h->round_ctrl, 3)).ok()) return s;
     CU(cudaMemset(h->round_ctrl, 0, 3 * sizeof(int32_t)));
@@ -380,15 +393,7 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
     const void* hist = round_hist_kernel(mode, h->hist_ng);
     h->round_hist_smem = round_hist_smem(mode, h->hist_ng);
     CU(cudaFuncSetAttribute(hist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->round_hist_smem));
-    const bool quant = mode == LGBM_B200_HIST_QUANT;
-    bool cats = false;
-    for (auto& f : h->feats) cats |= f.bin_type == 1;
-    const void* scan = quant ? (const void*)k_round_scan_int : (const void*)k_round_scan_f64;
-    const int scan_threads = quant ? kScanThreads : kF64ScanThreads;
-    h->round_scan_smem = quant ? round_scan_int_smem(cats) : round_scan_f64_smem();
     int per_sm = 0;
-    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, scan, scan_threads, h->round_scan_smem));
-    h->round_scan_grid = std::max(1, per_sm * h->num_sms / K);
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hist, kHistThreads, h->round_hist_smem));
     h->hist_grid = std::max(1, per_sm * h->num_sms / (h->ntiles * K));
     // a round's partition moves the rows of many leaves: 6 CTAs per SM keep more
@@ -516,10 +521,12 @@ Status quant_tables(LgbmB200Learner* h, int64_t rows) {
   return Status();
 }
 
-// CTAs of a step's histogram launch: whole clusters.
+// CTAs of a step's histogram launch: whole clusters, of the caller's shape or
+// of growth split by split (a learner whose trees grow in rounds keeps
+// another grid in hist_grid).
 static int step_hist_grid(const LgbmB200Learner* h) {
   const int cl = hist_cluster(h->cfg.hist_precision);
-  return (h->hist_grid + cl - 1) / cl * cl;
+  return ((h->shape_set ? h->hist_grid : h->step_hist_grid) + cl - 1) / cl * cl;
 }
 
 // One round's launches on stream s (root: the first, which only searches the
@@ -537,10 +544,10 @@ static Status enqueue_round(LgbmB200Learner* h, cudaStream_t s, bool root, cudaG
   CU(launch_round_hist(h->cfg.hist_precision, h->hist_ng, dim3(h->hist_grid, h->ntiles, K), h->round_hist_smem, s, c,
                        h->tiles, h->sub_rows));
   if (ev) CU(cudaEventRecord(ev[2], s));
-  const dim3 scan_grid(h->round_scan_grid, 1, K);
+  const dim3 scan_grid(h->scan_warp_grid, 1, K);
   if (h->cfg.hist_precision == LGBM_B200_HIST_QUANT)
-    k_round_scan_int<<<scan_grid, kScanThreads, h->round_scan_smem, s>>>(c);
-  else k_round_scan_f64<<<scan_grid, kF64ScanThreads, h->round_scan_smem, s>>>(c);
+    k_round_scan_int<<<scan_grid, kScanThreads, h->scan_warp_smem, s>>>(c);
+  else k_round_scan_f64<<<scan_grid, kF64ScanThreads, h->scan_warp_smem, s>>>(c);
   CU_LAUNCH();
   if (ev) CU(cudaEventRecord(ev[3], s));
   k_round_decide<<<dim3(1, 1, K), kDecideThreads, round_decide_smem(h->L), s>>>(
@@ -679,7 +686,8 @@ static Status launch_scan(LgbmB200Learner* h) {
   const dim3 g(h->nf, 2, h->K);
   cudaStream_t s = h->stream;
   if (h->cfg.hist_precision == LGBM_B200_HIST_QUANT) {
-    if (h->scan_wide) k_scan<true, kScanWideBlocks><<<g, kScanThreads, h->scan_smem, s>>>(c);
+    if (h->scan_wide)
+      k_scan_warp<<<dim3(std::min(2 * h->nf, h->scan_warp_grid), 1, h->K), kScanThreads, h->scan_warp_smem, s>>>(c);
     else k_scan<true, 1><<<g, kScanThreads, h->scan_smem, s>>>(c);
   } else if (h->scan_wide) {
     k_scan<false, kScanWideBlocks><<<g, kScanThreads, h->scan_smem, s>>>(c);
@@ -1036,6 +1044,7 @@ Status set_launch_shape(LgbmB200Learner* h, const LgbmB200LaunchShape& in) {
   h->part_grid = in.partition_ctas;
   h->hist_grid = (in.hist_ctas + cl - 1) / cl * cl;
   h->ctx.rows_per_block = in.hist_rows_per_block;
+  h->shape_set = true;
   if (h->scan_part) h->scan_part_grid = std::max(1, std::min(h->part_grid, h->scan_part_max));
   h->config_epoch += 1;
   if (h->graph_exec) {  // the captured launches carry the old grids
@@ -1426,6 +1435,10 @@ int lgbm_b200_learner_set_data_parallel(LgbmB200Learner* h, int64_t row_offset, 
   h->ctx.dp = 1;
   h->ctx.defer = 0;  // the step's end waits for the left count summed over the ranks
   h->rounds = false;  // step by step: the ranks reduce between a step's launches
+  if (!h->shape_set) {
+    h->hist_grid = h->step_hist_grid;
+    h->part_grid = h->step_part_grid;
+  }
   h->scan_part = false;
   h->cfg.persistent_grow = 0;
   h->cfg.use_cuda_graph = 0;

@@ -256,7 +256,9 @@ struct LgbmB200Learner {
   GrowSync* grow_sync = nullptr;
   long long* phase_ns = nullptr;  // persistent growth: device ns per phase
   size_t hist_smem = 0, scan_smem = 0;
-  int hist_grid = 148, part_grid = 592, root_grid = kRootBlocks;
+  int hist_grid = 148, part_grid = 592, root_grid = kRootBlocks;  // of the learner's form of growth
+  int step_hist_grid = 148, step_part_grid = 444;                 // of growth split by split
+  bool shape_set = false;  // the caller chose the launch shape
   int32_t sub_rows = 8192;
   std::vector<DSlot> slots_h;
   float2* gh_all = nullptr;  // [K x n] interleaved gradients of every slot
@@ -325,8 +327,8 @@ struct LgbmB200Learner {
   bool rounds = false;
   cudaStream_t body_stream = nullptr;  // captures the body of the rounds' loop
   int32_t* round_ctrl = nullptr;       // [3]: slots arrived, slots going on, whether another round runs
-  int round_scan_grid = 0;
-  size_t round_scan_smem = 0, round_hist_smem = 0;
+  int scan_warp_grid = 0;  // CTAs and shared memory of a launch of one scan a warp
+  size_t scan_warp_smem = 0, round_hist_smem = 0;
   int last_rounds = 0;
   // captured tree growth
   cudaGraphExec_t graph_exec = nullptr;

@@ -2081,7 +2081,6 @@ __global__ void __launch_bounds__(kScanThreads, kMinBlocks) k_scan(const __grid_
 template __global__ void k_scan<false, 1>(const __grid_constant__ DCtx);
 template __global__ void k_scan<true, 1>(const __grid_constant__ DCtx);
 template __global__ void k_scan<false, kScanWideBlocks>(const __grid_constant__ DCtx);
-template __global__ void k_scan<true, kScanWideBlocks>(const __grid_constant__ DCtx);
 
 // =====================================================================================
 // partition (partition.rs:107-174): out-of-place split of the leaf's rows into

@@ -435,6 +435,65 @@ constexpr size_t kScanWarpViews = (kScanThreads / 32) * (kViewPad * sizeof(int64
 constexpr size_t kScanWarpBase = kScanWarpViews + (kScanThreads / 32) * sizeof(DSplit);
 size_t round_scan_int_smem(bool cat) { return kScanWarpBase + (cat ? (kScanThreads / 32) * sizeof(CatScratch) : 0); }
 
+// One quantized scan by one warp: feature f, side (0 smaller, 1 larger) of job
+// j, whose histogram views are fixed, subtracted and stored; view, cat and out
+// are the warp's shared memory. The result goes to *dst when the feature is
+// searched (left in `out`, too); returns whether it is splittable.
+__device__ __forceinline__ bool scan_packed(const DCtx& c, const DSlot& s, const DFeature& m, int32_t f, int side,
+                                            const ScanJob& j, bool search, int64_t* view, CatScratch* cat, DSplit& out,
+                                            DSplit* dst) {
+  const int lane = threadIdx.x & 31;
+  const int len = m.view_len;
+  long long* hs = reinterpret_cast<long long*>(s.hist) + (size_t)j.s_buf * c.total_bins + m.view_start;
+  long long* hp = reinterpret_cast<long long*>(s.hist) + (size_t)j.l_buf * c.total_bins + m.view_start;
+  uint64_t v[kPer], pv[kPer];
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int t = 32 * k + lane;
+    // histogram cells are written by other CTAs' atomics: loaded through L2
+    v[k] = t < len ? (uint64_t)__ldcg(hs + t) : 0ull;
+    pv[k] = t < len && side == 1 ? (uint64_t)__ldcg(hp + t) : 0ull;
+  }
+  if (!search) return false;
+  // the smaller leaf's most frequent bin (histogram.rs:42-56; exact in any order)
+  if (m.most_freq_bin > 0) {
+    uint64_t part = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const int t = 32 * k + lane;
+      if (t < m.num_bin && t != m.most_freq_bin) part += v[k];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+    const uint64_t fixed = (uint64_t)j.sl.int_sum - part;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k)
+      if (32 * k + lane == m.most_freq_bin) {
+        v[k] = fixed;
+        if (side == 0) hs[m.most_freq_bin] = (long long)fixed;
+      }
+  }
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int t = 32 * k + lane;
+    if (side == 1) {  // larger = parent - smaller, in the parent's buffer (histogram.rs:59-63)
+      v[k] = pv[k] - v[k];
+      if (t < len) hp[t] = (long long)v[k];
+    }
+    view[view_at(t)] = (int64_t)v[k];
+  }
+  __syncwarp();
+  const bool ok = find_best_threshold_packed(view, cat, m, c.p, c.p_cat, leaf_ctx(c, j), out);
+  if (lane == 0) {
+    out.feature = m.real_index;
+    out.inner = f;
+  }
+  __syncwarp();
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(&out);
+  for (int k = lane; k < (int)(sizeof(DSplit) / 4); k += 32) reinterpret_cast<uint32_t*>(dst)[k] = src[k];
+  return ok;
+}
+
 // Grid (G, 1, slots), kScanThreads threads: each warp takes scans of its own;
 // neighbouring scans go to different CTAs, so a round of few scans spreads
 // over the SMs.
@@ -458,63 +517,49 @@ __global__ void __launch_bounds__(kScanThreads, kScanIntBlocks) k_round_scan_int
     const ScanJob j = round_job(c, s, root, e0 + (item >> 1), side, child, parent, depth);
     if (!j.live) continue;
     const uint8_t split_ok = parent < 0 ? 1 : r.splittable[(size_t)parent * nf + f];
-    const int len = m.view_len;
-    long long* hs = reinterpret_cast<long long*>(s.hist) + (size_t)j.s_buf * c.total_bins + m.view_start;
-    long long* hp = reinterpret_cast<long long*>(s.hist) + (size_t)j.l_buf * c.total_bins + m.view_start;
-    uint64_t v[kPer], pv[kPer];
-#pragma unroll
-    for (int k = 0; k < kPer; ++k) {
-      const int t = 32 * k + lane;
-      // histogram cells are written by other CTAs' atomics: loaded through L2
-      v[k] = t < len ? (uint64_t)__ldcg(hs + t) : 0ull;
-      pv[k] = t < len && side == 1 ? (uint64_t)__ldcg(hp + t) : 0ull;
-    }
+    const bool search = in_tree && split_ok;
     DSplit* dst = r.fres + ((size_t)item * nf + f);
-    bool ok = false;
-    if (in_tree && split_ok) {
-      // the smaller leaf's most frequent bin (histogram.rs:42-56; exact in any order)
-      if (m.most_freq_bin > 0) {
-        uint64_t part = 0;
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-          const int t = 32 * k + lane;
-          if (t < m.num_bin && t != m.most_freq_bin) part += v[k];
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        const uint64_t fixed = (uint64_t)j.sl.int_sum - part;
-#pragma unroll
-        for (int k = 0; k < kPer; ++k)
-          if (32 * k + lane == m.most_freq_bin) {
-            v[k] = fixed;
-            if (side == 0) hs[m.most_freq_bin] = (long long)fixed;
-          }
-      }
-#pragma unroll
-      for (int k = 0; k < kPer; ++k) {
-        const int t = 32 * k + lane;
-        if (side == 1) {  // larger = parent - smaller, in the parent's buffer (histogram.rs:59-63)
-          v[k] = pv[k] - v[k];
-          if (t < len) hp[t] = (long long)v[k];
-        }
-        view[view_at(t)] = (int64_t)v[k];
-      }
-      __syncwarp();
-      ok = find_best_threshold_packed(view, cat, m, c.p, c.p_cat, leaf_ctx(c, j), out);
-      if (lane == 0) {
-        out.feature = m.real_index;
-        out.inner = f;
-      }
-      __syncwarp();
-      const uint32_t* src = reinterpret_cast<const uint32_t*>(&out);
-      for (int k = lane; k < (int)(sizeof(DSplit) / 4); k += 32) reinterpret_cast<uint32_t*>(dst)[k] = src[k];
-    } else if (lane == 0) {
+    const bool ok = scan_packed(c, s, m, f, side, j, search, view, cat, out, dst);
+    if (!search && lane == 0) {
       dst->gain = -INFINITY;
       dst->feature = -1;
       dst->monotone_type = 0;
     }
     if (lane == 0) r.splittable[(size_t)child * nf + f] = ok;
     scans_stored(c, s, item, 1, child, depth);
+  }
+}
+
+// The scans of a split step, a warp each, in the place of k_scan where those
+// would run in waves (data-parallel growth of quantized trees on many
+// features: a block scan's 256 threads and barriers per scan are for few of
+// them). Grid (G, 1, slots), kScanThreads threads.
+__global__ void __launch_bounds__(kScanThreads, kScanIntBlocks) k_scan_warp(const __grid_constant__ DCtx c) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int kWarps = kScanThreads / 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int64_t* view = reinterpret_cast<int64_t*>(smem_raw) + (size_t)warp * kViewPad;
+  DSplit& out = reinterpret_cast<DSplit*>(smem_raw + kScanWarpViews)[warp];
+  CatScratch* cat = reinterpret_cast<CatScratch*>(smem_raw + kScanWarpBase) + warp;
+  const DSlot& s = c.slots[blockIdx.z];
+  const int32_t nf = c.num_features;
+  // the partition that follows claims its row tiles from this counter
+  if (blockIdx.x == 0 && threadIdx.x == 0 && !s.st->done) {
+    s.st->part_ticket = 0;
+    s.st->part_done = 0;
+  }
+  for (int32_t w = warp * gridDim.x + blockIdx.x; w < 2 * nf; w += kWarps * gridDim.x) {
+    const int32_t side = w / nf, f = w - side * nf;
+    const DFeature m = c.feats[f];
+    int32_t larger_leaf, L;
+    const ScanJob j = step_job(c, s, f, side, larger_leaf, L);
+    if (!j.live) continue;
+    if (!s.bytree[f] || (larger_leaf >= 0 && !s.splittable[L * nf + f])) continue;
+    const bool ok = scan_packed(c, s, m, f, side, j, true, view, cat, out, j.out);
+    if (lane == 0) s.feat_ok[w] = ok ? 1 : 0;
+    // the partition's goes-left table for this candidate, ready if it wins
+    if (ok) build_partition_lut(m, out, s.lut_cand + (size_t)w * kMaxBins, lane, 32);
+    __syncwarp();
   }
 }
 
