@@ -47,6 +47,96 @@ static Status shared_memory_limits() {
   return Status();
 }
 
+// The histogram buffers of every slot and, for growth in rounds, the arrays of
+// the explored tree. Allocated after everything else, because their sizes
+// follow the memory left. The explored tree may hold up to 16 times the splits
+// of the finished one: 1.4 times is usual, 2 to 3 times on late trees of a run,
+// whose gains hardly fall with depth. Only the nodes that may still be split
+// hold a histogram, so three times the splits suffice there. Both shrink when
+// that would take more than a sixteenth (nodes) or an eighth (histograms) of
+// what the learner's own needs leave free, the buffers that training adds later
+// among them; with none to spare, the rounds shrink to the one node the replay
+// waits for.
+static Status alloc_pools(LgbmB200Learner* h, size_t cells, size_t max_tiles) {
+  const int K = h->K, L = h->L, nf = h->nf;
+  DeviceArena& A = h->arena;
+  Status s;
+  int32_t ecap = 0, bmax = 0, pool = L, share = 6, least = 16;
+  if (h->rounds) {
+    const int32_t need = L - 1;
+    // A round costs about 50 us however few nodes it expands; an expansion
+    // costs two scans per feature and slot, of which the GPU does about 200 a
+    // microsecond. Many slots and features make a wasted expansion dear:
+    // multiclass K=10 x 200 features 7.7 ms an iteration at a quarter (at least
+    // 24), 6.9 at a sixth (12), 6.5 at a tenth (8); binary x 28 1.24, 1.20 and
+    // 1.4 ms.
+    if (2 * (int64_t)nf * K > 1000) {
+      share = 10;
+      least = 8;
+    }
+    bmax = std::max(1, std::min(kMaxRoundItems, std::max(least, (need + share - 1) / share)));
+    size_t free_b = 0, total_b = 0;
+    CU(cudaMemGetInfo(&free_b, &total_b));
+    const size_t hist_b = cells * 8 * (size_t)K;
+    const size_t node_b = 2 * (sizeof(RNode) + sizeof(DSplit) + sizeof(RPiece) + (size_t)nf + 64) * (size_t)K;
+    const size_t fixed = 2 * (size_t)bmax * nf * sizeof(DSplit) * K + max_tiles * 8 * K;
+    // host gradients and scores staged by the learner, and a booster's scores, labels and bag
+    const size_t later = (size_t)h->n * (32 + 16 * (size_t)K);
+    const size_t needed = (size_t)L * hist_b + (size_t)need * node_b + fixed + later;
+    const size_t spare = free_b > needed ? free_b - needed : 0;
+    ecap = need + (int32_t)std::min<size_t>(15 * (size_t)need, spare / 16 / node_b);
+    pool = L + (int32_t)std::min<size_t>(2 * (size_t)need + 2 * (size_t)bmax, spare / 8 / hist_b);
+  }
+  if (!(s = A.alloc(reinterpret_cast<void**>(&h->hist_all), 8 * cells * (size_t)pool * K)).ok()) return s;
+  for (int k = 0; k < K; ++k) h->slots_h[k].hist = h->hist_all + (size_t)k * pool * cells;
+  if (!h->rounds) return s;
+  // one block for every slot's arrays, each on a 256-byte boundary (an
+  // allocation per array made a many-class learner's creation a third longer)
+  std::vector<std::pair<void**, size_t>> pieces;
+  size_t bytes = 0;
+  auto take = [&](auto*& p, size_t count) {
+    pieces.emplace_back(reinterpret_cast<void**>(&p), bytes);
+    bytes += (count * sizeof(*p) + 255) / 256 * 256;
+  };
+  const size_t nodes = 2 * (size_t)ecap + 1;
+  for (int k = 0; k < K; ++k) {
+    DRounds& r = h->slots_h[k].r;
+    r.ecap = ecap;
+    r.bmax = bmax;
+    r.pool = pool;
+    r.share = share;
+    r.least = least;
+    r.st = reinterpret_cast<RoundState*>(h->rb_dev + (size_t)k * h->rb_slot + h->rb.rs);
+    take(r.node, nodes);
+    take(r.best, nodes);
+    take(r.gain, nodes);
+    take(r.feat, nodes);
+    take(r.exp, nodes);
+    take(r.splittable, nodes * nf);
+    take(r.exp_node, ecap);
+    take(r.item, bmax);
+    take(r.fres, 2 * (size_t)bmax * nf);
+    take(r.scan_cnt, 2 * (size_t)bmax);
+    take(r.cand, pool);
+    take(r.free, pool);
+    take(r.free_next, pool);
+    take(r.leaf_node, L);
+    take(r.pop_node, L);
+    take(r.pop_time, nodes);
+    take(r.node_leaf, nodes);
+    take(r.piece, (size_t)ecap + 1);
+    take(r.piece_num, 2 * (size_t)L);
+    take(r.status, max_tiles + bmax);
+  }
+  if (!(s = A.alloc(reinterpret_cast<void**>(&h->round_block), bytes)).ok()) return s;
+  for (auto& p : pieces) *p.first = h->round_block + p.second;
+  for (int k = 0; k < K; ++k) {
+    CU(cudaMemset(h->slots_h[k].r.st, 0, sizeof(RoundState)));
+    CU(cudaMemset(h->slots_h[k].r.status, 0, (max_tiles + bmax) * sizeof(unsigned long long)));
+  }
+  return s;
+}
+
 static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg, const uint8_t* bins, int64_t n,
                             int32_t nf, const LgbmB200FeatureMeta* metas) {
   h->cfg = *cfg;
@@ -218,35 +308,8 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
   const size_t cells = (size_t)h->total_bins * (mode == LGBM_B200_HIST_QUANT ? 1 : 2);
   const size_t max_tiles = ((size_t)n + kPartTileRows - 1) / kPartTileRows + 1;
   // Growth in rounds, unless a launch strategy that goes step by step is
-  // asked for (data-parallel growth also does, set after this). The explored
-  // tree may hold up to 16 times the splits of the finished one: 1.4 times is
-  // usual, 2 to 3 times on late trees of a run, whose gains hardly fall with
-  // depth. Only the nodes that may still be split hold a histogram, so three
-  // times the splits suffice there, less when that would take more than an
-  // eighth of the free memory (with none to spare, the rounds shrink to the
-  // one node the replay waits for).
+  // asked for (data-parallel growth also does, set after this).
   h->rounds = !cfg->persistent_grow && !h->scan_part;
-  int32_t ecap = 0, bmax = 0, pool = 0, share = 6, least = 16;
-  if (h->rounds) {
-    const int32_t need = L - 1;
-    size_t free_b = 0, total_b = 0;
-    CU(cudaMemGetInfo(&free_b, &total_b));
-    const size_t hist_b = cells * 8 * (size_t)K + 1;
-    const size_t node_b = 2 * (sizeof(RNode) + sizeof(DSplit) + (size_t)nf + 64) * (size_t)K;
-    // A round costs about 50 us however few nodes it expands; an expansion
-    // costs two scans per feature and slot, of which the GPU does about 200 a
-    // microsecond. Many slots and features make a wasted expansion dear:
-    // multiclass K=10 x 200 features 7.7 ms an iteration at a quarter (at least
-    // 24), 6.9 at a sixth (12), 6.5 at a tenth (8); binary x 28 1.24, 1.20 and
-    // 1.4 ms.
-    if (2 * (int64_t)nf * K > 1000) {
-      share = 10;
-      least = 8;
-    }
-    bmax = std::max(1, std::min(kMaxRoundItems, std::max(least, (need + share - 1) / share)));
-    ecap = need + (int32_t)std::min<size_t>(15 * (size_t)need, free_b / 16 / node_b);
-    pool = need + 1 + (int32_t)std::min<size_t>(2 * (size_t)need + 2 * (size_t)bmax, free_b / 8 / hist_b);
-  }
   {
     // the readback block: each slot's state, then its tree arrays, each
     // piece on a 256-byte boundary
@@ -302,11 +365,6 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
     ALLOC(d.splittable, (size_t)L * nf);
     ALLOC(d.cmin, L);
     ALLOC(d.cmax, L);
-    {
-      double* hp;
-      ALLOC(hp, cells * (size_t)std::max(L, pool));
-      d.hist = hp;
-    }
     ALLOC(d.feat_res, 2 * (size_t)nf);
     ALLOC(d.lut_cand, 2 * (size_t)nf * kMaxBins);
     ALLOC(d.leaf_lut, (size_t)L * kMaxBins);
@@ -338,38 +396,6 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
     t.internal_count = reinterpret_cast<int32_t*>(rbk + rb.ic);
     t.cat_bits = reinterpret_cast<uint32_t*>(rbk + rb.cb);
     t.node_gain = reinterpret_cast<double*>(rbk + rb.ng);
-    if (h->rounds) {
-      DRounds& r = d.r;
-      const size_t nodes = 2 * (size_t)ecap + 1;
-      r.ecap = ecap;
-      r.bmax = bmax;
-      r.pool = pool;
-      r.share = share;
-      r.least = least;
-      r.st = reinterpret_cast<RoundState*>(rbk + rb.rs);
-      ALLOC(r.node, nodes);
-      ALLOC(r.best, nodes);
-      ALLOC(r.gain, nodes);
-      ALLOC(r.feat, nodes);
-      ALLOC(r.exp, nodes);
-      ALLOC(r.splittable, nodes * nf);
-      ALLOC(r.exp_node, ecap);
-      ALLOC(r.item, bmax);
-      ALLOC(r.fres, 2 * (size_t)bmax * nf);
-      ALLOC(r.scan_cnt, 2 * (size_t)bmax);
-      ALLOC(r.cand, pool);
-      ALLOC(r.free, pool);
-      ALLOC(r.free_next, pool);
-      ALLOC(r.leaf_node, L);
-      ALLOC(r.pop_node, L);
-      ALLOC(r.pop_time, nodes);
-      ALLOC(r.node_leaf, nodes);
-      ALLOC(r.piece, (size_t)ecap + 1);
-      ALLOC(r.piece_num, 2 * (size_t)L);
-      ALLOC(r.status, max_tiles + bmax);
-      CU(cudaMemset(r.st, 0, sizeof(RoundState)));
-      CU(cudaMemset(r.status, 0, (max_tiles + bmax) * sizeof(unsigned long long)));
-    }
     CU(cudaMemset(d.st, 0, sizeof(DSlotState)));
     CU(cudaMemset(d.tile_status, 0, max_tiles * sizeof(unsigned long long)));
     CU(cudaMemset(d.root_counter, 0, sizeof(int32_t)));
@@ -431,6 +457,7 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
     if (!(s = A.alloc_n(&h->start_dev, (size_t)K)).ok()) return s;
     CU(cudaHostAlloc(reinterpret_cast<void**>(&h->start_h), sizeof(int64_t) * K, cudaHostAllocDefault));
   }
+  if (!(s = alloc_pools(h, cells, max_tiles)).ok()) return s;
   // context
   DCtx& c = h->ctx;
   c.bins = bins_d;
@@ -1431,6 +1458,22 @@ int lgbm_b200_learner_set_data_parallel(LgbmB200Learner* h, int64_t row_offset, 
   if (h->cfg.hist_precision == LGBM_B200_HIST_QUANT && h->cfg.stochastic_rounding &&
       !(s = quant_tables(h, global_num_data)).ok())
     return fail(s);
+  if (h->rounds) {
+    // the steps need no explored tree, and one histogram buffer a leaf (where
+    // there is no room for those beside the larger pool, the pool stays)
+    if (cudaStreamSynchronize(h->stream) != cudaSuccess) return fail(Status(LGBM_B200_ERR_CUDA, "synchronize"));
+    const size_t cells = (size_t)h->total_bins * (h->cfg.hist_precision == LGBM_B200_HIST_QUANT ? 1 : 2);
+    double* hist = nullptr;
+    if (A.alloc_n(&hist, cells * (size_t)L).ok()) {
+      A.release(h->hist_all);
+      d.hist = h->hist_all = hist;
+    } else {
+      cudaGetLastError();
+    }
+    A.release(h->round_block);
+    h->round_block = nullptr;
+    d.r = DRounds{};
+  }
   h->ctx.slots[0] = d;
   h->ctx.dp = 1;
   h->ctx.defer = 0;  // the step's end waits for the left count summed over the ranks

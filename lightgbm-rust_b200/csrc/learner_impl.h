@@ -1,6 +1,7 @@
 // Host-side internals of the learner handle shared by the CUDA translation
 // units (learner.cu, booster.cu).
 #pragma once
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -146,6 +147,12 @@ struct DeviceArena {
   template <class T>
   Status alloc_n(T** p, size_t n) {
     return alloc(reinterpret_cast<void**>(p), n * sizeof(T));
+  }
+  void release(void* p) {  // frees one allocation
+    auto it = std::find(ptrs.begin(), ptrs.end(), p);
+    if (it == ptrs.end()) return;
+    cudaFree(p);
+    ptrs.erase(it);
   }
   void free_all() {
     for (void* p : ptrs) cudaFree(p);
@@ -323,7 +330,9 @@ struct LgbmB200Learner {
   int config_epoch = 0;
   int32_t last_launches = 0;
   int32_t tree_launches = 0;  // of the last enqueue_tree, the rounds aside
+  double* hist_all = nullptr;  // every slot's histogram buffers
   // growth in rounds (round_kernels.cuh)
+  unsigned char* round_block = nullptr;  // every slot's arrays of the explored tree
   bool rounds = false;
   cudaStream_t body_stream = nullptr;  // captures the body of the rounds' loop
   int32_t* round_ctrl = nullptr;       // [3]: slots arrived, slots going on, whether another round runs
