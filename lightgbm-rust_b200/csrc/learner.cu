@@ -618,8 +618,15 @@ static Status enqueue_rounds(LgbmB200Learner* h) {
     CU(e);
     CU(cudaStreamUpdateCaptureDependencies(s, &node, 1, cudaStreamSetCaptureDependencies));
   } else {
+    // LGBM_B200_FAIL_ROUND: the round whose partition is reported as timed out
+    // (tests of the error path; nothing waits)
+    const char* fail_at = std::getenv("LGBM_B200_FAIL_ROUND");
     // every round splits at least one leaf of the final tree
     for (int round = 0; round < h->L; ++round) {
+      if (fail_at && std::atoi(fail_at) == round) {
+        const int32_t status = kStatusTimeout;
+        CU(cudaMemcpyAsync(&h->slots_h[0].st->status, &status, sizeof(status), cudaMemcpyHostToDevice, s));
+      }
       cudaEvent_t* ev = nullptr;
       if (h->timing) {
         while (h->ev.size() < (size_t)4 * (round + 1)) {

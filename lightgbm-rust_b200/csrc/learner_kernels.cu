@@ -2508,7 +2508,7 @@ __device__ int32_t tile_scatter(DSlotState* st, Shared& ps, unsigned long long* 
           const unsigned need = first_inc >= 31 ? 0xffffffffu : ((2u << first_inc) - 1u);
           if (bad_mask & need) {
             if (++spins > kSpinLimit) {  // give up: the prefix 0 keeps every write in the leaf's range;
-              if (lane == 0) st->status = kStatusTimeout;  // the step's end then finishes the tree
+              if (lane == 0) st->status = kStatusTimeout;  // the step's or round's end then finishes the tree
               acc = 0;
               break;
             }

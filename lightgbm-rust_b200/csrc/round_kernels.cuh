@@ -500,7 +500,9 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
     __syncthreads();
     const int32_t popped = s_popped, top = s_top;
     for (int32_t l = tid; l <= popped; l += kDecideThreads) r.leaf_node[l] = ln[l];
-    bool done = top < 0;
+    // a partition whose look-back gave up ends the tree here: its row lists are
+    // incomplete, and the rounds to come would each wait as long again
+    bool done = top < 0 || s.st->status != kStatusOk;
     if (!done && st.rounds > need) {  // every round replays a split: never more rounds than splits
       if (tid == 0) s.st->status = kStatusTimeout;
       done = true;
