@@ -11,7 +11,8 @@ constexpr int kRankMaxQuery = 10000;           // rows per query (size of the di
 // Device view of the objective's tables.
 struct DRank {
   const int32_t* bnd;          // query boundaries [nq + 1]
-  int32_t nq;
+  const int32_t* query;        // the queries with rows: num_large of more than a lane group's rows, then num_small
+  int32_t nq, num_large, num_small;
   const double* inv_max_dcg;   // [nq]
   const double* sigmoid_table; // [kRankSigmoidBins]
   const double* label_gain;    // [31]

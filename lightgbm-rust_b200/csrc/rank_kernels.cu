@@ -30,6 +30,12 @@ constexpr int kRankThreads = 128;
 constexpr int kRankTile = 1024;  // pairs evaluated between two barriers
 constexpr int kRankRows = 256;   // rows of a query whose sorted order stays in shared memory
 constexpr int kRankHold = 4;     // rows ranked at once by a thread of a larger query
+// Queries of so few rows are taken by 8 lanes each: a CTA's barriers and
+// idle threads cost them more than their pairs (an iteration of 800k rows in
+// queries of 2, trees of one split: 1160 us with a CTA each, 205 with these;
+// of 5, 682 and 195; of 10, which keep their CTAs, 498).
+constexpr int kRankSmall = 8;
+constexpr int kRankSmallPerCta = kRankThreads / kRankSmall;
 
 // Monotone map of a score onto uint64: larger score, larger key; -0 and +0
 // are equal, and a NaN orders after every number.
@@ -104,17 +110,16 @@ struct QueryView {
   bool scale_by_score;  // norm and best_score != worst_score (rank.rs:231-233)
 };
 
-// The pair of sorted positions a < b (labels differ, neither score the
-// minimum): its lambda and hessian by the reference's FP64 operations
-// (rank.rs:217-252); a_high: a is the higher-labelled of the two.
-__device__ __forceinline__ void pair_value(const DRank& r, const QueryView& v, int32_t a, int32_t b, bool a_high,
+// The pair of two rows whose labels differ, neither score the minimum: its
+// lambda and hessian by the reference's FP64 operations (rank.rs:217-252), from
+// the higher-labelled row's score and label gain less the other's and the
+// discounts of their places.
+__device__ __forceinline__ void pair_value(const DRank& r, double delta_score, double dcg_gap, double discount_high,
+                                           double discount_low, double inverse_max_dcg, bool scale_by_score,
                                            double& p_lambda, double& p_hessian) {
-  const int32_t high_rank = a_high ? a : b, low_rank = a_high ? b : a;
-  const double delta_score = v.score[high_rank] - v.score[low_rank];
-  const double dcg_gap = v.gain[high_rank] - v.gain[low_rank];
-  const double paired_discount = fabs(r.discount[high_rank] - r.discount[low_rank]);
-  double delta_pair_ndcg = dcg_gap * paired_discount * v.inverse_max_dcg;
-  if (v.scale_by_score) delta_pair_ndcg /= (double)0.01f + fabs(delta_score);
+  const double paired_discount = fabs(discount_high - discount_low);
+  double delta_pair_ndcg = dcg_gap * paired_discount * inverse_max_dcg;
+  if (scale_by_score) delta_pair_ndcg /= (double)0.01f + fabs(delta_score);
   double pl = rank_sigmoid(r, delta_score);
   double ph = pl * (1.0 - pl);
   pl *= -r.sigmoid * delta_pair_ndcg;
@@ -123,8 +128,91 @@ __device__ __forceinline__ void pair_value(const DRank& r, const QueryView& v, i
   p_hessian = ph;
 }
 
-// LambdarankNDCG::one_query (rank.rs:192-262), a CTA per query. Writes g/h
-// (class-major float arrays) or the interleaved pairs.
+// The query of kRankSmall rows at most that the 8 lanes of this thread's group
+// share, a row each (every thread of the warp calls it; cnt 0: no query). The
+// same pairs and sums as k_lambdarank's, passed between the lanes: outer row i's
+// pairs are evaluated side by side, their inner rows take them at once, and
+// the outer row and the FP64 chain add them in order.
+__device__ __forceinline__ void lambdarank_small(const DRank& r, int32_t b0, int32_t cnt, double inverse_max_dcg,
+                                                 const double* score, const float* label, float* g, float* h,
+                                                 float2* gh) {
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int W = kRankSmall;
+  const int l = threadIdx.x & (W - 1);
+  const bool live = l < cnt;
+  const int32_t most = __reduce_max_sync(kAll, cnt);  // of the warp's queries
+  double sc = live ? score[b0 + l] : 0.0;
+  float lab = live ? label[b0 + l] : 0.0f;
+  int32_t at = l;  // the row's place in the stable descending order
+  {
+    const uint64_t key = live ? rank_key(sc) : 0;
+    int32_t rank = 0;
+    for (int j = 0; j < most; ++j) {
+      const uint64_t kj = __shfl_sync(kAll, key, j, W);
+      if (j < cnt) rank += kj >= (j < l ? key : key + 1) ? 1 : 0;
+    }
+    if (live) at = rank;
+  }
+  int32_t row = l;  // the row at this lane's place
+  for (int j = 0; j < most; ++j)
+    if (__shfl_sync(kAll, at, j, W) == l) row = j;
+  sc = __shfl_sync(kAll, sc, row, W);
+  lab = __shfl_sync(kAll, lab, row, W);
+  const double gain = r.label_gain[(int32_t)lab], disc = r.discount[l];
+  int32_t worst = max(cnt - 1, 0);
+  const bool last_min = __shfl_sync(kAll, sc, worst, W) == kMinScoreD;
+  if (worst > 0 && last_min) worst -= 1;
+  const double best_score = __shfl_sync(kAll, sc, 0, W), worst_score = __shfl_sync(kAll, sc, worst, W);
+  const bool scale = r.norm && best_score != worst_score;
+  const int32_t outer = max(0, min(r.truncation_level, cnt - 1));
+  const int32_t most_outer = __reduce_max_sync(kAll, outer);
+  float acc_l = 0.0f, acc_h = 0.0f;
+  double sum_lambdas = 0.0;
+  for (int i = 0; i < most_outer; ++i) {
+    const double si = __shfl_sync(kAll, sc, i, W), gi = __shfl_sync(kAll, gain, i, W), di = __shfl_sync(kAll, disc, i, W);
+    const float li = __shfl_sync(kAll, lab, i, W);
+    const bool pair = i < outer && l > i && live;
+    const bool i_high = li > lab, counts = pair && li != lab && si != kMinScoreD && sc != kMinScoreD;
+    double pl = 0.0, ph = 0.0;
+    if (counts) {
+      const double gap = i_high ? gi - gain : gain - gi;
+      pair_value(r, i_high ? si - sc : sc - si, gap, i_high ? di : disc, i_high ? disc : di, inverse_max_dcg, scale, pl,
+                 ph);
+    }
+    const float vl = i_high ? (float)pl : -(float)pl, vh = (float)ph;
+    if (pair) {
+      acc_l -= vl;
+      acc_h += vh;
+    }
+    for (int j = i + 1; j < most; ++j) {
+      const float ol = __shfl_sync(kAll, vl, j, W), oh = __shfl_sync(kAll, vh, j, W);
+      const double oc = __shfl_sync(kAll, 2.0 * pl, j, W);  // 0 where the pair does not count
+      if (i < outer && j < cnt) {
+        sum_lambdas -= oc;
+        if (l == i) {
+          acc_l += ol;
+          acc_h += oh;
+        }
+      }
+    }
+  }
+  if (r.norm && sum_lambdas > 0.0) {
+    const double norm_factor = log2(1.0 + sum_lambdas) / sum_lambdas;
+    acc_l = (float)((double)acc_l * norm_factor);
+    acc_h = (float)((double)acc_h * norm_factor);
+  }
+  if (!live) return;
+  if (g) {
+    g[b0 + row] = acc_l;
+    h[b0 + row] = acc_h;
+  } else {
+    gh[b0 + row] = make_float2(acc_l, acc_h);
+  }
+}
+
+// LambdarankNDCG::one_query (rank.rs:192-262), a CTA per query of more than
+// kRankSmall rows, and CTAs that take kRankSmallPerCta of the others. Writes
+// g/h (class-major float arrays) or the interleaved pairs.
 //
 // What bounds it: issue slots (2.2 instructions a cycle) and the barriers
 // between the parts, since a pair costs an FP64 divide, index arithmetic and
@@ -149,16 +237,22 @@ __global__ void __launch_bounds__(kRankThreads, 9) k_lambdarank(DRank r, const d
   __shared__ int32_t t_count[kRankTile / 32];
   __shared__ double s_sum;
   const int tid = threadIdx.x, lane = tid & 31;
-  for (int64_t q = blockIdx.x; q < r.nq; q += gridDim.x) {
+  if ((int32_t)blockIdx.x >= r.num_large) {
+    const int32_t x = ((int32_t)blockIdx.x - r.num_large) * kRankSmallPerCta + tid / kRankSmall;
+    const int32_t q = x < r.num_small ? r.query[r.num_large + x] : -1;
+    const int32_t b0 = q >= 0 ? r.bnd[q] : 0, cnt = q >= 0 ? r.bnd[q + 1] - b0 : 0;
+    lambdarank_small(r, b0, cnt, q >= 0 ? r.inv_max_dcg[q] : 0.0, score, label, g, h, gh);
+    return;
+  }
+  {
+    const int32_t q = r.query[blockIdx.x];
     const int32_t b0 = r.bnd[q], cnt = r.bnd[q + 1] - b0;
-    if (cnt == 0) continue;  // uniform over the CTA
     const bool small = cnt <= kRankRows;
     QueryView v;
     v.score = small ? s_score : r.sorted_score + b0;
     v.gain = small ? s_gain : r.sorted_gain + b0;
     v.label = small ? s_label : r.sorted_label + b0;
     v.inverse_max_dcg = r.inv_max_dcg[q];
-    __syncthreads();  // the query before is done with shared memory
     if (small) {
       uint64_t* key = reinterpret_cast<uint64_t*>(t_chain);
       for (int32_t i = tid; i < cnt; i += kRankThreads) key[i] = rank_key(score[b0 + i]);
@@ -205,7 +299,11 @@ __global__ void __launch_bounds__(kRankThreads, 9) k_lambdarank(DRank r, const d
           const float li = v.label[i], lj = v.label[j];
           i_high = li > lj;
           counts = li != lj && v.score[i] != kMinScoreD && v.score[j] != kMinScoreD;
-          if (counts) pair_value(r, v, i, j, i_high, pl, ph);
+          if (counts) {
+            const int32_t high = i_high ? i : j, low = i_high ? j : i;
+            pair_value(r, v.score[high] - v.score[low], v.gain[high] - v.gain[low], r.discount[high], r.discount[low],
+                       v.inverse_max_dcg, v.scale_by_score, pl, ph);
+          }
         }
         t_lambda[t] = i_high ? (float)pl : -(float)pl;
         t_hess[t] = (float)ph;
@@ -277,7 +375,7 @@ __global__ void __launch_bounds__(kRankThreads, 9) k_lambdarank(DRank r, const d
       }
       __syncthreads();  // the sums are written, and the tile is free
     }
-    if (!r.norm) continue;
+    if (!r.norm) return;
     if (tid == 0) s_sum = sum_lambdas;
     __syncthreads();
     sum_lambdas = s_sum;
@@ -395,36 +493,53 @@ Status RankTables::build(const float* label_h, const int32_t* bnd_h, int32_t nq_
     double score = (double)i / idx_factor + min_in;
     table[i] = 1.0 / (1.0 + std::exp(score * sigmoid));
   }
+  // the queries with rows, those of more than kRankSmall first
+  std::vector<int32_t> query;
+  for (int large = 1; large >= 0; --large) {
+    for (int32_t q = 0; q < nq; ++q) {
+      const int32_t rows = bnd_h[q + 1] - bnd_h[q];
+      if (rows > 0 && (rows > kRankSmall) == (large != 0)) query.push_back(q);
+    }
+    if (large) d.num_large = (int32_t)query.size();
+  }
+  d.num_small = (int32_t)query.size() - d.num_large;
+  // one block, each array on a 256-byte boundary
+  size_t bytes = 0;
+  auto take = [&](size_t b) {
+    const size_t o = bytes;
+    bytes += (std::max<size_t>(b, 1) + 255) / 256 * 256;
+    return o;
+  };
+  const size_t rows = (size_t)n;
+  const size_t at_bnd = take(sizeof(int32_t) * ((size_t)nq + 1)), at_query = take(sizeof(int32_t) * query.size()),
+               at_inv = take(sizeof(double) * (size_t)nq), at_table = take(sizeof(double) * table.size()),
+               at_gain = take(sizeof(double) * label_gain.size()), at_disc = take(sizeof(double) * discount.size()),
+               at_sorted = take(sizeof(uint32_t) * rows), at_score = take(sizeof(double) * rows),
+               at_sgain = take(sizeof(double) * rows), at_label = take(sizeof(float) * rows);
   arena.free_all();
-  Status s;
-  int32_t* bnd_d;
-  double *inv_d, *table_d, *gain_d, *disc_d;
-  uint32_t* sorted_d;
-  double* sorted_score_d;
-  double* sorted_gain_d;
-  float* sorted_label_d;
-  const size_t n1 = (size_t)std::max<int64_t>(1, n);
-  if (!(s = arena.alloc_n(&bnd_d, (size_t)nq + 1)).ok() || !(s = arena.alloc_n(&inv_d, std::max<size_t>(1, nq))).ok() ||
-      !(s = arena.alloc_n(&table_d, table.size())).ok() || !(s = arena.alloc_n(&gain_d, label_gain.size())).ok() ||
-      !(s = arena.alloc_n(&disc_d, discount.size())).ok() || !(s = arena.alloc_n(&sorted_d, n1)).ok() ||
-      !(s = arena.alloc_n(&sorted_score_d, n1)).ok() || !(s = arena.alloc_n(&sorted_gain_d, n1)).ok() ||
-      !(s = arena.alloc_n(&sorted_label_d, n1)).ok())
-    return s;
-  CU(cudaMemcpy(bnd_d, bnd_h, sizeof(int32_t) * ((size_t)nq + 1), cudaMemcpyHostToDevice));
-  if (nq > 0) CU(cudaMemcpy(inv_d, inv.data(), sizeof(double) * nq, cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(table_d, table.data(), sizeof(double) * table.size(), cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(gain_d, label_gain.data(), sizeof(double) * label_gain.size(), cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(disc_d, discount.data(), sizeof(double) * discount.size(), cudaMemcpyHostToDevice));
-  d.bnd = bnd_d;
+  unsigned char* block = nullptr;
+  Status s = arena.alloc_n(&block, bytes);
+  if (!s.ok()) return s;
+  auto send = [&](size_t at, const void* src, size_t b) {
+    return b ? cudaMemcpy(block + at, src, b, cudaMemcpyHostToDevice) : cudaSuccess;
+  };
+  CU(send(at_bnd, bnd_h, sizeof(int32_t) * ((size_t)nq + 1)));
+  CU(send(at_query, query.data(), sizeof(int32_t) * query.size()));
+  CU(send(at_inv, inv.data(), sizeof(double) * inv.size()));
+  CU(send(at_table, table.data(), sizeof(double) * table.size()));
+  CU(send(at_gain, label_gain.data(), sizeof(double) * label_gain.size()));
+  CU(send(at_disc, discount.data(), sizeof(double) * discount.size()));
+  d.bnd = reinterpret_cast<const int32_t*>(block + at_bnd);
+  d.query = reinterpret_cast<const int32_t*>(block + at_query);
   d.nq = nq;
-  d.inv_max_dcg = inv_d;
-  d.sigmoid_table = table_d;
-  d.label_gain = gain_d;
-  d.discount = disc_d;
-  d.sorted = sorted_d;
-  d.sorted_score = sorted_score_d;
-  d.sorted_gain = sorted_gain_d;
-  d.sorted_label = sorted_label_d;
+  d.inv_max_dcg = reinterpret_cast<const double*>(block + at_inv);
+  d.sigmoid_table = reinterpret_cast<const double*>(block + at_table);
+  d.label_gain = reinterpret_cast<const double*>(block + at_gain);
+  d.discount = reinterpret_cast<const double*>(block + at_disc);
+  d.sorted = reinterpret_cast<uint32_t*>(block + at_sorted);
+  d.sorted_score = reinterpret_cast<double*>(block + at_score);
+  d.sorted_gain = reinterpret_cast<double*>(block + at_sgain);
+  d.sorted_label = reinterpret_cast<float*>(block + at_label);
   d.sigmoid = sigmoid;
   d.min_in = min_in;
   d.max_in = max_in;
@@ -437,7 +552,9 @@ Status RankTables::build(const float* label_h, const int32_t* bnd_h, int32_t nq_
 Status launch_lambdarank(const DRank& r, const float* label, const double* score, float* g, float* h, float2* gh,
                          cudaStream_t s) {
   if (r.nq == 0) return Status();
-  k_lambdarank<<<(unsigned)r.nq, kRankThreads, 0, s>>>(r, score, label, g, h, gh);
+  const int64_t grid = r.num_large + ((int64_t)r.num_small + kRankSmallPerCta - 1) / kRankSmallPerCta;
+  if (grid == 0) return Status();
+  k_lambdarank<<<(unsigned)grid, kRankThreads, 0, s>>>(r, score, label, g, h, gh);
   CU_LAUNCH();
   return Status();
 }
