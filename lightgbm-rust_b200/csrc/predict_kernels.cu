@@ -28,7 +28,8 @@
 
 namespace lgbm_b200 {
 
-constexpr int kPredictThreads = 128;  // of the wide layout's kernel
+constexpr int kRowThreads = 128;      // rows of a CTA of k_predict_rows
+constexpr int kRowStageCols = 223;    // columns up to which it stages them: 128 x 224 floats are half an SM's memory
 constexpr int kMaxPredictDevices = 64;
 constexpr int kPredictSmem = 224 * 1024;
 
@@ -200,26 +201,70 @@ __global__ void __launch_bounds__(1024) k_predict(const __grid_constant__ DFores
   }
 }
 
-// The wide layout: each thread walks its own row, read from global memory.
-__global__ void __launch_bounds__(kPredictThreads) k_predict_wide(const __grid_constant__ DForest f, const float* X,
-                                                                  int64_t nrow, int32_t ncol, double* out) {
-  const int64_t r = (int64_t)blockIdx.x * kPredictThreads + threadIdx.x;
+// A thread per row that walks one tree after the other, nodes read through
+// L1: the wide layout, and forests with too little work a row for the rounds'
+// barriers and staged trees (launch_predict). kStage: the CTA's rows, one
+// contiguous block of X, are staged in shared memory by row (`stride` floats
+// apart, odd), so that the loads are coalesced.
+template <bool kCompact, bool kStage>
+__global__ void __launch_bounds__(kRowThreads) k_predict_rows(const __grid_constant__ DForest f, const float* X,
+                                                              int64_t nrow, int32_t ncol, int32_t stride, double* out) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  float* xs = reinterpret_cast<float*>(smem);
+  const int64_t r0 = (int64_t)blockIdx.x * kRowThreads, r = r0 + threadIdx.x;
+  if constexpr (kStage) {
+    const int32_t total = (int32_t)min((int64_t)kRowThreads, nrow - r0) * ncol;
+    const float* src = X + r0 * ncol;
+    if ((ncol & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+      for (int32_t i = threadIdx.x; i < total >> 2; i += kRowThreads) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(src) + i);
+        const int32_t row = (i << 2) / ncol, col = (i << 2) - row * ncol;  // the 4 values lie in one row
+        float* d = xs + row * stride + col;
+        d[0] = drop_tiny(v.x);
+        d[1] = drop_tiny(v.y);
+        d[2] = drop_tiny(v.z);
+        d[3] = drop_tiny(v.w);
+      }
+    } else {
+      for (int32_t i = threadIdx.x; i < total; i += kRowThreads) {
+        const int32_t row = i / ncol;
+        xs[row * stride + i - row * ncol] = drop_tiny(__ldg(src + i));
+      }
+    }
+    __syncthreads();
+  }
   if (r >= nrow) return;
-  const float* row = X + r * ncol;
-  const DNodeWide* nodes = static_cast<const DNodeWide*>(f.nodes);
+  const float* row = kStage ? xs + threadIdx.x * stride : X + r * ncol;
+  auto value = [&](int32_t feat) {  // features past the row read 0.0
+    if (feat >= ncol) return 0.0f;
+    if constexpr (kStage) return row[feat];
+    else return drop_tiny(__ldg(row + feat));
+  };
   const int ntpi = f.ntpi;
   for (int k = 0; k < ntpi; ++k) {
     double acc = 0.0;
     for (int32_t t = k; t < f.num_trees; t += ntpi) {
-      const int4 tt = f.tree[t];  // first node, first leaf, num_leaves
-      int32_t node = 0;
-      if (tt.z > 1) {
+      const int4 tt = __ldg(&f.tree[t]);
+      int32_t leaf = 0;
+      if constexpr (kCompact) {
+        const PNode* nodes = static_cast<const PNode*>(f.nodes) + tt.x;
+        uint32_t at = tt.z > 1 ? 0 : 1;  // a constant tree's leaf is at place 1
+        while (tt.z > 1) {
+          const uint2 u = __ldg(reinterpret_cast<const uint2*>(nodes + at));
+          const PNode n{__uint_as_float(u.x), u.y};
+          const uint32_t first = n.meta & 0xffffu;
+          if (first < at) break;  // a leaf: a node's children lie behind it
+          const float v = value((int32_t)(n.meta >> 16) & ((1 << kPNodeFeatureBits) - 1));
+          at = first + (to_first<true>(f, n, v) ? 0u : 1u);
+        }
+        leaf = tt.x + (int32_t)at;
+      } else {
+        const DNodeWide* nodes = static_cast<const DNodeWide*>(f.nodes) + tt.x;
+        int32_t node = tt.z > 1 ? 0 : ~0;
         while (node >= 0) {
-          const DNodeWide n = nodes[tt.x + node];
-          const int32_t feat = n.feat_dt & ((1 << kNodeFeatureBits) - 1);
+          const DNodeWide n = nodes[node];
           const int8_t dt = (int8_t)(n.feat_dt >> kNodeFeatureBits);
-          // features past the row read 0.0
-          double v = feat < ncol ? (double)drop_tiny(row[feat]) : 0.0;
+          double v = (double)value(n.feat_dt & ((1 << kNodeFeatureBits) - 1));
           bool left;
           if (dt & 1) {
             left = category_left(f, (int32_t)__double_as_longlong(n.threshold), (float)v);
@@ -233,9 +278,9 @@ __global__ void __launch_bounds__(kPredictThreads) k_predict_wide(const __grid_c
           }
           node = left ? n.left : n.right;
         }
-        node = ~node;
+        leaf = tt.y + ~node;
       }
-      acc += f.leaf_value[tt.y + node];
+      acc += __ldg(f.leaf_value + leaf);
     }
     out[r * ntpi + k] = acc;
   }
@@ -271,6 +316,8 @@ static cudaError_t predict_device(int* sms) {
       opt((const void*)predict_kernel<2>(i & 1, i & 2, i & 4));
       opt((const void*)predict_kernel<4>(i & 1, i & 2, i & 4));
     }
+    opt((const void*)k_predict_rows<true, true>);
+    opt((const void*)k_predict_rows<false, true>);
     g_predict_err[dev] = x;
   });
   *sms = g_predict_sms[dev];
@@ -279,15 +326,10 @@ static cudaError_t predict_device(int* sms) {
 
 cudaError_t launch_predict(const DForest& f, const float* X, int64_t nrow, int32_t ncol, double* out, cudaStream_t s) {
   if (nrow <= 0) return cudaSuccess;
-  if (!f.compact) {
-    const int64_t blocks = (nrow + kPredictThreads - 1) / kPredictThreads;
-    if (blocks > 0x7fffffff) return cudaErrorInvalidValue;
-    k_predict_wide<<<(unsigned)blocks, kPredictThreads, 0, s>>>(f, X, nrow, ncol, out);
-    return cudaGetLastError();
-  }
   int sms = 148;
   cudaError_t e = predict_device(&sms);
   if (e != cudaSuccess) return e;
+  const int32_t per_class = (f.num_trees + f.ntpi - 1) / f.ntpi;
   // A CTA's threads are R rows times G groups that walk different trees: the
   // rows take the most shared memory, and a walk is a chain of dependent
   // loads, so several warps share a row's staged values. 128 rows where that
@@ -299,7 +341,6 @@ cudaError_t launch_predict(const DForest& f, const float* X, int64_t nrow, int32
   const bool rows = R * col <= 150 * 1024;
   const size_t row_bytes = rows ? R * col : 0;
   const size_t tree = sizeof(PNode) * (size_t)f.max_nodes;
-  const int32_t per_class = (f.num_trees + f.ntpi - 1) / f.ntpi;
   // a round's trees in two buffers, two leaf values per row and tree and two
   // indices per tree, beside the rows
   const size_t left = kPredictSmem - row_bytes;
@@ -321,6 +362,36 @@ cudaError_t launch_predict(const DForest& f, const float* X, int64_t nrow, int32
     G = Gs;
   } else {
     while (G > 1 && bytes(G * walks, false) > left) --G;
+  }
+  // no more groups than the rounds need: 20 trees are two rounds of 5 groups, not of 8
+  const int rounds = std::max(1, (per_class + G * walks - 1) / (G * walks));
+  G = std::max(1, (per_class + rounds * walks - 1) / (rounds * walks));
+  // A thread a row where a row's walks are too short for the rounds' barriers
+  // and staged trees. One tree a class: 1M rows x 28, 31 leaves, 47 us against
+  // 83; ten classes 159 against 294 (few rows the same). Few levels in all, with
+  // rows enough for a wave of CTAs' walks to hide another's loads: three trees of
+  // 31 leaves 65 against 84, six 97 against 100, eight 118 against 102; 12 of 2
+  // leaves 73 against 119; 100k rows, two of 31 leaves 23 against 25, six 31
+  // against 27. Half as many where several classes share the rows' staging: two
+  // trees a class, ten classes, 31 leaves 268 against 309, 255 leaves 372
+  // against 351. Constant trees. Where the trees are too large to stage, both read
+  // them through L1 and rows enough hide it: 1M rows, 20 trees of 30,000 leaves
+  // 577 against 670, 100k rows 131 against 94.
+  int levels = 0;
+  while ((1 << levels) < f.max_nodes) ++levels;
+  const bool by_row = !f.compact || per_class <= 1 || levels <= 1 ||
+                      (nrow >= (int64_t)sms * 512 && per_class * levels * (f.ntpi > 1 ? 2 : 1) <= 24) ||
+                      (nrow >= (int64_t)sms * 2048 && !staged && per_class <= 20);
+  if (by_row) {
+    const int64_t blocks = (nrow + kRowThreads - 1) / kRowThreads;
+    if (blocks > 0x7fffffff) return cudaErrorInvalidValue;
+    const bool stage = ncol <= kRowStageCols;
+    const int32_t stride = ncol | 1;
+    const size_t smem = stage ? sizeof(float) * kRowThreads * (size_t)stride : 0;
+    auto kernel = f.compact ? (stage ? k_predict_rows<true, true> : k_predict_rows<true, false>)
+                            : (stage ? k_predict_rows<false, true> : k_predict_rows<false, false>);
+    kernel<<<(unsigned)blocks, kRowThreads, smem, s>>>(f, X, nrow, ncol, stride, out);
+    return cudaGetLastError();
   }
   const size_t smem = bytes(G * walks, staged) + row_bytes;
   const int64_t blocks = (nrow + R - 1) / R;
