@@ -157,7 +157,7 @@ struct RoundState {
   int32_t root;          // 1: the first round, which only searches the root
   int32_t rounds;        // rounds run
   int32_t npiece;        // row pieces of the leaves that lost their lists (k_round_restore, k_round_order)
-  int32_t disorder;      // 1: some piece is not ascending or descending (k_round_order leaves the pieces as they are)
+  int32_t disorder;      // 1: some piece is not ascending or descending (k_round_check)
   int32_t ncand, nfree;  // lengths of cand and free
   double root_value;     // the root's output
 };
@@ -167,8 +167,9 @@ struct RPiece {
   int32_t begin, count, side;  // in index buffer `side`
   int32_t desc;                // 1: descending rows
   int32_t leaf;
-  int32_t first, num;          // the leaf's pieces
+  int32_t next;                // another piece of the leaf, -1 none
   int32_t leaf_desc;           // 1: the leaf's own list is descending
+  int32_t pad;
 };
 struct DRounds {
   RoundState* st;
@@ -190,7 +191,7 @@ struct DRounds {
   int32_t* pop_time;     // [node] scratch of k_round_emit: split index, -1
   int32_t* node_leaf;    // [node] scratch of k_round_emit: leaf index, -1
   RPiece* piece;         // [ecap + 1]
-  int32_t* piece_num;    // [2][num_leaves] scratch of k_round_emit: each leaf's pieces, and those placed so far
+  int32_t* piece_head;   // [num_leaves]: a leaf's first piece, -1 none
   unsigned long long* status;  // look-back words of a round's row tiles
   int32_t ecap, bmax, pool;
   int32_t share, least;  // a round expands at most 1 / share of the splits to come, but may take `least`

@@ -131,6 +131,7 @@ __global__ void k_round_decide(const __grid_constant__ DCtx c, int32_t* ctrl, cu
                                int32_t use_cond);
 __global__ void k_round_emit(const __grid_constant__ DCtx c);
 __global__ void k_round_restore(const __grid_constant__ DCtx c);
+__global__ void k_round_check(const __grid_constant__ DCtx c);
 __global__ void k_round_order(const __grid_constant__ DCtx c);
 __global__ void k_transpose_bins(const uint8_t* bins, int64_t n, int32_t stride, int32_t nf, uint8_t* colbins);
 __global__ void k_leaf_sums(const __grid_constant__ DCtx c, double* partial, int32_t* rank);

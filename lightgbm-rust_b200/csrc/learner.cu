@@ -125,7 +125,7 @@ static Status alloc_pools(LgbmB200Learner* h, size_t cells, size_t max_tiles) {
     take(r.pop_time, nodes);
     take(r.node_leaf, nodes);
     take(r.piece, (size_t)ecap + 1);
-    take(r.piece_num, 2 * (size_t)L);
+    take(r.piece_head, L);
     take(r.status, max_tiles + bmax);
   }
   if (!(s = A.alloc(reinterpret_cast<void**>(&h->round_block), bytes)).ok()) return s;
@@ -438,7 +438,7 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
     CU(cudaMemcpy(h->n_used_dev, &nn, sizeof(int32_t), cudaMemcpyHostToDevice));
   }
   // leaf renewal: a sum pair per (warp share, leaf) segment and each leaf's rank
-  if (!(s = A.alloc_n(&h->leaf_sums, (size_t)K * (leaf_sum_warps(h) + L) * 2)).ok()) return s;
+  if (!(s = A.alloc_n(&h->leaf_sums, (size_t)K * (leaf_sum_warps(h) + L) * 4)).ok()) return s;
   if (!(s = A.alloc_n(&h->leaf_rank, (size_t)K * (L + 1))).ok()) return s;
   if (!(s = A.alloc_n(&h->leaf_values_dev, (size_t)K * L)).ok()) return s;
   if (cfg->persistent_grow) {
@@ -649,10 +649,6 @@ static Status enqueue_rounds(LgbmB200Learner* h) {
   CU_LAUNCH();
   k_round_restore<<<dim3(std::max(1, 2 * h->num_sms / h->K), 1, h->K), 256, 0, s>>>(h->ctx);
   CU_LAUNCH();
-  if (renews_leaves(h)) {  // the renewal's sums follow the lists' order
-    k_round_order<<<dim3(std::max(1, 2 * h->num_sms / h->K), 1, h->K), 256, 0, s>>>(h->ctx);
-    CU_LAUNCH();
-  }
   return Status();
 }
 
@@ -701,7 +697,7 @@ Status enqueue_tree(LgbmB200Learner* h) {
     CU_LAUNCH();
   }
   // a tree in rounds adds its rounds' launches when it is read back
-  h->tree_launches = 1 + (h->rounds ? 2 + renews_leaves(h) : h->cfg.persistent_grow ? 1 : 2 * (L - 1) + (c.defer ? 1 : 0)) +
+  h->tree_launches = 1 + (h->rounds ? 2 : h->cfg.persistent_grow ? 1 : 2 * (L - 1) + (c.defer ? 1 : 0)) +
                      (renews_leaves(h) ? 2 : 0);
   return Status();
 }
@@ -1404,6 +1400,7 @@ int lgbm_b200_learner_get_partition(LgbmB200Learner* h, int32_t slot, int32_t* l
   if (h->rounds && h->trained) {  // leaves that lost their lists in the lists' order
     DCtx c = h->ctx;
     c.slots[0] = h->ctx.slots[slot];
+    k_round_check<<<2 * h->num_sms, 256, 0, s>>>(c);
     k_round_order<<<2 * h->num_sms, 256, 0, s>>>(c);
     if (cudaGetLastError() != cudaSuccess) return fail(Status(LGBM_B200_ERR_CUDA, "launch"));
   }

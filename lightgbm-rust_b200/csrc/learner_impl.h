@@ -282,7 +282,7 @@ struct LgbmB200Learner {
   int32_t* n_used_dev = nullptr;  // in-bag row count read by k_tree_init
   int32_t n_used = 0;
   bool bagging = false;
-  // leaf renewal scratch: [K][leaf_sum_warps + L][2] segment sums, [K][L + 1] leaf ranks
+  // leaf renewal scratch: [K][leaf_sum_warps + L][4] segment sums, [K][L + 1] leaf ranks
   double* leaf_sums = nullptr;
   int32_t* leaf_rank = nullptr;
   double* leaf_values_dev = nullptr;  // [K][L] for add_leaf_outputs

@@ -2916,19 +2916,46 @@ __device__ __forceinline__ void walk_leaf_positions(const LeafTable& t, Visit vi
   end_leaf(r);
 }
 
-// FP64 (g, h) sums of each leaf's rows for the leaf renewal
-// (learner/mod.rs:736-747), in a fixed order so that a tree's leaf values
-// are the same on every run. Grid (G, 1, slots), 256 threads. Warp w takes
-// the positions [w * per, (w + 1) * per) (per = the positions over the
-// warps, rounded up to 32) and visits the leaves its share meets in
-// position order. For each it sums the share's part of the leaf lane-wise
-// (position q to lane q mod 32, in order) and across lanes by a fixed
-// butterfly, and stores the pair at segment w + rank, where rank is the
-// leaf's place in position order. Along the positions both w and rank only
-// grow and one of them grows at every new segment, so no two segments share
-// an index. Block 0 also records each leaf's rank and the share size for
-// k_leaf_renew, which adds a leaf's segments in warp order.
-// partial: [slots][G * 8 + num_leaves][2]; rank: [slots][num_leaves + 1].
+// A sum that keeps what its additions round off (Knuth's TwoSum) in a second
+// FP64 value: s + e is the exact sum of f32 values that span up to 50 binary
+// orders, whatever the order of the additions.
+struct ExactSum {
+  double s = 0.0, e = 0.0;
+  __device__ __forceinline__ void add(double v) {
+    const double t = s + v, w = t - s;
+    e += (s - (t - w)) + (v - w);
+    s = t;
+  }
+  __device__ __forceinline__ void add(const ExactSum& o) {
+    add(o.s);
+    e += o.e;
+  }
+  __device__ __forceinline__ void over_warp() {
+    for (int o = 16; o > 0; o >>= 1) {
+      ExactSum other;
+      other.s = __shfl_xor_sync(0xffffffffu, s, o);
+      other.e = __shfl_xor_sync(0xffffffffu, e, o);
+      add(other);
+    }
+  }
+  __device__ __forceinline__ double value() const { return isfinite(e) ? s + e : s; }  // an infinite sum has no e
+};
+
+// The (g, h) sums of each leaf's rows for the leaf renewal
+// (learner/mod.rs:736-747), rounded once, so that they depend neither on the
+// order of a leaf's list (which the rounds change where they expand a leaf past
+// the finished tree, as far as the memory free for that goes) nor on the split
+// over warps. (Putting those lists back in order instead, each row by its
+// rank among the pieces, took 3 ms a tree of 500,000 rows and 255 leaves.)
+// Grid (G, 1, slots), 256 threads. Warp w takes the positions
+// [w * per, (w + 1) * per) (per = the positions over the warps, rounded up to
+// 32) and visits the leaves its share meets in position order. It stores the
+// share's part of a leaf at segment w + rank, where rank is the leaf's place
+// in position order. Along the positions both w and rank only grow and one of
+// them grows at every new segment, so no two segments share an index. Block 0
+// also records each leaf's rank and the share size for k_leaf_renew, which
+// adds a leaf's segments.
+// partial: [slots][G * 8 + num_leaves][4]; rank: [slots][num_leaves + 1].
 __global__ void __launch_bounds__(256) k_leaf_sums(const __grid_constant__ DCtx c, double* partial, int32_t* rank) {
   extern __shared__ int32_t lt_smem[];
   const DSlot& s = c.slots[blockIdx.z];
@@ -2945,22 +2972,23 @@ __global__ void __launch_bounds__(256) k_leaf_sums(const __grid_constant__ DCtx 
   }
   const int32_t p0 = min(t.total, gw * per), p1 = min(t.total, p0 + per);
   if (p0 >= p1 || t.n == 0) return;
-  double* base = partial + (size_t)blockIdx.z * (nwarps + c.p.num_leaves) * 2;
+  double2* base = reinterpret_cast<double2*>(partial) + (size_t)blockIdx.z * (nwarps + c.p.num_leaves) * 2;
   int32_t r = leaf_rank_of(t, p0);
   for (int32_t q0 = p0; q0 < p1; ++r) {
     const int32_t end = min(p1, r + 1 < t.n ? t.begin[r + 1] : t.total);
     const uint32_t* idx = s.idx[t.side[r]];
-    double g = 0.0, h = 0.0;
+    ExactSum g, h;
+#pragma unroll 4
     for (int32_t q = q0 + lane; q < end; q += 32) {
       const float2 v = s.gh[idx[q]];
-      g += (double)v.x;
-      h += (double)v.y;
+      g.add((double)v.x);
+      h.add((double)v.y);
     }
-    g = warp_sum_d(g);
-    h = warp_sum_d(h);
+    g.over_warp();
+    h.over_warp();
     if (lane == 0) {
-      base[2 * (gw + r)] = g;
-      base[2 * (gw + r) + 1] = h;
+      base[2 * (gw + r)] = make_double2(g.s, g.e);
+      base[2 * (gw + r) + 1] = make_double2(h.s, h.e);
     }
     q0 = end;
   }
@@ -2968,9 +2996,8 @@ __global__ void __launch_bounds__(256) k_leaf_sums(const __grid_constant__ DCtx 
 
 // Leaf outputs from the segment sums of k_leaf_sums (grid (G, 1, slots), a
 // warp per leaf): a leaf at rank r covering positions [b, e) adds segments
-// w + r for w = b / per ... (e - 1) / per, lane-wise in order and across lanes
-// by a fixed butterfly. (One thread per leaf took 35 us where one leaf held
-// most of 1.1M rows.)
+// w + r for w = b / per ... (e - 1) / per. (One thread per leaf took 35 us
+// where one leaf held most of 1.1M rows.)
 __global__ void __launch_bounds__(256) k_leaf_renew(const __grid_constant__ DCtx c, const double* partial,
                                                     const int32_t* rank, int32_t nwarps, double* totals) {
   const DSlot& s = c.slots[blockIdx.z];
@@ -2978,28 +3005,33 @@ __global__ void __launch_bounds__(256) k_leaf_renew(const __grid_constant__ DCtx
   const int lane = threadIdx.x & 31;
   const int32_t* rk = rank + (size_t)blockIdx.z * (c.p.num_leaves + 1);
   const int32_t per = rk[c.p.num_leaves];
-  const double* base = partial + (size_t)blockIdx.z * (nwarps + c.p.num_leaves) * 2;
+  const double2* base = reinterpret_cast<const double2*>(partial) + (size_t)blockIdx.z * (nwarps + c.p.num_leaves) * 2;
   for (int32_t leaf = (int32_t)(blockIdx.x * 8 + (threadIdx.x >> 5)); leaf < st->num_leaves_cur;
        leaf += (int32_t)gridDim.x * 8) {
     const int32_t cnt = s.leaf_count[leaf];
-    double g = 0.0, h = 0.0;
+    ExactSum g, h;
     if (cnt > 0) {
       const int32_t b = s.leaf_begin[leaf], r = rk[leaf], last = (b + cnt - 1) / per;
 #pragma unroll 4
       for (int32_t w = b / per + lane; w <= last; w += 32) {
-        const double2 v = *reinterpret_cast<const double2*>(base + 2 * (w + r));
-        g += v.x;
-        h += v.y;
+        const double2 x = base[2 * (w + r)], y = base[2 * (w + r) + 1];
+        ExactSum o;
+        o.s = x.x;
+        o.e = x.y;
+        g.add(o);
+        o.s = y.x;
+        o.e = y.y;
+        h.add(o);
       }
     }
-    g = warp_sum_d(g);
-    h = warp_sum_d(h);
+    g.over_warp();
+    h.over_warp();
     if (lane != 0) continue;
     if (totals) {  // data-parallel: this rank's sums, refit after the reduction over ranks
-      totals[((size_t)blockIdx.z * c.p.num_leaves + leaf) * 2] = g;
-      totals[((size_t)blockIdx.z * c.p.num_leaves + leaf) * 2 + 1] = h;
+      totals[((size_t)blockIdx.z * c.p.num_leaves + leaf) * 2] = g.value();
+      totals[((size_t)blockIdx.z * c.p.num_leaves + leaf) * 2 + 1] = h.value();
     } else {
-      s.tree.leaf_value[leaf] = maybe_round_to_zero(refit_leaf_output(g, h, c.p, s.leaf_gcount[leaf]));
+      s.tree.leaf_value[leaf] = maybe_round_to_zero(refit_leaf_output(g.value(), h.value(), c.p, s.leaf_gcount[leaf]));
     }
   }
 }

@@ -689,7 +689,7 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
 // k_round_order.
 __global__ void __launch_bounds__(kDecideThreads) k_round_emit(const __grid_constant__ DCtx c) {
   __shared__ unsigned long long warp_sums[kDecideThreads / 32];
-  __shared__ int32_t s_bad;
+  __shared__ int32_t s_bad, s_pieces;
   const DSlot& s = c.slots[blockIdx.z];
   const DRounds& r = s.r;
   RoundState* rs = r.st;
@@ -701,10 +701,8 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_emit(const __grid_cons
     r.pop_time[v] = -1;
     r.node_leaf[v] = -1;
   }
-  int32_t* piece_num = r.piece_num;
-  int32_t* placed = r.piece_num + c.p.num_leaves;
-  for (int32_t l = tid; l <= P; l += kDecideThreads) piece_num[l] = placed[l] = 0;
-  if (tid == 0) s_bad = 0;
+  for (int32_t l = tid; l <= P; l += kDecideThreads) r.piece_head[l] = -1;
+  if (tid == 0) s_bad = s_pieces = 0;
   __syncthreads();
   for (int32_t i = tid; i < P; i += kDecideThreads) r.pop_time[r.pop_node[i]] = i;
   for (int32_t l = tid; l <= P; l += kDecideThreads) r.node_leaf[r.leaf_node[l]] = l;
@@ -772,40 +770,22 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_emit(const __grid_cons
       t.leaf_depth[l] = nd.depth;
     }
   }
-  // unexpanded nodes under a leaf that lost its list: visit(node, leaf, the leaf's node)
-  auto each_piece = [&](auto visit) {
-    for (int32_t v = tid; v < N; v += kDecideThreads) {
-      if (r.exp[v] >= 0 || r.node_leaf[v] >= 0 || r.node[v].count == 0) continue;
-      int32_t up = r.node[v].parent;
-      while (r.node_leaf[up] < 0) up = r.node[up].parent;
-      const int32_t e = r.exp[up];
-      if (r.exp[2 * e + 1] >= 0 || r.exp[2 * e + 2] >= 0) visit(v, r.node_leaf[up], up);
-    }
-  };
-  each_piece([&](int32_t, int32_t l, int32_t) { atomicAdd(&piece_num[l], 1); });
-  __syncthreads();
-  int32_t pieces = 0;
-  for (int32_t l0 = 0; l0 <= P; l0 += kDecideThreads) {
-    const int32_t l = l0 + tid;
-    const int32_t num = l <= P ? piece_num[l] : 0;
-    unsigned long long tot;
-    const int32_t first = (int32_t)block_prefix<kDecideThreads>((unsigned long long)num, warp_sums, tot);
-    if (l <= P) placed[l] = pieces + first;
-    pieces += (int32_t)tot;
-  }
-  __syncthreads();
-  each_piece([&](int32_t v, int32_t l, int32_t up) {
+  // unexpanded nodes under a leaf that lost its list
+  for (int32_t v = tid; v < N; v += kDecideThreads) {
+    if (r.exp[v] >= 0 || r.node_leaf[v] >= 0) continue;
+    int32_t up = r.node[v].parent;
+    while (r.node_leaf[up] < 0) up = r.node[up].parent;
+    const int32_t e = r.exp[up];
+    const bool lost = r.exp[2 * e + 1] >= 0 || r.exp[2 * e + 2] >= 0;
     const RNode& nd = r.node[v];
-    const int32_t at = atomicAdd(&placed[l], 1);
-    r.piece[at] = RPiece{nd.begin, nd.count, nd.side, nd.desc, l, 0, piece_num[l], r.node[up].desc};
-  });
-  __syncthreads();
-  for (int32_t i = tid; i < pieces; i += kDecideThreads) {
-    const int32_t l = r.piece[i].leaf;
-    r.piece[i].first = placed[l] - piece_num[l];
+    if (lost && nd.count > 0) {
+      const int32_t l = r.node_leaf[up], at = atomicAdd(&s_pieces, 1);
+      r.piece[at] = RPiece{nd.begin, nd.count, nd.side, nd.desc, l, atomicExch(&r.piece_head[l], at), r.node[up].desc, 0};
+    }
   }
+  __syncthreads();
   if (tid == 0) {
-    rs->npiece = pieces;
+    rs->npiece = s_pieces;
     rs->disorder = 0;
     st->num_leaves_cur = P + 1;
     st->num_cat = cats;
@@ -815,33 +795,47 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_emit(const __grid_cons
 }
 
 // The listed row pieces that lie in the leaf's own buffer copied into the
-// other one, at the same positions (every piece owns its positions in both),
-// and every piece's order checked. Grid (G, 1, slots).
+// other one, at the same positions (every piece owns its positions in both).
+// Grid (G, 1, slots).
 __global__ void __launch_bounds__(256) k_round_restore(const __grid_constant__ DCtx c) {
   __shared__ RPiece piece[256];
   const DSlot& s = c.slots[blockIdx.z];
   const int32_t n = s.r.st->npiece;
-  bool disorder = false;
   for (int32_t i0 = 0; i0 < n; i0 += 256) {
     const int32_t m = min(256, n - i0);
     __syncthreads();
-    if ((int)threadIdx.x < m) piece[threadIdx.x] = s.r.piece[i0 + threadIdx.x];
+    if ((int)threadIdx.x < m) {
+      RPiece p = s.r.piece[i0 + threadIdx.x];
+      if (p.side == s.leaf_side[p.leaf]) p.count = 0;
+      piece[threadIdx.x] = p;
+    }
     __syncthreads();
     for (int32_t i = 0; i < m; ++i) {
       const RPiece p = piece[i];
-      const int32_t target = s.leaf_side[p.leaf];
       const uint32_t* from = s.idx[p.side] + p.begin;
-      uint32_t* to = s.idx[target] + p.begin;
+      uint32_t* to = s.idx[1 - p.side] + p.begin;
       // small pieces start at different CTAs
       const uint32_t b = (blockIdx.x + (uint32_t)i * 37u) % gridDim.x;
-      for (uint32_t k = b * 256u + threadIdx.x; k < (uint32_t)p.count; k += gridDim.x * 256u) {
-        const uint32_t row = from[k];
-        if (k + 1 < (uint32_t)p.count) disorder |= (from[k + 1] < row) != (p.desc != 0);
-        if (p.side != target) to[k] = row;
-      }
+      for (uint32_t k = b * 256u + threadIdx.x; k < (uint32_t)p.count; k += gridDim.x * 256u) to[k] = from[k];
     }
   }
-  if (disorder) s.r.st->disorder = 1;
+}
+
+// Whether every listed piece, in the children's buffer (k_round_restore), is
+// ascending or descending as its node's list is: a bag in no order leaves
+// none. Grid (G, 1, slots).
+__global__ void __launch_bounds__(256) k_round_check(const __grid_constant__ DCtx c) {
+  const DSlot& s = c.slots[blockIdx.z];
+  const DRounds& r = s.r;
+  const int32_t n = r.st->npiece;
+  bool disorder = false;
+  for (int32_t i = 0; i < n; ++i) {
+    const RPiece p = r.piece[i];
+    const uint32_t* x = s.idx[1 - r.node[r.leaf_node[p.leaf]].side] + p.begin;
+    for (uint32_t k = blockIdx.x * 256u + threadIdx.x; k + 1 < (uint32_t)p.count; k += gridDim.x * 256u)
+      disorder |= (x[k + 1] < x[k]) != (p.desc != 0);
+  }
+  if (disorder) r.st->disorder = 1;
 }
 
 // Rows of the list x[0, n) below `row`.
@@ -860,29 +854,46 @@ __device__ __forceinline__ int32_t rows_below(const uint32_t* x, int32_t n, bool
 // its right rows', so every list of the tree is ascending or descending and a
 // row's place is its rank among the leaf's pieces, found by bisection. The
 // pieces lie in the children's buffer (k_round_restore); the leaf's own takes
-// the result. Without this, sums in list order (k_leaf_sums) would depend on
-// how far the rounds had expanded a leaf, and so on the memory that was free
-// for the explored nodes. Grid (G, 1, slots); a second run changes nothing.
+// the result. For the partition's readback alone; the lists' other readers
+// take a leaf's rows in any order. Grid (G, 1, slots); a second run changes
+// nothing.
 __global__ void __launch_bounds__(256) k_round_order(const __grid_constant__ DCtx c) {
+  // a chunk of the pieces and their leaves' lists, loaded side by side: one
+  // piece at a time, each cost a chain of four loads (40 us of a 31-leaf tree)
+  __shared__ RPiece piece[256];
+  __shared__ int32_t own[256], begin[256], count[256], head[256];
   const DSlot& s = c.slots[blockIdx.z];
   const DRounds& r = s.r;
   const int32_t n = r.st->npiece;
   if (r.st->disorder) return;
-  for (int32_t i = 0; i < n; ++i) {
-    const RPiece p = r.piece[i];
-    const int32_t own = r.node[r.leaf_node[p.leaf]].side, lb = s.leaf_begin[p.leaf], lc = s.leaf_count[p.leaf];
-    const uint32_t* from = s.idx[1 - own];
-    const uint32_t b = (blockIdx.x + (uint32_t)i * 37u) % gridDim.x;
-    for (uint32_t k = b * 256u + threadIdx.x; k < (uint32_t)p.count; k += gridDim.x * 256u) {
-      const uint32_t row = from[p.begin + k];
-      int32_t rank = p.desc ? p.count - 1 - (int32_t)k : (int32_t)k;
-      for (int32_t q = p.first; q < p.first + p.num; ++q) {
-        if (q == i) continue;
-        const RPiece& o = r.piece[q];
-        rank += rows_below(from + o.begin, o.count, o.desc != 0, row);
-      }
-      s.idx[own][lb + (p.leaf_desc ? lc - 1 - rank : rank)] = row;
+  for (int32_t i0 = 0; i0 < n; i0 += 256) {
+    const int32_t m = min(256, n - i0);
+    __syncthreads();
+    if ((int)threadIdx.x < m) {
+      const RPiece p = r.piece[i0 + threadIdx.x];
+      piece[threadIdx.x] = p;
+      own[threadIdx.x] = r.node[r.leaf_node[p.leaf]].side;
+      begin[threadIdx.x] = s.leaf_begin[p.leaf];
+      count[threadIdx.x] = s.leaf_count[p.leaf];
+      head[threadIdx.x] = r.piece_head[p.leaf];
     }
-    if (i == p.first && b == 0 && threadIdx.x == 0) s.leaf_side[p.leaf] = own;
+    __syncthreads();
+    for (int32_t i = 0; i < m; ++i) {
+      const RPiece p = piece[i];
+      const uint32_t* from = s.idx[1 - own[i]];
+      uint32_t* to = s.idx[own[i]] + begin[i];
+      const uint32_t b = (blockIdx.x + (uint32_t)(i0 + i) * 37u) % gridDim.x;
+      for (uint32_t k = b * 256u + threadIdx.x; k < (uint32_t)p.count; k += gridDim.x * 256u) {
+        const uint32_t row = from[p.begin + k];
+        int32_t rank = p.desc ? p.count - 1 - (int32_t)k : (int32_t)k;
+        for (int32_t q = head[i]; q >= 0;) {
+          const RPiece o = q >= i0 && q < i0 + m ? piece[q - i0] : r.piece[q];
+          if (q != i0 + i) rank += rows_below(from + o.begin, o.count, o.desc != 0, row);
+          q = o.next;
+        }
+        to[p.leaf_desc ? count[i] - 1 - rank : rank] = row;
+      }
+      if (p.next < 0 && b == 0 && threadIdx.x == 0) s.leaf_side[p.leaf] = own[i];  // the leaf's last piece
+    }
   }
 }

@@ -1,10 +1,10 @@
-"""The order of a leaf's rows does not depend on how far the rounds expanded it.
+"""What a leaf gives does not depend on how far the rounds expanded it.
 
-A leaf expanded past the finished tree loses its row list to its descendants'
-and gets it back in the list's own order. Renewed leaf values are FP64 sums in
-that order, so rounds and growth split by split (persistent_grow, whose lists
-are never lost) must give the same bits from gradients that round in every
-order."""
+A leaf expanded past the finished tree loses its row list to its descendants'.
+Renewed leaf values are sums over that list, so rounds and growth split by
+split (persistent_grow, whose lists are never lost) must give the same bits
+from gradients that an FP64 sum rounds in every order; and the partition's
+readback must give the lists in their own order."""
 import numpy as np
 import pytest
 
