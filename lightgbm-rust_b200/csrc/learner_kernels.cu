@@ -1200,20 +1200,20 @@ __device__ __noinline__ bool scan_categorical(Scratch& sm, const DFeature m, con
       used_bin += __popc(mask);
     }
     __syncwarp();
+    // a NaN key (an empty bin without smoothing, NaN gradients) counts as
+    // infinite, so that the ranks are a permutation whatever the keys
     for (int k = lane; k < used_bin; k += 32) {
       int i = sm.tpos[k];
-      sm.key[k] = G(i) / (H(i) + p.cat_smooth);
+      const double v = G(i) / (H(i) + p.cat_smooth);
+      sm.key[k] = isnan(v) ? INFINITY : v;
     }
     __syncwarp();
-    // NaN keys (an empty bin without smoothing, NaN gradients) come after the
-    // numbers, in bin order: the ranks are a permutation whatever the keys
-    auto before = [](double a, double b) { return a < b || (b != b && a == a); };
     for (int k = lane; k < used_bin; k += 32) {
       double kk = sm.key[k];
       int rank = 0;
       for (int j = 0; j < used_bin; ++j) {
         double kj = sm.key[j];
-        if (before(kj, kk) || (j < k && !before(kk, kj))) ++rank;
+        if (kj < kk || (j < k && !(kk < kj) && !(kj < kk))) ++rank;
       }
       sm.sorted[rank] = sm.tpos[k];
     }

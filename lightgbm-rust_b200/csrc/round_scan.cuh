@@ -1,9 +1,9 @@
 // The threshold scans of a growth round: both children of every expanded
 // node, all features, in one launch (included by round_kernels.cuh).
 //
-// A round searches up to 64 nodes x 2 children x features at once, so unlike
-// a single split step it is bound by throughput: what counts is work per
-// warp instruction, not the latency of one scan.
+// A round searches up to 256 nodes (43 of a 255-leaf tree) x 2 children x
+// features at once, so unlike a single split step it is bound by throughput:
+// what counts is work per warp instruction, not the latency of one scan.
 //
 //   quantized   one warp per scan: the views are loaded coalesced, and packed
 //               integer sums are exact in any order (a warp prefix).
@@ -21,17 +21,24 @@
 // FP32's range and a largest gain above 1e-30: a square below FP32's normal
 // numbers is off by up to 2^-150, and over a divisor of 1e-8 or more by 7e-38,
 // which 1e-5 of such a gain covers; the approximate divide returns 0 from a
-// divisor of 2^126 on. Thresholds outside are evaluated in FP64. Parameters
-// that change the gain's formula (L1, max_delta_step, path smoothing, monotone
-// bounds) evaluate all in FP64.
+// divisor of 2^126 on. The least hessian sum of a leaf usually says so for a
+// whole scan (a test of each estimate cost multiclass trees 2%); else the
+// admissible thresholds are tested, and one outside has all evaluated in FP64.
+// Parameters that change the gain's formula (L1, max_delta_step, path
+// smoothing, monotone bounds) evaluate all in FP64.
 #pragma once
 
-// FP32 estimate of the plain gain of a threshold; NaN, which no floor leaves
-// out, where it could be too far off.
+// FP32 estimate of the plain gain of a threshold.
 __device__ __forceinline__ float gain_estimate(float lg, float lh, float rg, float rh, float l2) {
-  const float ld = lh + l2, rd = rh + l2;
-  const bool safe = fminf(ld, rd) >= 1e-8f && fmaxf(ld, rd) <= 1e37f;
-  return safe ? __fdividef(lg * lg, ld) + __fdividef(rg * rg, rd) : NAN;
+  return __fdividef(lg * lg, lh + l2) + __fdividef(rg * rg, rh + l2);
+}
+// Whether the estimates hold for divisors lh + l2 and rh + l2.
+__device__ __forceinline__ bool divisors_safe(float lh, float rh, float l2) {
+  return fminf(lh, rh) + l2 >= 1e-8f && fmaxf(lh, rh) + l2 <= 1e37f;
+}
+// Whether they hold for every admissible threshold of a leaf whose hessians sum up to `total`.
+__device__ __forceinline__ bool scan_safe(const DParams& p, double total) {
+  return p.min_sum_hessian_in_leaf + p.lambda_l2 >= 2e-8 && total + p.lambda_l2 <= 1e36;
 }
 // The estimates from which a threshold is evaluated in FP64, given the
 // largest: all of them when it is outside FP32's comfortable range.
@@ -196,6 +203,54 @@ __device__ __forceinline__ HessRange admissible_hess(const DParams& p, const Lea
   return HessRange{(uint32_t)lo, (uint32_t)(past - 1)};
 }
 
+// The admissible thresholds of a view whose packed sums do not only grow, by
+// the reference's tests one by one: too little on the accumulated side passes
+// over a threshold, on the other side it ends the scan. Bit j of the result is
+// bin 8 lane + j (t_lo .. t_hi except skip_t are visited), bit 8, on lane 0, the
+// extra candidate before them (extra; its sum is base). One warp; out of line
+// for its registers, and the sums formed again, since bagged trees alone come
+// here.
+__device__ __noinline__ uint32_t admissible_one_by_one(const int64_t* view, int32_t t_lo, int32_t t_hi, int32_t skip_t,
+                                                       bool reverse, bool extra, uint64_t base, uint64_t sum, double hs,
+                                                       int32_t num_data, double cnt_factor, int32_t min_data,
+                                                       double min_hess) {
+  const int lane = threadIdx.x & 31;
+  auto visited = [&](int t) { return t >= t_lo && t <= t_hi && t != skip_t; };
+  uint64_t pre = 0;
+  for (int j = 0; j < kPer; ++j)
+    if (visited(lane * kPer + j)) pre += (uint64_t)view[view_at(lane * kPer + j)];
+  uint64_t run = pre;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint64_t other = __shfl_up_sync(0xffffffffu, run, o);
+    if (lane >= o) run += other;
+  }
+  // the sum before this lane's bins in scan order
+  run = reverse ? __shfl_sync(0xffffffffu, run, 31) - run : base + run - pre;
+  uint32_t pend = 0;
+  int32_t brk = reverse ? INT32_MIN : INT32_MAX;
+  auto test = [&](uint64_t a, int32_t t) {
+    const double h = (double)int_hess((int64_t)a);
+    const int32_t ac = round_int(h * cnt_factor);
+    if (ac < min_data || h * hs < min_hess) return false;
+    const bool end = num_data - ac < min_data || (double)int_hess((int64_t)(sum - a)) * hs < min_hess;
+    if (end) brk = reverse ? max(brk, t) : min(brk, t);
+    return !end;
+  };
+  for (int i = 0; i < kPer; ++i) {
+    const int j = reverse ? kPer - 1 - i : i, t = lane * kPer + j;
+    if (!visited(t)) continue;
+    run += (uint64_t)view[view_at(t)];
+    if (test(run, t)) pend |= 1u << j;
+  }
+  if (extra && test(base, -1)) pend |= 1u << kPer;
+  brk = reverse ? __reduce_max_sync(0xffffffffu, brk) : __reduce_min_sync(0xffffffffu, brk);
+  for (int j = 0; j < kPer; ++j) {
+    const int t = lane * kPer + j;
+    if (reverse ? t <= brk : t >= brk) pend &= ~(1u << j);
+  }
+  return pend;
+}
+
 // One direction of the quantized scan (split.rs:995-1190) by one warp, over
 // the view in shared memory (its most frequent bin fixed).
 __device__ __forceinline__ bool scan_direction_packed(const int64_t* view, const DFeature& m, const DParams& p,
@@ -288,36 +343,10 @@ __device__ __forceinline__ bool scan_direction_packed(const int64_t* view, const
       if ((visited >> j & 1) && admissible(q[j])) pend |= 1u << j;
     extra = extra && admissible(base);
   } else {
-    // the reference's tests one by one: too little on the accumulated side
-    // passes over a threshold, on the other side it ends the scan
-    uint32_t stop = 0;
-    auto test = [&](uint64_t a, bool& end) {
-      const double h = (double)int_hess((int64_t)a);
-      const int32_t ac = round_int(h * cnt_factor);
-      if (ac < p.min_data_in_leaf || h * lc.hs < p.min_sum_hessian_in_leaf) return false;
-      end = lc.num_data - ac < p.min_data_in_leaf ||
-            (double)int_hess((int64_t)(sum - a)) * lc.hs < p.min_sum_hessian_in_leaf;
-      return !end;
-    };
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-      bool end = false;
-      if ((visited >> j & 1) && test(q[j], end)) pend |= 1u << j;
-      if (end) stop |= 1u << j;
-    }
-    int32_t brk = reverse ? INT32_MIN : INT32_MAX;
-    if (stop) brk = lane * kPer + (reverse ? 31 - __clz(stop) : __ffs(stop) - 1);
-    if (extra) {
-      bool end = false;
-      extra = test(base, end);
-      if (end) brk = -1;
-    }
-    brk = reverse ? __reduce_max_sync(0xffffffffu, brk) : __reduce_min_sync(0xffffffffu, brk);
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-      const int t = lane * kPer + j;
-      if (reverse ? t <= brk : t >= brk) pend &= ~(1u << j);
-    }
+    pend = admissible_one_by_one(view, t_lo, t_hi, skip_t, reverse, extra, base, sum, lc.hs, lc.num_data, cnt_factor,
+                                 p.min_data_in_leaf, p.min_sum_hessian_in_leaf);
+    extra = pend >> kPer & 1;
+    pend &= (1u << kPer) - 1;
   }
   // their estimates
   float est[kPer];
@@ -329,6 +358,15 @@ __device__ __forceinline__ bool scan_direction_packed(const int64_t* view, const
   }
   if (extra) most = fmaxf(most, estimate(base));
   if (!__any_sync(0xffffffffu, pend != 0 || extra)) return false;
+  if (!scan_safe(p, 4294967296.0 * lc.hs)) {  // a packed hessian is 32 bits, whatever the leaf's sum
+    auto safe = [&](uint64_t a) {
+      return divisors_safe((float)int_hess((int64_t)a) * hsf, (float)int_hess((int64_t)(sum - a)) * hsf, l2f);
+    };
+#pragma unroll
+    for (int j = 0; j < kPer; ++j)
+      if ((pend >> j & 1) && !safe(q[j])) most = INFINITY;  // no floor
+    if (extra && !safe(base)) most = INFINITY;
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
   const float floor = plain ? estimate_floor(most) : -INFINITY;
@@ -810,6 +848,12 @@ __device__ __forceinline__ bool scan_direction_f64(const double* cg, const doubl
   }
   if (extra) most = fmaxf(most, estimate(base_g, base_h));
   if (!__any_sync(0xffffffffu, pend != 0 || extra)) return false;
+  if (!scan_safe(p, lc.sum_h)) {
+#pragma unroll
+    for (int j = 0; j < kPer; ++j)
+      if ((pend >> j & 1) && !divisors_safe((float)b[j], (float)(lc.sum_h - b[j]), l2f)) most = INFINITY;  // no floor
+    if (extra && !divisors_safe((float)base_h, (float)(lc.sum_h - base_h), l2f)) most = INFINITY;
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
   const float floor = plain ? estimate_floor(most) : -INFINITY;
