@@ -15,8 +15,8 @@
 // wasted work (about half as many again on a 255-leaf tree, but of small
 // leaves: 8% more rows) and leaves no trace.
 //
-// On a 255-leaf tree of 500,000 rows this takes 16 rounds instead of 254
-// steps.
+// A 255-leaf tree takes 16 (the first of a run, whose gains fall with depth) to
+// 30 rounds instead of 254 steps.
 //
 // Included by learner_kernels.cu, whose histogram, scan and partition bodies
 // the round kernels share.
@@ -41,7 +41,7 @@ struct RoundPartShared {
 // the item's fresh one) and before_find_best_split (learner/mod.rs:712-731). A child
 // without rows cannot be searched; the tree fails only if the replay splits
 // the parent (k_round_emit).
-__device__ void round_children(const DCtx& c, const DSlot& s, int32_t e, const RItem& it, int32_t nl) {
+__device__ void round_children(const DCtx& c, const DSlot& s, int32_t e, const RItem& it, int32_t nl, bool last_split) {
   const DRounds& r = s.r;
   const DParams& p = c.p;
   const RNode up = r.node[it.node];
@@ -61,6 +61,7 @@ __device__ void round_children(const DCtx& c, const DSlot& s, int32_t e, const R
   bool need = (left_smaller ? nl : nr) > 0;
   if (p.max_depth > 0 && up.depth + 1 >= p.max_depth) need = false;
   else if (nr < p.min_data_in_leaf * 2 && nl < p.min_data_in_leaf * 2) need = false;
+  else if (last_split) need = false;  // the tree's: its children are not searched
   a.need = b.need = need ? 1 : 0;
   a.ls = DLeafSplits{0, nl, info.left_sum_gradient, info.left_sum_hessian, info.left_sum_gh, info.left_output};
   b.ls = DLeafSplits{0, nr, info.right_sum_gradient, info.right_sum_hessian, info.right_sum_gh, info.right_output};
@@ -94,6 +95,7 @@ __global__ void __launch_bounds__(kPartThreads) k_round_part(const __grid_consta
   const int tid = threadIdx.x;
   const int32_t nb = rs->nb, e0 = rs->e0, ntiles = rs->ntiles;
   const uint32_t epoch = rs->epoch;
+  const bool last_split = rs->popped + 2 >= c.p.num_leaves;
   if (nb == 0) return;
   int32_t next = -1;
   if (tid == 0) next = atomicAdd(&rs->ticket, 1);
@@ -154,7 +156,7 @@ __global__ void __launch_bounds__(kPartThreads) k_round_part(const __grid_consta
                                                nleft, out);
     if (tid == 0 && t0 + kPartTileRows >= cnt) {
       atomicAdd(reinterpret_cast<unsigned long long*>(&s.st->part_rows), (unsigned long long)cnt);
-      round_children(c, s, e0 + lo, it, lefts);
+      round_children(c, s, e0 + lo, it, lefts, last_split);
     }
   }
 }
@@ -287,7 +289,7 @@ cudaError_t launch_round_hist(int mode, int ng, dim3 grid, size_t smem, cudaStre
 
 // ---- the decision between rounds ----------------------------------------------------
 
-// Leaves the replay keeps in registers (8 a lane); larger trees use shared memory.
+// Leaves (of trees of more than 256, groups of leaves) the replay keeps in a lane's registers.
 constexpr int kReplaySlots = 8;
 
 // The explored nodes as the replay and the ranking read them, in shared
@@ -315,38 +317,49 @@ __device__ __forceinline__ unsigned long long order_key(double v) {
 // largest gain (then smallest feature, then smallest leaf) is split as long
 // as it has been expanded. ln: the node of each leaf of the replayed tree. Returns the node the replay waits for, or -1 when the
 // tree is finished. Lane l owns leaves l, l + 32, ...; up to 256 leaves their
-// gains stay in registers.
+// gains stay in registers, of larger trees the best of each of 8 groups.
 template <bool kRegs>
 __device__ int32_t replay(const DRounds& r, const NodeFacts& nd, int32_t* ln, int32_t need, int32_t& popped) {
   const int lane = threadIdx.x & 31;
-  unsigned long long own[kReplaySlots];  // order keys of this lane's leaves
-  unsigned long long best = 0;           // the largest, 0: none
-  int32_t bl = INT32_MAX;                // and its leaf
-  auto own_best = [&](int32_t leaves) {
-    best = 0;
-    bl = INT32_MAX;
-    if constexpr (kRegs) {
-#pragma unroll
-      for (int k = 0; k < kReplaySlots; ++k) {
-        const int32_t l = lane + 32 * k;
-        if (l < leaves && (own[k] > best || (own[k] == best && bl != INT32_MAX && better_than(0.0, nd.feat[ln[l]], 0.0, nd.feat[ln[bl]])))) {
-          best = own[k];
-          bl = l;
-        }
-      }
-    } else {
-      for (int32_t l = lane; l < leaves; l += 32) {
-        const unsigned long long k = order_key(nd.gain[ln[l]]);
-        if (k > best || (k == best && bl != INT32_MAX && better_than(0.0, nd.feat[ln[l]], 0.0, nd.feat[ln[bl]]))) {
-          best = k;
-          bl = l;
-        }
+  // kRegs: the order keys of this lane's leaves; else, of each group of `per`
+  // of them, the largest and its leaf (with all of a lane's leaves looked
+  // through at every split an iteration of 200k rows x 28 took 242 ms at 8000
+  // leaves and 45 at 4095; 59 and 18)
+  unsigned long long own[kReplaySlots];
+  int32_t own_leaf[kReplaySlots];
+  unsigned long long best = 0;  // the largest, 0: none
+  int32_t bl = INT32_MAX;       // and its leaf
+  const int32_t per = (need / 32 + kReplaySlots) / kReplaySlots;
+  auto better = [&](unsigned long long k, int32_t l, unsigned long long than, int32_t of) {
+    return k > than || (k == than && of != INT32_MAX && l != INT32_MAX && better_than(0.0, nd.feat[ln[l]], 0.0, nd.feat[ln[of]]));
+  };
+  auto group_best = [&](int32_t g, int32_t leaves, unsigned long long& key, int32_t& leaf) {
+    key = 0;
+    leaf = INT32_MAX;
+    for (int32_t l = lane + 32 * per * g; l < min(leaves, 32 * per * (g + 1)); l += 32) {
+      const unsigned long long k = order_key(nd.gain[ln[l]]);
+      if (better(k, l, key, leaf)) {
+        key = k;
+        leaf = l;
       }
     }
   };
-  if constexpr (kRegs) {
+  auto own_best = [&](int32_t leaves) {
+    best = 0;
+    bl = INT32_MAX;
 #pragma unroll
-    for (int k = 0; k < kReplaySlots; ++k) own[k] = lane + 32 * k <= popped ? order_key(nd.gain[ln[lane + 32 * k]]) : 0ull;
+    for (int k = 0; k < kReplaySlots; ++k) {
+      const int32_t l = kRegs ? lane + 32 * k : own_leaf[k];
+      if ((!kRegs || l < leaves) && better(own[k], l, best, bl)) {
+        best = own[k];
+        bl = l;
+      }
+    }
+  };
+#pragma unroll
+  for (int k = 0; k < kReplaySlots; ++k) {
+    if constexpr (kRegs) own[k] = lane + 32 * k <= popped ? order_key(nd.gain[ln[lane + 32 * k]]) : 0ull;
+    else group_best(k, popped + 1, own[k], own_leaf[k]);
   }
   own_best(popped + 1);
   const unsigned long long zero = order_key(0.0);
@@ -392,6 +405,22 @@ __device__ int32_t replay(const DRounds& r, const NodeFacts& nd, int32_t* ln, in
         if (l == lane + 32 * k) own[k] = ka;
         if (R == lane + 32 * k) own[k] = kb;
       }
+    } else {
+#pragma unroll 1
+      for (int side = 0; side < 2; ++side) {  // the groups of the two leaves
+        const int32_t x = side ? R : l;
+        if (lane != (x & 31)) continue;
+        const int32_t g = (x >> 5) / per;
+        unsigned long long key;
+        int32_t leaf;
+        group_best(g, popped + 1, key, leaf);
+#pragma unroll
+        for (int k = 0; k < kReplaySlots; ++k)
+          if (k == g) {
+            own[k] = key;
+            own_leaf[k] = leaf;
+          }
+      }
     }
     if (lane == (l & 31) || lane == (R & 31)) own_best(popped + 1);
   }
@@ -433,6 +462,7 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
   const int tid = threadIdx.x;
   const int32_t L = c.p.num_leaves, need = L - 1;
   const RoundState st = *rs;
+  const int32_t status = s.st->status;
   int32_t active = 0;
   if (!st.done) {
     const int32_t E = st.e0 + st.nb, N = 2 * E + 1;
@@ -502,14 +532,15 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_decide(const __grid_co
     for (int32_t l = tid; l <= popped; l += kDecideThreads) r.leaf_node[l] = ln[l];
     // a partition whose look-back gave up ends the tree here: its row lists are
     // incomplete, and the rounds to come would each wait as long again
-    bool done = top < 0 || s.st->status != kStatusOk;
+    bool done = top < 0 || status != kStatusOk;
     if (!done && st.rounds > need) {  // every round replays a split: never more rounds than splits
       if (tid == 0) s.st->status = kStatusTimeout;
       done = true;
     }
     if (!done) {
       const int32_t open = need - popped, spare = min(st.nfree, r.ecap - E);
-      const int32_t most = max(1, min(min(r.bmax, spare - open + 1), max(r.least, (open + r.share - 1) / r.share)));
+      // only the node the replay waits for when one split is left to come
+      const int32_t most = open == 1 ? 1 : max(1, min(min(r.bmax, spare - open + 1), max(r.least, (open + r.share - 1) / r.share)));
       // 0: the node cannot be split; positive for every positive gain
       auto key_of = [&](int32_t v) {
         float k = nd.gain[v] > 0.0 ? fmaxf((float)nd.gain[v], 1.4e-45f) : 0.0f;
