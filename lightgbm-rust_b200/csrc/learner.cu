@@ -308,8 +308,21 @@ static Status setup_learner(LgbmB200Learner* h, const LgbmB200LearnerConfig* cfg
   const size_t cells = (size_t)h->total_bins * (mode == LGBM_B200_HIST_QUANT ? 1 : 2);
   const size_t max_tiles = ((size_t)n + kPartTileRows - 1) / kPartTileRows + 1;
   // Growth in rounds, unless a launch strategy that goes step by step is
-  // asked for (data-parallel growth also does, set after this).
-  h->rounds = !cfg->persistent_grow && !h->scan_part;
+  // asked for (data-parallel growth also does, set after this) or the tree
+  // takes few steps: a round is four launches and a decision, a step three
+  // short launches. Microseconds of a boosting iteration, steps and rounds:
+  // 200k x 28 quantized, 8 leaves 268 and 311, 13 leaves 355 and 417, 16 leaves
+  // 397 and 455, 20 leaves 491 and 484, 31 leaves 692 and 551 (3k x 10: 366 and
+  // 417 at 16, 429 and 424 at 20; 2M x 28: 676 and 790 at 20, 911 and 888 at
+  // 31). A step's scans cost more on many features (50k x 300: 532 and 471 at
+  // 13; a train call 311 and 331 at 8, 410 and 379 at 12) and with several slots (two of 50k x 40: 406 and 446
+  // at 10, 470 and 468 at 13; three of 50k x 20: 547 and 598 at 13, 621 and 621
+  // at 16; five: 593 and 631 at 8, 669 and 665 at 10; sixteen of 20k x 20, a
+  // train call: 1322 and 1279 at 2).
+  // The float forms' rounds have the faster histogram (200k x 28, a train call:
+  // 256 and 261 at 2, 534 and 424 at 8) and are never left.
+  const int few = h->K == 1 ? (nf <= 150 ? 18 : 10) : h->K <= 3 ? 12 : h->K <= 5 ? 8 : 0;
+  h->rounds = !cfg->persistent_grow && !h->scan_part && (mode != LGBM_B200_HIST_QUANT || L > few);
   {
     // the readback block: each slot's state, then its tree arrays, each
     // piece on a 256-byte boundary
@@ -652,6 +665,24 @@ static Status enqueue_rounds(LgbmB200Learner* h) {
   return Status();
 }
 
+// The threshold scans of a split step.
+static Status launch_scan(LgbmB200Learner* h) {
+  const DCtx& c = h->ctx;
+  const dim3 g(h->nf, 2, h->K);
+  cudaStream_t s = h->stream;
+  if (h->cfg.hist_precision == LGBM_B200_HIST_QUANT) {
+    if (h->scan_wide)
+      k_scan_warp<<<dim3(std::min(2 * h->nf, h->scan_warp_grid), 1, h->K), kScanThreads, h->scan_warp_smem, s>>>(c);
+    else k_scan<true, 1><<<g, kScanThreads, h->scan_smem, s>>>(c);
+  } else if (h->scan_wide) {
+    k_scan<false, kScanWideBlocks><<<g, kScanThreads, h->scan_smem, s>>>(c);
+  } else {
+    k_scan<false, 1><<<g, kScanThreads, h->scan_smem, s>>>(c);
+  }
+  CU_LAUNCH();
+  return Status();
+}
+
 // Enqueue one whole tree (every slot) on the stream: init, its growth and
 // leaf renewal.
 Status enqueue_tree(LgbmB200Learner* h) {
@@ -670,20 +701,31 @@ Status enqueue_tree(LgbmB200Learner* h) {
     if (h->timing) CU(cudaMemsetAsync(h->phase_ns, 0, 4 * sizeof(long long), s));
     CU(launch_grow(mode, h->hist_ng, h->grow_grid, h->grow_smem, s, c, h->tiles, h->sub_rows, h->ntiles,
                    h->grow_sync, L - 1, h->timing ? h->phase_ns : nullptr));
-  } else {  // step by step, the scans and the partition of a step in one launch
+  } else {  // step by step
     const dim3 hist_grid(step_hist_grid(h), h->ntiles, K);
-    const dim3 g(h->scan_part_grid, 1, K);
+    // in a captured graph the events are recorded at every replay, and are no edges of it
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CU(cudaStreamIsCapturing(s, &cs));
+    const unsigned flag = cs == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault;
     for (int step = 0; step < L - 1; ++step) {
       cudaEvent_t* ev = h->timing ? &h->ev[(size_t)4 * step] : nullptr;
-      if (ev) CU(cudaEventRecordWithFlags(ev[0], s, cudaEventRecordExternal));
+      if (ev) CU(cudaEventRecordWithFlags(ev[0], s, flag));
       CU(launch_hist(mode, h->hist_ng, hist_grid, h->hist_smem, s, c, h->tiles, h->sub_rows, c.defer && step > 0));
-      if (ev) CU(cudaEventRecordWithFlags(ev[1], s, cudaEventRecordExternal));
-      // the scan interval records as empty
-      if (ev) CU(cudaEventRecordWithFlags(ev[2], s, cudaEventRecordExternal));
-      if (mode == LGBM_B200_HIST_QUANT)
-        CU(launch_coop(k_scan_partition<true>, g, dim3(kPartThreads), h->scan_smem, s, c));
-      else CU(launch_coop(k_scan_partition<false>, g, dim3(kPartThreads), h->scan_smem, s, c));
-      if (ev) CU(cudaEventRecordWithFlags(ev[3], s, cudaEventRecordExternal));
+      if (ev) CU(cudaEventRecordWithFlags(ev[1], s, flag));
+      if (h->scan_part) {  // scans and partition in one launch: the scan interval records as empty
+        if (ev) CU(cudaEventRecordWithFlags(ev[2], s, flag));
+        const dim3 g(h->scan_part_grid, 1, K);
+        if (mode == LGBM_B200_HIST_QUANT)
+          CU(launch_coop(k_scan_partition<true>, g, dim3(kPartThreads), h->scan_smem, s, c));
+        else CU(launch_coop(k_scan_partition<false>, g, dim3(kPartThreads), h->scan_smem, s, c));
+      } else {
+        Status st = launch_scan(h);
+        if (!st.ok()) return st;
+        if (ev) CU(cudaEventRecordWithFlags(ev[2], s, flag));
+        k_partition<<<dim3(h->part_grid, 1, K), kPartThreads, 0, s>>>(c);
+        CU_LAUNCH();
+      }
+      if (ev) CU(cudaEventRecordWithFlags(ev[3], s, flag));
     }
     if (c.defer) {  // the last split step's end (the earlier ones ran beside the histograms)
       k_finish<<<dim3(1, 1, K), kPartThreads, 0, s>>>(c);
@@ -697,8 +739,8 @@ Status enqueue_tree(LgbmB200Learner* h) {
     CU_LAUNCH();
   }
   // a tree in rounds adds its rounds' launches when it is read back
-  h->tree_launches = 1 + (h->rounds ? 2 : h->cfg.persistent_grow ? 1 : 2 * (L - 1) + (c.defer ? 1 : 0)) +
-                     (renews_leaves(h) ? 2 : 0);
+  const int steps = (h->scan_part ? 2 : 3) * (L - 1) + (c.defer ? 1 : 0);
+  h->tree_launches = 1 + (h->rounds ? 2 : h->cfg.persistent_grow ? 1 : steps) + (renews_leaves(h) ? 2 : 0);
   return Status();
 }
 
@@ -708,23 +750,6 @@ Status dp_allreduce(LgbmB200Learner* h, void* buf, int64_t count, int32_t dtype,
   CU(cudaStreamSynchronize(h->stream));
   const int32_t rc = h->dp_fn(buf, count, dtype, op, h->dp_user);
   if (rc != 0) return Status(LGBM_B200_ERR_INTERNAL, "data-parallel all-reduce failed with " + std::to_string(rc));
-  return Status();
-}
-
-static Status launch_scan(LgbmB200Learner* h) {
-  const DCtx& c = h->ctx;
-  const dim3 g(h->nf, 2, h->K);
-  cudaStream_t s = h->stream;
-  if (h->cfg.hist_precision == LGBM_B200_HIST_QUANT) {
-    if (h->scan_wide)
-      k_scan_warp<<<dim3(std::min(2 * h->nf, h->scan_warp_grid), 1, h->K), kScanThreads, h->scan_warp_smem, s>>>(c);
-    else k_scan<true, 1><<<g, kScanThreads, h->scan_smem, s>>>(c);
-  } else if (h->scan_wide) {
-    k_scan<false, kScanWideBlocks><<<g, kScanThreads, h->scan_smem, s>>>(c);
-  } else {
-    k_scan<false, 1><<<g, kScanThreads, h->scan_smem, s>>>(c);
-  }
-  CU_LAUNCH();
   return Status();
 }
 
