@@ -168,8 +168,7 @@ struct RPiece {
   int32_t desc;                // 1: descending rows
   int32_t leaf;
   int32_t next;                // another piece of the leaf, -1 none
-  int32_t leaf_desc;           // 1: the leaf's own list is descending
-  int32_t pad;
+  int32_t leaf_desc, own;      // the leaf's own list: 1 descending; its index buffer
 };
 struct DRounds {
   RoundState* st;

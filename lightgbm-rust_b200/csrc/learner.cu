@@ -735,7 +735,7 @@ Status enqueue_tree(LgbmB200Learner* h) {
   if (renews_leaves(h)) {
     k_leaf_sums<<<dim3(leaf_sum_warps(h) / 8, 1, K), 256, 16 * (size_t)L, s>>>(c, h->leaf_sums, h->leaf_rank);
     CU_LAUNCH();
-    k_leaf_renew<<<dim3((L + 7) / 8, 1, K), 256, 0, s>>>(c, h->leaf_sums, h->leaf_rank, leaf_sum_warps(h), nullptr);
+    k_leaf_renew<<<dim3(std::min(L, 2048), 1, K), 256, 0, s>>>(c, h->leaf_sums, h->leaf_rank, leaf_sum_warps(h), nullptr);
     CU_LAUNCH();
   }
   // a tree in rounds adds its rounds' launches when it is read back
@@ -799,7 +799,7 @@ static Status run_tree_dp(LgbmB200Learner* h) {
   if (mode == LGBM_B200_HIST_QUANT && h->cfg.quant_train_renew_leaf) {
     k_leaf_sums<<<dim3(leaf_sum_warps(h) / 8, 1, 1), 256, 16 * (size_t)L, s>>>(c, h->leaf_sums, h->leaf_rank);
     CU_LAUNCH();
-    k_leaf_renew<<<(L + 7) / 8, 256, 0, s>>>(c, h->leaf_sums, h->leaf_rank, leaf_sum_warps(h), h->dp_f64);
+    k_leaf_renew<<<std::min(L, 2048), 256, 0, s>>>(c, h->leaf_sums, h->leaf_rank, leaf_sum_warps(h), h->dp_f64);
     CU_LAUNCH();
     if (!(st = dp_allreduce(h, h->dp_f64, 2 * (int64_t)L, LGBM_B200_DT_FLOAT64, LGBM_B200_OP_SUM)).ok()) return st;
     k_dp_leaf_apply<<<1, 256, 0, s>>>(c, h->dp_f64);

@@ -2941,6 +2941,8 @@ struct ExactSum {
   __device__ __forceinline__ double value() const { return isfinite(e) ? s + e : s; }  // an infinite sum has no e
 };
 
+constexpr int kSumAhead = 4;  // values a lane loads before it adds them
+
 // The (g, h) sums of each leaf's rows for the leaf renewal
 // (learner/mod.rs:736-747), rounded once, so that they depend neither on the
 // order of a leaf's list (which the rounds change where they expand a leaf past
@@ -2978,11 +2980,15 @@ __global__ void __launch_bounds__(256) k_leaf_sums(const __grid_constant__ DCtx 
     const int32_t end = min(p1, r + 1 < t.n ? t.begin[r + 1] : t.total);
     const uint32_t* idx = s.idx[t.side[r]];
     ExactSum g, h;
-#pragma unroll 4
-    for (int32_t q = q0 + lane; q < end; q += 32) {
-      const float2 v = s.gh[idx[q]];
-      g.add((double)v.x);
-      h.add((double)v.y);
+    for (int32_t q = q0 + lane; q < end; q += 32 * kSumAhead) {
+      float2 v[kSumAhead];
+#pragma unroll
+      for (int u = 0; u < kSumAhead; ++u) v[u] = q + 32 * u < end ? s.gh[idx[q + 32 * u]] : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < kSumAhead; ++u) {
+        g.add((double)v[u].x);
+        h.add((double)v[u].y);
+      }
     }
     g.over_warp();
     h.over_warp();
@@ -2994,39 +3000,55 @@ __global__ void __launch_bounds__(256) k_leaf_sums(const __grid_constant__ DCtx 
   }
 }
 
-// Leaf outputs from the segment sums of k_leaf_sums (grid (G, 1, slots), a
-// warp per leaf): a leaf at rank r covering positions [b, e) adds segments
-// w + r for w = b / per ... (e - 1) / per. (One thread per leaf took 35 us
-// where one leaf held most of 1.1M rows.)
+// Leaf outputs from the segment sums of k_leaf_sums (grid (G, 1, slots), 256
+// threads, a CTA per leaf): a leaf at rank r covering positions [b, e) adds
+// segments w + r for w = b / per ... (e - 1) / per. (Where one leaf holds most
+// of 500,000 rows, a warp per leaf took 20 us for the loads of its 3900
+// segments.)
 __global__ void __launch_bounds__(256) k_leaf_renew(const __grid_constant__ DCtx c, const double* partial,
                                                     const int32_t* rank, int32_t nwarps, double* totals) {
+  __shared__ double part[8][4];  // each warp's (g, h) sums
   const DSlot& s = c.slots[blockIdx.z];
   DSlotState* st = s.st;
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int32_t* rk = rank + (size_t)blockIdx.z * (c.p.num_leaves + 1);
   const int32_t per = rk[c.p.num_leaves];
   const double2* base = reinterpret_cast<const double2*>(partial) + (size_t)blockIdx.z * (nwarps + c.p.num_leaves) * 2;
-  for (int32_t leaf = (int32_t)(blockIdx.x * 8 + (threadIdx.x >> 5)); leaf < st->num_leaves_cur;
-       leaf += (int32_t)gridDim.x * 8) {
+  for (int32_t leaf = (int32_t)blockIdx.x; leaf < st->num_leaves_cur; leaf += (int32_t)gridDim.x) {
     const int32_t cnt = s.leaf_count[leaf];
     ExactSum g, h;
     if (cnt > 0) {
       const int32_t b = s.leaf_begin[leaf], r = rk[leaf], last = (b + cnt - 1) / per;
-#pragma unroll 4
-      for (int32_t w = b / per + lane; w <= last; w += 32) {
-        const double2 x = base[2 * (w + r)], y = base[2 * (w + r) + 1];
-        ExactSum o;
-        o.s = x.x;
-        o.e = x.y;
-        g.add(o);
-        o.s = y.x;
-        o.e = y.y;
-        h.add(o);
+      for (int32_t w = b / per + (int32_t)threadIdx.x; w <= last; w += 256 * kSumAhead) {
+        double2 x[kSumAhead], y[kSumAhead];
+#pragma unroll
+        for (int u = 0; u < kSumAhead; ++u) {
+          const bool in = w + 256 * u <= last;
+          x[u] = in ? base[2 * (w + 256 * u + r)] : make_double2(0.0, 0.0);
+          y[u] = in ? base[2 * (w + 256 * u + r) + 1] : make_double2(0.0, 0.0);
+        }
+#pragma unroll
+        for (int u = 0; u < kSumAhead; ++u) {
+          g.add(ExactSum{x[u].x, x[u].y});
+          h.add(ExactSum{y[u].x, y[u].y});
+        }
       }
     }
     g.over_warp();
     h.over_warp();
-    if (lane != 0) continue;
+    __syncthreads();  // the leaf before is done with `part`
+    if (lane == 0) {
+      part[warp][0] = g.s;
+      part[warp][1] = g.e;
+      part[warp][2] = h.s;
+      part[warp][3] = h.e;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) continue;
+    for (int w = 1; w < 8; ++w) {
+      g.add(ExactSum{part[w][0], part[w][1]});
+      h.add(ExactSum{part[w][2], part[w][3]});
+    }
     if (totals) {  // data-parallel: this rank's sums, refit after the reduction over ranks
       totals[((size_t)blockIdx.z * c.p.num_leaves + leaf) * 2] = g.value();
       totals[((size_t)blockIdx.z * c.p.num_leaves + leaf) * 2 + 1] = h.value();

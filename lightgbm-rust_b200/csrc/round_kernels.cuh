@@ -811,7 +811,7 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_emit(const __grid_cons
     const RNode& nd = r.node[v];
     if (lost && nd.count > 0) {
       const int32_t l = r.node_leaf[up], at = atomicAdd(&s_pieces, 1);
-      r.piece[at] = RPiece{nd.begin, nd.count, nd.side, nd.desc, l, atomicExch(&r.piece_head[l], at), r.node[up].desc, 0};
+      r.piece[at] = RPiece{nd.begin, nd.count, nd.side, nd.desc, l, atomicExch(&r.piece_head[l], at), r.node[up].desc, r.node[up].side};
     }
   }
   __syncthreads();
@@ -829,25 +829,27 @@ __global__ void __launch_bounds__(kDecideThreads) k_round_emit(const __grid_cons
 // other one, at the same positions (every piece owns its positions in both).
 // Grid (G, 1, slots).
 __global__ void __launch_bounds__(256) k_round_restore(const __grid_constant__ DCtx c) {
-  __shared__ RPiece piece[256];
+  __shared__ int4 piece[256];  // begin, count, side and index of those that move
+  __shared__ int32_t s_moves;
   const DSlot& s = c.slots[blockIdx.z];
   const int32_t n = s.r.st->npiece;
   for (int32_t i0 = 0; i0 < n; i0 += 256) {
-    const int32_t m = min(256, n - i0);
     __syncthreads();
-    if ((int)threadIdx.x < m) {
-      RPiece p = s.r.piece[i0 + threadIdx.x];
-      if (p.side == s.leaf_side[p.leaf]) p.count = 0;
-      piece[threadIdx.x] = p;
+    if (threadIdx.x == 0) s_moves = 0;
+    __syncthreads();
+    if (i0 + (int)threadIdx.x < n) {
+      const RPiece p = s.r.piece[i0 + threadIdx.x];
+      if (p.side == p.own) piece[atomicAdd(&s_moves, 1)] = make_int4(p.begin, p.count, p.side, i0 + (int)threadIdx.x);
     }
     __syncthreads();
+    const int32_t m = s_moves;
     for (int32_t i = 0; i < m; ++i) {
-      const RPiece p = piece[i];
-      const uint32_t* from = s.idx[p.side] + p.begin;
-      uint32_t* to = s.idx[1 - p.side] + p.begin;
+      const int4 p = piece[i];
+      const uint32_t* from = s.idx[p.z] + p.x;
+      uint32_t* to = s.idx[1 - p.z] + p.x;
       // small pieces start at different CTAs
-      const uint32_t b = (blockIdx.x + (uint32_t)i * 37u) % gridDim.x;
-      for (uint32_t k = b * 256u + threadIdx.x; k < (uint32_t)p.count; k += gridDim.x * 256u) to[k] = from[k];
+      const uint32_t b = (blockIdx.x + (uint32_t)p.w * 37u) % gridDim.x;
+      for (uint32_t k = b * 256u + threadIdx.x; k < (uint32_t)p.y; k += gridDim.x * 256u) to[k] = from[k];
     }
   }
 }
@@ -862,7 +864,7 @@ __global__ void __launch_bounds__(256) k_round_check(const __grid_constant__ DCt
   bool disorder = false;
   for (int32_t i = 0; i < n; ++i) {
     const RPiece p = r.piece[i];
-    const uint32_t* x = s.idx[1 - r.node[r.leaf_node[p.leaf]].side] + p.begin;
+    const uint32_t* x = s.idx[1 - p.own] + p.begin;
     for (uint32_t k = blockIdx.x * 256u + threadIdx.x; k + 1 < (uint32_t)p.count; k += gridDim.x * 256u)
       disorder |= (x[k + 1] < x[k]) != (p.desc != 0);
   }
@@ -892,7 +894,7 @@ __global__ void __launch_bounds__(256) k_round_order(const __grid_constant__ DCt
   // a chunk of the pieces and their leaves' lists, loaded side by side: one
   // piece at a time, each cost a chain of four loads (40 us of a 31-leaf tree)
   __shared__ RPiece piece[256];
-  __shared__ int32_t own[256], begin[256], count[256], head[256];
+  __shared__ int32_t begin[256], count[256], head[256];
   const DSlot& s = c.slots[blockIdx.z];
   const DRounds& r = s.r;
   const int32_t n = r.st->npiece;
@@ -903,7 +905,6 @@ __global__ void __launch_bounds__(256) k_round_order(const __grid_constant__ DCt
     if ((int)threadIdx.x < m) {
       const RPiece p = r.piece[i0 + threadIdx.x];
       piece[threadIdx.x] = p;
-      own[threadIdx.x] = r.node[r.leaf_node[p.leaf]].side;
       begin[threadIdx.x] = s.leaf_begin[p.leaf];
       count[threadIdx.x] = s.leaf_count[p.leaf];
       head[threadIdx.x] = r.piece_head[p.leaf];
@@ -911,8 +912,8 @@ __global__ void __launch_bounds__(256) k_round_order(const __grid_constant__ DCt
     __syncthreads();
     for (int32_t i = 0; i < m; ++i) {
       const RPiece p = piece[i];
-      const uint32_t* from = s.idx[1 - own[i]];
-      uint32_t* to = s.idx[own[i]] + begin[i];
+      const uint32_t* from = s.idx[1 - p.own];
+      uint32_t* to = s.idx[p.own] + begin[i];
       const uint32_t b = (blockIdx.x + (uint32_t)(i0 + i) * 37u) % gridDim.x;
       for (uint32_t k = b * 256u + threadIdx.x; k < (uint32_t)p.count; k += gridDim.x * 256u) {
         const uint32_t row = from[p.begin + k];
@@ -924,7 +925,7 @@ __global__ void __launch_bounds__(256) k_round_order(const __grid_constant__ DCt
         }
         to[p.leaf_desc ? count[i] - 1 - rank : rank] = row;
       }
-      if (p.next < 0 && b == 0 && threadIdx.x == 0) s.leaf_side[p.leaf] = own[i];  // the leaf's last piece
+      if (p.next < 0 && b == 0 && threadIdx.x == 0) s.leaf_side[p.leaf] = p.own;  // the leaf's last piece
     }
   }
 }
