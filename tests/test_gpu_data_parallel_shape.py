@@ -55,3 +55,27 @@ def test_scans_by_warp_grow_the_same_trees(lgb, f):
         for name in ("num_leaves", "split_feature", "threshold_in_bin", "decision_type", "leaf_count", "leaf_value",
                      "split_gain_f64", "cat_threshold"):
             assert np.array_equal(a[name], b[name]), name
+
+
+@pytest.mark.parametrize("form", ["quantized", "f64", "f32c"])
+def test_wide_scans_grow_the_same_trees(lgb, monkeypatch, form):
+    """Both scans of a split step (LGBM_B200_SCAN_WIDE: the 256-thread scan with
+    one CTA an SM; the register-capped one, or, quantized, a warp a scan), which
+    data-parallel growth alone launches, on numerical and categorical features
+    with missing values, and the rounds' scan."""
+    ds, params, y, rng = _case(lgb, form, 20, 3)
+    learners = [lgb.Learner(ds, params)]
+    for wide in "01":
+        monkeypatch.setenv("LGBM_B200_SCAN_WIDE", wide)
+        learners.append(_parallel(lgb.Learner(ds, params), len(y)))
+    categorical = False
+    for it in range(2):
+        # on a grid, so that FP64 sums are exact in any order
+        g = np.round((0.5 - y + 0.3 * rng.standard_normal(len(y))) * 1024).astype(np.float32) / 1024
+        h = np.round((0.1 + 0.2 * rng.random(len(y))) * 1024).astype(np.float32) / 1024
+        rounds, narrow, wide = (learner.train(g, h)[0] for learner in learners)
+        for name in ("num_leaves", "split_feature", "threshold_in_bin", "decision_type", "leaf_count", "cat_threshold"):
+            assert np.array_equal(narrow[name], wide[name]), name
+            assert np.array_equal(narrow[name], rounds[name]), name
+        categorical |= bool((np.asarray(narrow["decision_type"]) & 1).any())
+    assert categorical
