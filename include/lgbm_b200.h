@@ -283,9 +283,10 @@ int lgbm_b200_learner_set_data_parallel(LgbmB200Learner* h, int64_t row_offset, 
                                         LgbmB200AllReduceFn fn, void* user);
 
 /* Launch shape of the growth kernels (the default launch strategy;
- * the persistent one has none). A round of the default growth divides
- * its rows evenly over the histogram's CTAs; hist_rows_per_block counts where
- * trees grow split by split. No field changes a result: the shapes differ
+ * the persistent one has none). hist_rows_per_block is the least number of
+ * rows a histogram CTA takes, which sets how many CTAs a launch's rows spread
+ * over; in a round of the default growth every child whose histogram is built
+ * counts 512 rows more, for its cells. No field changes a result: the shapes differ
  * only in speed. No counterpart in the reference, whose CPU learner has a
  * thread count instead. */
 typedef struct {

@@ -69,7 +69,9 @@ static Status alloc_pools(LgbmB200Learner* h, size_t cells, size_t max_tiles) {
     // microsecond. Many slots and features make a wasted expansion dear:
     // multiclass K=10 x 200 features 7.7 ms an iteration at a quarter (at least
     // 24), 6.9 at a sixth (12), 6.5 at a tenth (8); binary x 28 1.24, 1.20 and
-    // 1.4 ms.
+    // 1.4 ms. A sixth and a tenth meet between 600 scans an expansion (100k rows
+    // x 300, a train call: quantized 1.89 and 1.97 ms, FP64 3.18 and 3.25) and
+    // 1400 (x 700: 3.36 and 3.24, 6.72 and 5.90; K=10 x 70 4.37 and 4.37).
     if (2 * (int64_t)nf * K > 1000) {
       share = 10;
       least = 8;
