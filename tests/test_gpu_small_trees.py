@@ -57,3 +57,40 @@ def test_few_leaves(lgb, f, k, few, graph):
         one.train(g, h)
         if leaves <= few:
             assert len(one.step_times()) == leaves - 1
+
+
+OPTIONS = {
+    "l1_delta": dict(lambda_l1=2.0, max_delta_step=0.4), "smooth": dict(path_smooth=5.0, min_gain_to_split=0.5),
+    "monotone": dict(monotone_constraints=[1, -1, 0, 1], monotone_penalty=1.5), "max_depth": dict(max_depth=3),
+    "no_split": dict(min_data_in_leaf=2500, feature_pre_filter=False), "rows_run_out": dict(min_data_in_leaf=600),
+    "no_renewal": dict(quant_train_renew_leaf=False), "many_bins": dict(num_grad_quant_bins=32),
+}
+
+
+@pytest.mark.parametrize("option", sorted(OPTIONS))
+def test_options(lgb, option):
+    """The other rules of growth, a feature mask and data-parallel growth (one rank) of a learner of few leaves."""
+    rng = np.random.default_rng(9)
+    n, f = 4099, 12
+    X = rng.standard_normal((n, f)).astype(np.float32)
+    X[rng.random(X.shape) < 0.05] = 0.0
+    y = (X[:, 0] + X[:, 1] * X[:, 2] + 0.5 * rng.standard_normal(n) > 0).astype(np.float32)
+    params = {"objective": "binary", "num_leaves": 15, "num_threads": 4, "seed": 3, "use_quantized_grad": True,
+              "num_grad_quant_bins": 4, "stochastic_rounding": True, "quant_train_renew_leaf": True, **OPTIONS[option]}
+    ds = binned_dataset(lgb, X, y, params)
+    one, parallel = lgb.Learner(ds, params), lgb.Learner(ds, params)
+    steps = lgb.Learner(ds, dict(params, persistent_grow=True))
+    parallel.set_data_parallel(0, n, lambda ptr, count, dtype, op: None)
+    mask = np.ones(ds.binned()["num_features"], np.uint8)
+    for it in range(3):
+        if it == 2:
+            mask[::2] = 0
+            for learner in (one, parallel, steps):
+                learner.set_feature_mask(0, mask)
+        g = (0.5 - y + 0.3 * rng.standard_normal(n)).astype(np.float32)
+        h = (0.1 + 0.2 * rng.random(n)).astype(np.float32)
+        a, b, c = (learner.train(g, h)[0] for learner in (one, parallel, steps))
+        for name in a:
+            assert np.array_equal(a[name], c[name]), name
+        for name in ("num_leaves", "split_feature", "threshold_in_bin", "leaf_count"):
+            assert np.array_equal(b[name], c[name]), name
